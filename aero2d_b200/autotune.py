@@ -8,10 +8,11 @@ are bitwise the same; include/aero2d_b200.h, a2d_plan_set_tuning):
             stencil, run gmres_restart + 1 times per Newton step: "32x8",
             "32x16", "64x4" or "16x16" (the halo is recomputed per tile, so
             taller tiles compute less and hold more shared memory);
-  sweep     the line sweep's kernel, by warps per half line group: "lanes"
-            (one warp, a lane solving all four block rows of its line),
-            "pairs" (two warps, two lanes per line with two block rows each)
-            or "rows" (four warps, a warp per block row).
+  sweep     the line sweep's kernel: a launch per sweep, by warps per half line
+            group "lanes" (one warp, a lane solving all four block rows of its
+            line), "pairs" (two warps, two lanes per line with two block rows
+            each) or "rows" (four warps, a warp per block row); or "halves", one
+            launch for every sweep of an application (a cluster per case).
 
 The best configuration depends on the grid sizes in a batch, the batch size and
 the precision.  `apply(plan, measure=True)` looks the plan's key up in the

@@ -119,10 +119,12 @@ void launch_face_jac(const Batch& b, const JacArgs& a, cudaStream_t s);
 template <typename TJ, typename TF>
 void launch_factor(const Batch& b, const FactorArgs& a, cudaStream_t s);
 
-// kernel variants of the line-Jacobi sweep, a plan's tuning knob, by warps per
-// half line group: one, a lane solving all four block rows of its line
-// (sweep.cu); two, two lanes per line with two block rows each (sweep_pairs.cu);
-// four, a warp per block row (sweep_rows.cu)
+// kernel variants of the line-Jacobi sweep, a plan's tuning knob.  One launch per sweep,
+// by warps per half line group: one, a lane solving all four block rows of its line
+// (lanes, sweep.cu); two, two lanes per line with two block rows each (pairs, sweep_pairs.cu);
+// four, a warp per block row (rows, sweep_rows.cu).  All sweeps of an application
+// in one launch, a cluster per case (lines.cu): halves, and on FP64 plans lanes, where
+// every case fits it (lines_clusters); the per-sweep kernels otherwise
 enum : int { kSweepLanes = 0, kSweepRows = 1, kSweepPairs = 2, kSweepHalves = 3, kNumSweepVariants = 4 };
 
 // one line-Jacobi sweep; FIRST: the sweep without i-coupling; last: x is the
@@ -134,13 +136,20 @@ template <typename TI, bool FIRST>
 void launch_sweep_rows(const Batch& b, const SweepArgs& a, bool last, cudaStream_t s);
 template <typename TI, bool FIRST>
 void launch_sweep_pairs(const Batch& b, const SweepArgs& a, bool last, cudaStream_t s);
-template <bool FIRST>   // mixed precision only
-void launch_sweep_halves(const Batch& b, const SweepArgs& a, bool last, cudaStream_t s);
+// every sweep of an application, x = M^-1 r (r, x, e0 and the factors of a), for `count`
+// cases of `groups` line groups each (cases: their indices, on the device) and at most
+// `rows` rows
+template <typename TI>
+void launch_lines(const Batch& b, const SweepArgs& a, const int* cases, int count, int groups, int rows, int sweeps,
+                  cudaStream_t s);
+// clusters of that launch that the current device holds at once; 0: it cannot run there (host)
+template <typename TI>
+int lines_clusters(int groups, int rows);
 
 // raises the dynamic shared-memory limit of the sweep kernels (host, once per device)
 cudaError_t sweep_init();
 cudaError_t sweep_rows_init();
 cudaError_t sweep_pairs_init();
-cudaError_t sweep_halves_init();
+cudaError_t lines_init();
 
 }  // namespace a2d

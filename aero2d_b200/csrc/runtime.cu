@@ -14,6 +14,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <map>
 #include <string>
 #include <type_traits>
 #include <vector>
@@ -86,6 +87,15 @@ struct a2d_plan {
   std::vector<Chunk> chunks;
   std::vector<Group> groups;
   std::vector<long long> cp_off;
+  // cases by line-group count, for the one-launch preconditioner (lines.cu): a launch per
+  // class; line_cases holds the case indices class after class
+  struct LineClass {
+    int groups, rows, first, count;
+  };
+  std::vector<LineClass> line_classes;
+  std::vector<int> line_cases;
+  bool lines_fit = false;      // every class runs on the device bound to (set at bind)
+  size_t o_lcases = 0, o_E0 = 0;   // o_E0: inv r of the lines, kept between the sweeps of an application
   long long C = 0, rows_nc = 0, rows_nc1 = 0, total_ni = 0;
   size_t tj = 8, tb = 8;   // bytes of face-Jacobian and basis storage entries
   size_t tf = 8;           // bytes of the sweep factor entries (G, C, P, Q)
@@ -174,6 +184,14 @@ static void build_tables(a2d_plan* P, const int* ni, const int* nc, const void* 
   P->total_ni = cpo;
   for (int sh = 0; sh < kNumTileShapes; ++sh) P->max_jtiles = std::max(P->max_jtiles, (int)tile_list(P, sh).size());
   P->jtiles = tile_list(P, P->jvp_tile);
+  std::map<int, std::vector<int>> by_groups;
+  for (int k = 0; k < P->ncases; ++k) by_groups[P->cases[k].ngroups].push_back(k);
+  for (const auto& g : by_groups) {
+    a2d_plan::LineClass c{g.first, 0, (int)P->line_cases.size(), (int)g.second.size()};
+    for (int k : g.second) c.rows = std::max(c.rows, nc[k]);
+    P->line_cases.insert(P->line_cases.end(), g.second.begin(), g.second.end());
+    P->line_classes.push_back(c);
+  }
 }
 
 static void layout(a2d_plan* P) {
@@ -198,6 +216,7 @@ static void layout(a2d_plan* P) {
   P->o_INV = cv.take(P->tj * lb * P->rows_nc);
   P->o_CF = cv.take(P->tf * lb * P->rows_nc);
   P->o_PQG = cv.take(3 * P->tf * lb * P->rows_nc);
+  P->o_E0 = cv.take(P->tj * lb / 4 * P->rows_nc);
   P->o_V = cv.take(P->tb * 4 * C * (size_t)(P->m + 1));
   P->o_H = cv.take(8 * (size_t)B * kMaxRestart * (kMaxRestart + 1));
   P->o_h1 = cv.take(8 * (size_t)B * kHStride);
@@ -220,6 +239,7 @@ static void layout(a2d_plan* P) {
   P->o_idx = cv.take(sizeof(int) * (size_t)B);   // case index lists of a2d_case_restart / _retire
   P->o_sat = cv.take(sizeof(unsigned long long));
   P->o_jtiles = cv.take(sizeof(Tile) * (size_t)P->max_jtiles);
+  P->o_lcases = cv.take(sizeof(int) * (size_t)B);
   P->bytes = cv.off + 256;
 }
 
@@ -396,12 +416,25 @@ static FactorArgs factor_args(const a2d_plan* P, uint32_t need) {
   return fa;
 }
 
+// whether an application's sweeps run as one launch per line-group count (lines.cu)
+static bool one_launch(const a2d_plan* P) {
+  return P->lines_fit && P->sweep_variant == (P->p.precision == A2D_MIXED ? kSweepHalves : kSweepLanes);
+}
+
 // x = M^-1 r: jacobi_sweeps line-Jacobi sweeps (aero2d/implicit.py:150-157);
 // rin may be dst
 template <typename TJ>
 static void precond(a2d_plan* P, const Batch& B, const double* rin, double* dst, uint32_t need, cudaStream_t s) {
   SweepArgs a = sweep_args(P, need);
   const int sweeps = std::max(1, P->p.jacobi_sweeps);
+  if (one_launch(P)) {
+    a.r = rin;
+    a.e0 = P->at<double>(P->o_E0);
+    a.x = dst;
+    for (const a2d_plan::LineClass& c : P->line_classes)
+      launch_lines<TJ>(B, a, P->at<int>(P->o_lcases) + c.first, c.count, c.groups, c.rows, sweeps, s);
+    return;
+  }
   double* bufs[2] = {P->vec(kPA), P->vec(kPB)};
   a.r = rin;
   a.e0 = sweeps > 1 ? P->vec(kPE) : nullptr;
@@ -824,10 +857,22 @@ int a2d_plan_bind(a2d_plan* P, void* workspace, size_t bytes, void* stream) {
   P->jbatch = B;
   P->jbatch.tiles = P->at<Tile>(P->o_jtiles);
   P->jbatch.ntiles = (int)P->jtiles.size();
+  A2D_CK(cudaMemcpyAsync(P->ws + P->o_lcases, P->line_cases.data(), sizeof(int) * P->line_cases.size(),
+                         cudaMemcpyHostToDevice, s));
   if (P->host_count == nullptr) A2D_CK(cudaMallocHost(&P->host_count, 2 * sizeof(int)));
   A2D_CK(cudaMemsetAsync(P->ws + P->o_cnt, 0, 8, s));
   A2D_CK(cudaMemsetAsync(P->ws + P->o_sat, 0, sizeof(unsigned long long), s));
   A2D_CK(sweep_init());
+  P->lines_fit = true;
+  for (const a2d_plan::LineClass& c : P->line_classes) {
+    const bool mixed = P->p.precision == A2D_MIXED;
+    const int n = mixed ? lines_clusters<float>(c.groups, c.rows) : lines_clusters<double>(c.groups, c.rows);
+    // FP64 holds one CTA per SM, and a cluster is bound by the length of its lines: past
+    // the cases that run at once the per-sweep kernels win (256 x 64, B200: 8 cases 111 against
+    // 193 us, 16 cases in two waves 196 against 180); the mixed one wins at every count measured
+    // (1 to 64 cases: 39 against 85, 137 against 180)
+    P->lines_fit = P->lines_fit && (mixed ? n > 0 : n >= c.count);
+  }
   A2D_CK(gs_init());
   stencil_init_fp64();
   stencil_init_fp32();
@@ -1138,6 +1183,9 @@ int a2d_time_kernel(a2d_plan* P, int which, int reps, float* ms, void* stream) {
   const bool mixed = P->p.precision == A2D_MIXED;
   const size_t vs = 4 * (size_t)P->C;
   const int half = std::max(1, P->m / 2);
+  // where the sweeps of an application are one launch, that launch is timed and its
+  // time shared between them
+  const bool whole = one_launch(P) && (which == A2D_K_SWEEP || which == A2D_K_SWEEP_FIRST);
   auto launch_once = [&]() {
     switch (which) {
       case A2D_K_JVP: {
@@ -1163,6 +1211,11 @@ int a2d_time_kernel(a2d_plan* P, int which, int reps, float* ms, void* stream) {
         break;
       }
       case A2D_K_SWEEP: {
+        if (whole) {
+          if (mixed) precond<float>(P, B, P->vec(kZ), P->vec(kPA), 0, s);
+          else precond<double>(P, B, P->vec(kZ), P->vec(kPA), 0, s);
+          break;
+        }
         SweepArgs a = sweep_args(P, 0);
         a.e0 = P->vec(kPE);
         a.xprev = P->vec(kPB);
@@ -1172,6 +1225,11 @@ int a2d_time_kernel(a2d_plan* P, int which, int reps, float* ms, void* stream) {
         break;
       }
       case A2D_K_SWEEP_FIRST: {
+        if (whole) {
+          if (mixed) precond<float>(P, B, P->vec(kZ), P->vec(kPA), 0, s);
+          else precond<double>(P, B, P->vec(kZ), P->vec(kPA), 0, s);
+          break;
+        }
         SweepArgs a = sweep_args(P, 0);
         a.r = P->vec(kZ);
         a.e0 = P->vec(kPE);
@@ -1257,7 +1315,7 @@ int a2d_time_kernel(a2d_plan* P, int which, int reps, float* ms, void* stream) {
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   A2D_CK(cudaGetLastError());
-  *ms = t / reps;
+  *ms = t / reps / (whole ? std::max(1, P->p.jacobi_sweeps) : 1);
   return A2D_OK;
 }
 

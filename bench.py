@@ -316,9 +316,11 @@ def step_profile(step_ms, live, B):
             if ((live >= lo) & (live <= hi)).any()}
 
 
-def algorithmic_bytes(kernel: str, cells: int, restart: int, mixed: bool) -> float:
+def algorithmic_bytes(kernel: str, cells: int, restart: int, mixed: bool, one_launch: bool = False) -> float:
     """Bytes a kernel must move per launch for the whole batch (cells = total
-    cells); counts the matrix and vector words of the kernel's definition once."""
+    cells); counts the matrix and vector words of the kernel's definition once.
+    one_launch: all four sweeps of an application are one launch, and a sweep is a
+    quarter of it (the factors counted once per application)."""
     f = 4 if mixed else 8
     h = 2 if mixed else 8   # sweep factors G, C, P, Q (FP16 in the mixed path)
     v = 4 if mixed else 8   # intermediate vectors of the sweeps (FP32 in the mixed path)
@@ -340,6 +342,9 @@ def algorithmic_bytes(kernel: str, cells: int, restart: int, mixed: bool) -> flo
         # pass 3: w, restart/2 basis vectors, the next basis vector written
         "update": 4 * d + half * 4 * kb + 4 * kb,
     }[kernel]
+    if one_launch and kernel.startswith("sweep"):
+        # r, inv, P, Q, G, C, x
+        per_cell = (4 * d + 16 * f + 4 * 16 * h + 4 * d) / 4
     return float(per_cell) * cells
 
 
@@ -533,12 +538,14 @@ def gpu_arm(args, rank: int, world: int, dist):
     share = {k: ktimes[k] * launches_per_step(k, args.restart) for k in kernels}
     dom = max(share, key=share.get)
     peak, peak_kind = measured_peak()
-    achieved = algorithmic_bytes(dom, cells, args.restart, True) / (ktimes[dom] / 1e3) / 1e9
+    one = plan.tuning()[1] == "halves"
+    dom_bytes = algorithmic_bytes(dom, cells, args.restart, True, one)
+    achieved = dom_bytes / (ktimes[dom] / 1e3) / 1e9
     traffic_per_cell = read_traffic(dom)
     out["roofline"] = {"kernel": dom, "bound": "hbm", "achieved": round(achieved, 1), "peak": peak,
                        "unit": "GB/s", "frac": round(achieved / peak, 3), "peak_source": peak_kind,
                        "traffic": (round(traffic_per_cell * cells) if traffic_per_cell else None),
-                       "algorithmic_bytes_per_launch": algorithmic_bytes(dom, cells, args.restart, True),
+                       "algorithmic_bytes_per_launch": dom_bytes,
                        "ms_per_launch": round(ktimes[dom], 4)}
     out["kernels_ms_per_launch"] = {k: round(v, 4) for k, v in ktimes.items()}
     out["kernels_ms_per_newton_step"] = {k: round(v, 3) for k, v in share.items()}

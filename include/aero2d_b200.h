@@ -106,12 +106,13 @@ int a2d_plan_ncases(const a2d_plan* plan);
 #define A2D_JVP_TILE_32x16 1    /* always use 32 x 8 */
 #define A2D_JVP_TILE_64x4 2
 #define A2D_JVP_TILE_16x16 3
-#define A2D_SWEEP_LANES 0       /* line sweep: one warp per half line group, a lane per line   */
-#define A2D_SWEEP_ROWS 1        /* line sweep: four warps per half line group, a warp per block row */
-#define A2D_SWEEP_PAIRS 2       /* line sweep: two warps per half line group, two lanes per line */
-#define A2D_SWEEP_HALVES 3      /* line sweep: a cluster of two CTAs per line group, one per half,  */
-                                /* a warp per block row, the halves meeting in distributed shared  */
-                                /* memory                                                           */
+#define A2D_SWEEP_LANES 0       /* a launch per sweep: one warp per half line group, a lane per line;   */
+                                /* FP64 plans: as HALVES while every case's cluster runs at once       */
+#define A2D_SWEEP_ROWS 1        /* a launch per sweep: four warps per half line group, a warp per block row */
+#define A2D_SWEEP_PAIRS 2       /* a launch per sweep: two warps per half line group, two lanes per line */
+#define A2D_SWEEP_HALVES 3      /* every sweep of an application in one launch: a cluster per case, a   */
+                                /* CTA per line group, a recurrence warp per half (cases of more than  */
+                                /* 512 lines or rows past the shared memory: as ROWS)                   */
 /* a new plan starts with A2D_JVP_TILE_32x16 and A2D_SWEEP_HALVES (FP64 plans: A2D_SWEEP_LANES);
  * A2D_SWEEP_ROWS and A2D_SWEEP_HALVES are refused on FP64 plans (A2D_ERR_ARG) */
 /* any time, bound or not; a change re-captures the Newton step's graph at the next step */
@@ -260,7 +261,8 @@ int a2d_plan_stats(const a2d_plan* plan, int* kernels_per_step, int* steps_taken
 #define A2D_K_JVP 0        /* linearised residual stencil on the whole batch            */
 #define A2D_K_SWEEP 1      /* one coupled line-Jacobi sweep (right-hand side + both     */
                            /* block-Thomas recurrences, fused)                          */
-#define A2D_K_SWEEP_FIRST 2 /* the first sweep of a preconditioner application         */
+#define A2D_K_SWEEP_FIRST 2 /* the first sweep of a preconditioner application; where   */
+                           /* one launch runs all sweeps, both are its time / sweeps    */
 #define A2D_K_DOTS 3       /* Gram-Schmidt pass 1: projections on restart/2 vectors     */
 #define A2D_K_UPDATE 4     /* Gram-Schmidt pass 3: subtraction, next basis vector       */
 #define A2D_K_RESIDUAL 5   /* FP64 residual stencil                                     */

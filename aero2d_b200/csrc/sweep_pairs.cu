@@ -313,6 +313,8 @@ __global__ void __launch_bounds__(kSweepThreads) k_sweep(Batch b, SweepArgs a) {
     const bool ok = mbar_wait(&sm.full[h][t % S], (t / S) & 1);
     return __all_sync(0xffffffffu, ok);
   };
+  // the warp is done with stage t: called after the exchange (or a store) of a value computed
+  // from the stage, since an arrival alone does not wait for the stage's loads to return
   auto release = [&](int t) {
     __syncwarp();
     if (lane == 0) mbar_arrive(&sm.empty[h][t % S]);
@@ -342,11 +344,11 @@ __global__ void __launch_bounds__(kSweepThreads) k_sweep(Batch b, SweepArgs a) {
           TC d[2];
           rhs(s, roff, re[uu], rx[uu], rl[uu], rr[uu], d);
           addmv(s, kOffG, dprev, d);
-          release(t);
 #pragma unroll
           for (int q = 0; q < 2; ++q)
             if (owner) dvb[q * comp + roff] = d[q];
           full4(p, d, dprev);
+          release(t);
           roff += rstep;
           load_vec(t + L, voff, uu);
           voff += rstep;
@@ -385,12 +387,12 @@ __global__ void __launch_bounds__(kSweepThreads) k_sweep(Batch b, SweepArgs a) {
       rhs(s, k * ni, ve, vx, vl, vr, xv);
       addmv(s, kOffG, dprev, xv);
       addmv(s, kOffH, dpl, xv);
-      release(t);
 #pragma unroll
       for (int q = 0; q < 2; ++q) {
         sm.xk[l][r0 + q] = xv[q];
         if (owner) xb[q * comp + k * ni] = TX(xv[q]);
       }
+      release(t);
     }
     if (fail && lane == 0) sm.failed[0] = 1;
   }
@@ -431,13 +433,13 @@ __global__ void __launch_bounds__(kSweepThreads) k_sweep(Batch b, SweepArgs a) {
               for (int c = 1; c < 4; ++c) acc += cv[c] * xn[c];
               xv[q] = dbuf[u][q] - acc;
             }
-            release(t);
 #pragma unroll
             for (int q = 0; q < 2; ++q) {
               if (owner) xb[q * comp + boff] = TX(xv[q]);
               if (t + LB < nsteps) dbuf[u][q] = dvb[q * comp + poff];
             }
             full4(p, xv, xn);
+            release(t);
             boff += bstep;
             poff += bstep;
           }

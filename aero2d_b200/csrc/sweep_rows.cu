@@ -298,7 +298,8 @@ __global__ void __launch_bounds__(kSweepThreads, 4) k_sweep(Batch b, SweepArgs a
   auto wait_full = [&](int t) {
     if (!mbar_wait(&sm.full[h][t % S], (t / S) & 1)) wfail = true;
   };
-  // this warp is done with stage t % S
+  // this warp is done with stage t % S: called after a store of a value computed from the
+  // stage, since an arrival alone does not wait for the stage's loads to return
   auto release = [&](int t) {
     __syncwarp();
     if (lane == 0) mbar_arrive(&sm.empty[h][t % S]);
@@ -361,12 +362,12 @@ __global__ void __launch_bounds__(kSweepThreads, 4) k_sweep(Batch b, SweepArgs a
         const TC e = rhs(t, s, roff);
         TC gv[4], dp[4];
         load4(reinterpret_cast<const TF*>(sm.mat[h][s] + kOffG) + eo, gv);
-        release(t);
         load4(&sm.xchg[h][(t + 1) & 1][l][0], dp);
         TC d = e;
 #pragma unroll
         for (int c = 0; c < 4; ++c) d += gv[c] * dp[c];
         sm.xchg[h][t & 1][l][q] = d;
+        release(t);
         if (owner) dvb[roff] = d;
         roff += rstep;
         store_vec(t + 1 < nvec, (t + 1) & 1, (uu + 1) % L);   // step t+1's entries, published by the barrier
@@ -388,7 +389,6 @@ __global__ void __launch_bounds__(kSweepThreads, 4) k_sweep(Batch b, SweepArgs a
     TC gv[4], hv[4], dm[4], dpl[4];
     load4(reinterpret_cast<const TF*>(sm.mat[h][s] + kOffG) + eo, gv);
     load4(reinterpret_cast<const TF*>(sm.mat[h][s] + kOffH) + eo, hv);
-    release(t);
     load4(&sm.xchg[0][(k + 1) & 1][l][0], dm);                        // d_{k-1}
     if (nf1 > 0) load4(&sm.xchg[1][(nf1 + 1) & 1][l][0], dpl);        // d'_{k+1}
     else dpl[0] = dpl[1] = dpl[2] = dpl[3] = TC(0);
@@ -398,6 +398,7 @@ __global__ void __launch_bounds__(kSweepThreads, 4) k_sweep(Batch b, SweepArgs a
 #pragma unroll
     for (int c = 0; c < 4; ++c) xv += hv[c] * dpl[c];
     sm.xk[l][q] = xv;
+    release(t);
     if (owner) xb[koff] = TX(xv);
     if (half_sync_or(h, wfail)) {
       tstop = t;
@@ -435,13 +436,13 @@ __global__ void __launch_bounds__(kSweepThreads, 4) k_sweep(Batch b, SweepArgs a
           }
           TC cv[4], xn[4];
           load4(reinterpret_cast<const TF*>(sm.mat[h][s] + (h == 0 ? pslot - u % kPack : u % kPack) * kBytesF) + eo, cv);
-          if (u % kPack == kPack - 1 || t + 1 == nsteps) release(n);
           load4(t == t0 ? &sm.xk[l][0] : &sm.xchg[h][(t + 1) & 1][l][0], xn);
           TC acc = cv[0] * xn[0];
 #pragma unroll
           for (int c = 1; c < 4; ++c) acc += cv[c] * xn[c];
           const TC xv = dbuf[u] - acc;
           sm.xchg[h][t & 1][l][q] = xv;
+          if (u % kPack == kPack - 1 || t + 1 == nsteps) release(n);
           if (owner) xb[boff] = TX(xv);
           boff += bstep;
           if (t + kBackAhead < nsteps) dbuf[u] = dvb[poff];

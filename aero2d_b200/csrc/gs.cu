@@ -3,59 +3,56 @@
 // Krylov basis per Arnoldi step.
 //
 //   pass 1  k_gs_dots     raw projections V_raw[q] . w and w . w, per chunk
-//   reduce  k_gs_reduce   per case, fixed chunk order: h1_q = s_q (V_raw[q] . w)
-//   pass 2  k_gs_project  w' = w - sum_q V_raw[q] s_q h1_q and V_raw[q] . w' from one
-//                         read of the basis (the sub-tile stays in shared memory
-//                         between the subtraction and the projection)
-//   reduce  k_gs_reduce   h2_q
-//   pass 3  k_gs_sub      w'' = w - sum_q V_raw[q] s_q (h1_q + h2_q), written as the
-//                         next raw basis vector, with its squared norm
+//   pass 2  k_gs_project  h1_q = s_q (V_raw[q] . w) reduced over the case's chunks, then
+//                         w' = w - sum_q V_raw[q] s_q h1_q and V_raw[q] . w' from one
+//                         read of the basis
+//   pass 3  k_gs_sub      h2_q the same way, w'' = w - sum_q V_raw[q] s_q (h1_q + h2_q),
+//                         written as the next raw basis vector, with its squared norm
 //   close   k_gs_close    per case: h_{k+1,k} = ||w''||, the breakdown test against
 //                         eps ||w|| (jax.scipy.sparse.linalg.gmres semantics), the
 //                         Hessenberg column and s_{k+1} = 1 / ||w''||
 //
-// The three passes stream a 4096-entry chunk per CTA through shared memory by
-// bulk copies (see "streaming passes" below); a thread keeps one partial sum
-// per basis vector in registers (the count is a template tier NQ of 8, 16, 24
-// or 32), so a chunk needs a single block reduction.  Bases of more than 32
-// vectors are processed in slices of 32 by chained launches.  Basis vectors
-// are stored unnormalised with their scale s_q, so no normalisation pass is
-// needed; w' is never stored, since pass 3 subtracts h1 + h2 from the
+// Basis vectors are stored unnormalised with their scale s_q, so no normalisation
+// pass is needed; w' is never stored, since pass 3 subtracts h1 + h2 from the
 // original w (equal to the two successive subtractions in exact arithmetic).
+//
+// The order of every sum.  A chunk of 4096 entries is 8 rows of 32 lanes with 16 entries
+// each.  A lane's products are added one after the other (chain index i = 0 .. 15), the 32
+// lanes of a row by a fixed tree, a chunk's 8 rows in order, a case's chunks in
+// warp_chunk_sum's order.  None of it depends on how rows and vectors are dealt to warps
+// and CTAs, nor on the other cases of a batch.  A subtraction's sum runs over the vectors in
+// order, 32 at a time (the slices it was once cut into).  Products are fused into the sums
+// and differences are not, spelled out, so that no unrolling changes a bit: h2 is made of w's
+// rounding, and a marginal case's path follows it.
+//
+// What bounds the passes: the basis from HBM (each pass reads it once from there), with few
+// chunks the latency of one CTA.  A warp owns a row (in split launches a quarter of one)
+// and runs it through alone: the row's entries of w stay in registers from the subtraction to
+// the projections, the vectors go by through a ring of asynchronous copies of 1 KB each that every
+// lane reads back itself, so nothing waits on a barrier, and pass 2's second reading of
+// the row comes from L2.  (Partial sums of all vectors in a thread's registers, as
+// the passes had before, held an SM to 16 warps.)  Where a batch has too few chunks for the
+// GPU, the rows of a chunk are the CTAs of a cluster, whose first CTA adds their sums.
+// Measured (B200, BF16, average over an Arnoldi process of 30 vectors, 64 cases of 256 x 64,
+// passes 1 / 2 / 3): 46 / 64 / 40 -> 33 / 51 / 36 us, of 24 / 24 / 26 us at the HBM peak; one
+// case of 128 x 48, 27 vectors: 19 / 25 / 17 -> 6 / 12 / 12 us; FP64, 16 cases of 256 x 64, 27
+// vectors: 53 / 96 / 66 -> 39 / 75 / 45 us.  A ring of 8 KB or 2 KB, and four CTAs per SM, were slower.
 #include <cfloat>
 #include <cuda_bf16.h>
 #include <type_traits>
 
 #include "batch.cuh"
 #include "gs.cuh"
-#include "tma.cuh"
 
 namespace a2d {
 
-constexpr int kGB = 256;                 // threads per block
-constexpr int kGE = kChunk / kGB;        // entries per thread
-static_assert(kGE * kGB == kChunk, "chunk must split evenly over the block");
-
-// fixed-order reduction of NV values over the block; thread t < NV receives value t
-template <int NV>
-__device__ __forceinline__ double gs_reduce_to_thread(double (&v)[NV], double* scratch /* 8*NV */) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-  for (int q = 0; q < NV; ++q) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v[q] += __shfl_down_sync(0xffffffffu, v[q], o);
-  }
-  if (lane == 0) {
-#pragma unroll
-    for (int q = 0; q < NV; ++q) scratch[warp * NV + q] = v[q];
-  }
-  __syncthreads();
-  double s = 0.0;
-  if (threadIdx.x < NV) {
-    for (int w = 0; w < kGB / 32; ++w) s += scratch[w * NV + threadIdx.x];
-  }
-  return s;
-}
+constexpr int kRows = kGsRows;           // rows of a chunk
+// warps of a CTA: a row of the chunk each, or (split) four on the chunk's row blockIdx.y
+constexpr int warps_of(bool split) { return split ? 4 : kRows; }
+constexpr int kBatchQ = 8;               // vectors projected on at a time
+constexpr int kChain = 16;               // entries of a lane in a row
+static_assert(kRows * 32 * kChain == kChunk, "a chunk is 8 rows of 32 lanes with 16 entries");
+constexpr int kSlice = 32;               // vectors of one subtraction sum
 
 // fixed-order sum of a per-chunk partial over a case's chunks (every lane gets it)
 __device__ __forceinline__ double warp_chunk_sum(const double* p, size_t stride, int nchunks) {
@@ -67,35 +64,27 @@ __device__ __forceinline__ double warp_chunk_sum(const double* p, size_t stride,
   return s;
 }
 
-// s_q (h1_q [+ h2_q]) of the slice's vectors into shared memory
-template <typename TB>
-__device__ __forceinline__ void coef_to_smem(const GsArgs<TB>& a, int cs, int ncases, double* coef, bool both) {
-  for (int q = threadIdx.x; q < a.nq; q += blockDim.x) {
-    const int qq = a.q0 + q;
-    double h = a.h1[(size_t)cs * kHStride + qq];
-    if (both) h += a.h2[(size_t)cs * kHStride + qq];
-    coef[q] = h * a.scale[(size_t)qq * ncases + cs];
-  }
-  __syncthreads();
-}
-
-// the same from the folded reduction: one warp per coefficient reduces the case's
-// chunk partials in k_gs_reduce's order; the case's first chunk stores the result
-template <typename TB>
-__device__ __forceinline__ void coef_folded(const GsArgs<TB>& a, const CaseDev& cs, int cs_id, int ncases,
-                                            bool first_chunk, double* coef, bool both) {
+// this pass's coefficients s_q h_q of every vector into shared memory: one warp per
+// coefficient reduces the case's partials of the pass before; the case's first CTA stores
+// the result
+template <bool SPLIT, typename TB>
+__device__ __forceinline__ void coefficients(const GsArgs<TB>& a, const CaseDev& cs, int cs_id, int ncases, bool first,
+                                             double* coef, bool both) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int nred = a.nq + (a.fold_wn0 != nullptr ? 1 : 0);
-  for (int q = warp; q < nred; q += blockDim.x >> 5) {
-    const double sum = warp_chunk_sum(a.fold_part + (size_t)cs.chunk0 * a.pstride + q, a.pstride, cs.nchunks);
+  const double* part = a.fold_part + (size_t)cs.chunk0 * a.pstride;
+#pragma unroll 4
+  for (int q = warp; q < nred; q += warps_of(SPLIT)) {
+    const double sum = warp_chunk_sum(part + q, a.pstride, cs.nchunks);
     if (lane == 0) {
       if (q < a.nq) {
         const double sc = a.scale[(size_t)q * ncases + cs_id];
-        const double h = sum * sc;
-        if (first_chunk) a.fold_h[(size_t)cs_id * kHStride + q] = h;
-        const double hh = both ? a.h1[(size_t)cs_id * kHStride + q] + h : h;
+        // rounded as H's column is (k_gs_close adds the stored h1 and h2)
+        const double h = __dmul_rn(sum, sc);
+        if (first) a.fold_h[(size_t)cs_id * kHStride + q] = h;
+        const double hh = both ? __dadd_rn(a.h1[(size_t)cs_id * kHStride + q], h) : h;
         coef[q] = hh * sc;
-      } else if (first_chunk) {
+      } else if (first) {
         a.fold_wn0[cs_id] = sqrt(sum);
       }
     }
@@ -103,382 +92,504 @@ __device__ __forceinline__ void coef_folded(const GsArgs<TB>& a, const CaseDev& 
   __syncthreads();
 }
 
-// vector loads and stores of N consecutive entries (chunks start on multiples of
-// 4 entries and every case vector and basis vector on a 256-byte boundary)
-__device__ __forceinline__ void ldv(const float* p, double (&v)[4]) {
-  const float4 t = *reinterpret_cast<const float4*>(p);
-  v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
+// ---- a lane's entries of a row, four at a time (quad m: chain indices 4 m .. 4 m + 3) ----
+// BF16: four consecutive entries, m a quarter of the chunk apart; FP64: entries a
+// sixteenth of the chunk apart, so that a warp's loads are runs of 256 bytes either way
+template <typename TB> struct Quad;
+template <> struct Quad<__nv_bfloat16> {
+  uint2 raw;
+  static __device__ __forceinline__ int at(int r, int m, int lane) { return m * (kChunk / 4) + (32 * r + lane) * 4; }
+  __device__ __forceinline__ void load(const __nv_bfloat16* p, int r, int m, int lane, int len) {
+    const int e = at(r, m, lane);
+    raw = e < len ? __ldg(reinterpret_cast<const uint2*>(p + e)) : make_uint2(0u, 0u);
+  }
+  __device__ __forceinline__ void read(const uint64_t* s, int m) { raw = *reinterpret_cast<const uint2*>(s + m * 32); }
+  __device__ __forceinline__ double operator[](int t) const {
+    const uint32_t w = t < 2 ? raw.x : raw.y;
+    return (double)__uint_as_float(t & 1 ? w & 0xffff0000u : w << 16);
+  }
+};
+template <> struct Quad<double> {
+  double v[4];
+  static __device__ __forceinline__ int at(int r, int i, int lane) { return i * (kChunk / 16) + 32 * r + lane; }
+  __device__ __forceinline__ void load(const double* p, int r, int m, int lane, int len) {
+#pragma unroll
+    for (int t = 0; t < 4; ++t) {
+      const int e = at(r, 4 * m + t, lane);
+      v[t] = e < len ? __ldg(p + e) : 0.0;
+    }
+  }
+  __device__ __forceinline__ void read(const uint64_t* s, int m) {
+#pragma unroll
+    for (int t = 0; t < 4; ++t) v[t] = reinterpret_cast<const double*>(s)[(4 * m + t) * 32];
+  }
+  __device__ __forceinline__ double operator[](int t) const { return v[t]; }
+};
+// the same entries of an FP64 vector; and calling f(t, entry offset) for those in the chunk
+template <typename TB>
+__device__ __forceinline__ void load_w(const double* w, int r, int m, int lane, int len, double (&v)[4]) {
+  if constexpr (std::is_same<TB, double>::value) {
+    Quad<double> q;
+    q.load(w, r, m, lane, len);
+#pragma unroll
+    for (int t = 0; t < 4; ++t) v[t] = q[t];
+  } else {
+    const int e = Quad<TB>::at(r, m, lane);
+    const double2 z = make_double2(0.0, 0.0);
+    const double2 a = e < len ? __ldg(reinterpret_cast<const double2*>(w + e)) : z;
+    const double2 b = e < len ? __ldg(reinterpret_cast<const double2*>(w + e + 2)) : z;
+    v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
+  }
 }
+__device__ __forceinline__ void store_quad(__nv_bfloat16* p, int r, int m, int lane, int len, const double (&v)[4]) {
+  const int e = Quad<__nv_bfloat16>::at(r, m, lane);
+  if (e >= len) return;
+  __nv_bfloat162 lo = __floats2bfloat162_rn((float)v[0], (float)v[1]);
+  __nv_bfloat162 hi = __floats2bfloat162_rn((float)v[2], (float)v[3]);
+  *reinterpret_cast<uint2*>(p + e) = make_uint2(*reinterpret_cast<uint32_t*>(&lo), *reinterpret_cast<uint32_t*>(&hi));
+}
+__device__ __forceinline__ void store_quad(double* p, int r, int m, int lane, int len, const double (&v)[4]) {
+#pragma unroll
+  for (int t = 0; t < 4; ++t) {
+    const int e = Quad<double>::at(r, 4 * m + t, lane);
+    if (e < len) p[e] = v[t];
+  }
+}
+
+// The sums over the 32 lanes of N values, by the tree l + (l + 16), .. + 8, 4, 2, 1: while more
+// than one value is left a lane keeps half of them and hands the other half over, so N
+// values take about N + 4 exchanges instead of 5 N.  The result's value index is lane_value<N>().
+template <int N>
+__device__ __forceinline__ double warp_tree(double (&v)[N], int o = 16) {
+  const bool up = threadIdx.x & o;
+  if constexpr (N == 1) {
+    double s = v[0];
+    for (; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    return s;
+  } else {
+    constexpr int H = (N + 1) / 2;
+    double k[H];
+#pragma unroll
+    for (int q = 0; q < H; ++q) {
+      const double hi = q + H < N ? v[q + H] : 0.0;
+      const double give = up ? v[q] : hi, keep = up ? hi : v[q];
+      k[q] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+    }
+    return warp_tree<H>(k, o >> 1);
+  }
+}
+// which of the N values this lane's sum is (-1: none), and whether it is the lane that stores it
+template <int N>
+__device__ __forceinline__ int lane_value(bool& owner, int o = 16) {
+  if constexpr (N == 1) {
+    owner = (threadIdx.x & (2 * o - 1)) == 0;
+    return 0;
+  } else {
+    constexpr int H = (N + 1) / 2;
+    const int inner = lane_value<H>(owner, o >> 1);
+    const int q = inner + (threadIdx.x & o ? H : 0);
+    return inner < 0 || q >= N ? -1 : q;
+  }
+}
+
+// ---- a row of the basis, vector after vector, through a warp's ring in shared memory ----
+// Every lane copies (cp.async, 8 bytes) and reads back its own entries only, so the ring needs no
+// barrier, and the bytes in flight do not depend on registers: 24 warps of an SM keep
+// kRingDepth KB each (BF16) on the way.
+template <typename TB> struct RingDepth { static constexpr int value = 4; };
+template <> struct RingDepth<double> { static constexpr int value = 2; };
+template <typename TB>
+struct Ring {
+  static constexpr int D = RingDepth<TB>::value;
+  static constexpr int kWords = 32 * kChain * sizeof(TB) / 8;   // 8-byte words of a row
+  static constexpr int kLaneWords = kWords / 32;
+  static constexpr uint32_t kBytes = D * kWords * 8;            // per warp
+  const TB* V;          // the chunk's first entry of vector 0
+  size_t vstride;
+  const uint64_t* mem;  // this lane's words: [slot][word][lane]
+  int nq, r, lane, len;
+  __device__ __forceinline__ void issue(int q, int slot) {
+    if (q < nq) {
+      const TB* src = V + (size_t)q * vstride;
+      const uint32_t dst = static_cast<uint32_t>(__cvta_generic_to_shared(mem + slot * kWords));
+#pragma unroll
+      for (int k = 0; k < kLaneWords; ++k) {
+        const int e = Quad<TB>::at(r, k, lane);
+        const uint32_t n = e < len ? 8u : 0u;
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(dst + k * 256), "l"(src + (e < len ? e : 0)),
+                     "r"(n)
+                     : "memory");
+      }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  }
+  __device__ __forceinline__ void start() {
+#pragma unroll
+    for (int q = 0; q < D; ++q) issue(q, q);
+  }
+  // quads of vector q (in slot), which is then refilled with vector q + D
+  __device__ __forceinline__ void take(int q, int slot, Quad<TB> (&v)[4]) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(D - 1) : "memory");
+    const uint64_t* s = mem + slot * kWords;
+#pragma unroll
+    for (int m = 0; m < 4; ++m) v[m].read(s, m);
+    issue(q + D, slot);
+  }
+};
+
+// ---- a chunk's sums from its rows', added in order ----
+// split: the rows are CTAs of one cluster (rank = row), whose sums the first one reads from
+// their shared memory
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ double peer_value(const double* p, int rank) {
+  uint32_t addr;
+  double v;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;"
+               : "=r"(addr)
+               : "r"(static_cast<uint32_t>(__cvta_generic_to_shared(p))), "r"(rank));
+  asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(addr) : "memory");
+  return v;
+}
+// out[q] = the chunk's sum q < n; rowsum: the CTA's rows (split: its one row)
+template <bool SPLIT>
+__device__ __forceinline__ void store_chunk(double* out, const double (*rowsum)[kMaxRestart + 1], int n) {
+  if constexpr (SPLIT) {
+    cluster_sync();
+    if (blockIdx.y == 0 && threadIdx.x < n) {
+      double v[kRows], s = 0.0;
+#pragma unroll
+      for (int r = 0; r < kRows; ++r) v[r] = peer_value(&rowsum[0][threadIdx.x], r);
+#pragma unroll
+      for (int r = 0; r < kRows; ++r) s += v[r];
+      out[threadIdx.x] = s;
+    }
+    cluster_sync();   // the rows' shared memory stays until it is read
+  } else {
+    __syncthreads();
+    for (int q = threadIdx.x; q < n; q += 32 * warps_of(SPLIT)) {
+      double s = 0.0;
+#pragma unroll
+      for (int r = 0; r < kRows; ++r) s += rowsum[r][q];
+      out[q] = s;
+    }
+  }
+}
+
+// the projections of a row, whose entries of w are wv, on the vectors q0, q0 + step, ..;
+// vec(v, q, m) gives quad m of vector q.  The sums go to rowsum[q].
+template <typename TB, class F>
+__device__ __forceinline__ void project_row(int nq, int q0, int step, F vec, const double (&wv)[kChain],
+                                            double* rowsum) {
+#pragma unroll 1
+  for (int qb = q0; qb < nq; qb += kBatchQ * step) {
+    double acc[kBatchQ];
+#pragma unroll
+    for (int j = 0; j < kBatchQ; ++j) acc[j] = 0.0;
+#pragma unroll
+    for (int j = 0; j < kBatchQ; ++j) {
+      const int q = qb + step * j;
+      if (q < nq) {
+        Quad<TB> v[4];
+#pragma unroll
+        for (int m = 0; m < 4; ++m) vec(v[m], q, m);
+#pragma unroll
+        for (int m = 0; m < 4; ++m)
+#pragma unroll
+          for (int t = 0; t < 4; ++t) acc[j] = fma(v[m][t], wv[4 * m + t], acc[j]);
+      }
+    }
+    bool owner;
+    const int j = lane_value<kBatchQ>(owner);
+    const double s = warp_tree<kBatchQ>(acc);
+    const int q = qb + step * j;
+    if (owner && q < nq) rowsum[q] = s;
+  }
+}
+
+// x = w - sum_q V_q coef_q for one quad of entries, 32 vectors to a sum; vec(v, q) gives the
+// quad of vector q
+template <typename TB, class F>
+__device__ __forceinline__ void subtract(int nq, F vec, const double* coef, double (&x)[4]) {
+  constexpr int kAhead = std::is_same<TB, double>::value ? 4 : 8;   // quads loaded at a time
+  for (int q0 = 0; q0 < nq; q0 += kSlice) {
+    const int q1 = min(nq, q0 + kSlice);
+    double sub[4] = {0.0, 0.0, 0.0, 0.0};
+    auto take = [&](int q, int n, auto whole) {
+      Quad<TB> v[kAhead];
+#pragma unroll
+      for (int j = 0; j < kAhead; ++j)
+        if (decltype(whole)::value || j < n) vec(v[j], q + j);
+#pragma unroll
+      for (int j = 0; j < kAhead; ++j)
+        if (decltype(whole)::value || j < n) {
+#pragma unroll
+          for (int t = 0; t < 4; ++t) sub[t] = fma(v[j][t], coef[q + j], sub[t]);
+        }
+    };
+    int q = q0;
+#pragma unroll 1
+    for (; q + kAhead <= q1; q += kAhead) take(q, kAhead, std::true_type());
+    if (q < q1) take(q, q1 - q, std::false_type());
+#pragma unroll
+    for (int t = 0; t < 4; ++t) x[t] = __dsub_rn(x[t], sub[t]);
+  }
+}
+
+template <typename TB>
+__device__ __forceinline__ Ring<TB> ring_of(unsigned char* sm, const TB* V, const GsArgs<TB>& a, int r, int len) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  return Ring<TB>{V, a.vstride, reinterpret_cast<const uint64_t*>(sm + warp * Ring<TB>::kBytes) + lane, a.nq, r, lane, len};
+}
+
+// the same two for a warp with the row to itself, every vector through its ring
+template <typename TB>
+__device__ __forceinline__ void project_ring(Ring<TB>& ring, const double (&wv)[kChain], double* rowsum) {
+  constexpr int D = Ring<TB>::D;
+  static_assert(kBatchQ % D == 0, "slots are known at compile time");
+  ring.start();
+#pragma unroll 1
+  for (int qb = 0; qb < ring.nq; qb += kBatchQ) {
+    double acc[kBatchQ];
+#pragma unroll
+    for (int j = 0; j < kBatchQ; ++j) {
+      acc[j] = 0.0;
+      if (qb + j < ring.nq) {
+        Quad<TB> v[4];
+        ring.take(qb + j, j % D, v);
+#pragma unroll
+        for (int m = 0; m < 4; ++m)
+#pragma unroll
+          for (int t = 0; t < 4; ++t) acc[j] = fma(v[m][t], wv[4 * m + t], acc[j]);
+      }
+    }
+    bool owner;
+    const int j = lane_value<kBatchQ>(owner);
+    const double s = warp_tree<kBatchQ>(acc);
+    if (owner && qb + j < ring.nq) rowsum[qb + j] = s;
+  }
+}
+template <typename TB>
+__device__ __forceinline__ void subtract_ring(Ring<TB>& ring, const double* coef, double (&x)[4][4]) {
+  constexpr int D = Ring<TB>::D;
+  static_assert(kSlice % D == 0, "slots are known at compile time");
+  for (int q0 = 0; q0 < ring.nq; q0 += kSlice) {
+    const int q1 = min(ring.nq, q0 + kSlice);
+    double sub[4][4];
+#pragma unroll
+    for (int m = 0; m < 4; ++m)
+#pragma unroll
+      for (int t = 0; t < 4; ++t) sub[m][t] = 0.0;
+#pragma unroll 1
+    for (int qb = q0; qb < q1; qb += D) {
+#pragma unroll
+      for (int j = 0; j < D; ++j) {
+        if (qb + j < q1) {
+          Quad<TB> v[4];
+          ring.take(qb + j, j, v);
+          const double c = coef[qb + j];
+#pragma unroll
+          for (int m = 0; m < 4; ++m)
+#pragma unroll
+            for (int t = 0; t < 4; ++t) sub[m][t] = fma(v[m][t], c, sub[m][t]);
+        }
+      }
+    }
+#pragma unroll
+    for (int m = 0; m < 4; ++m)
+#pragma unroll
+      for (int t = 0; t < 4; ++t) x[m][t] = __dsub_rn(x[m][t], sub[m][t]);
+  }
+}
+
+// pass 1 -----------------------------------------------------------------------
+template <typename TB, bool SPLIT>
+__global__ void __launch_bounds__(32 * warps_of(SPLIT), SPLIT ? 4 : (sizeof(TB) == 8 ? 2 : 3)) k_gs_dots(Batch b, GsArgs<TB> a) {
+  extern __shared__ __align__(16) unsigned char gs_sm[];
+  __shared__ double rowsum[SPLIT ? 1 : kRows][kMaxRestart + 1];
+  const Chunk ch = b.chunks[blockIdx.x];
+  if (!case_live(b, ch.cs, a.need)) return;
+  const size_t base = 4 * b.cases[ch.cs].cell_off + ch.begin;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, len = ch.len;
+  const int r = SPLIT ? blockIdx.y : warp;
+  const TB* V = a.V + base;
+  double* rs = rowsum[SPLIT ? 0 : r];
+  double wv[kChain];
+#pragma unroll
+  for (int m = 0; m < 4; ++m) {
+    double t[4];
+    load_w<TB>(a.w + base, r, m, lane, len, t);
+#pragma unroll
+    for (int u = 0; u < 4; ++u) wv[4 * m + u] = t[u];
+  }
+  if constexpr (SPLIT) {
+    project_row<TB>(
+        a.nq, warp, warps_of(true),
+        [&](Quad<TB>& v, int q, int m) { v.load(V + (size_t)q * a.vstride, r, m, lane, len); }, wv, rs);
+  } else {
+    Ring<TB> ring = ring_of<TB>(gs_sm, V, a, r, len);
+    project_ring(ring, wv, rs);
+  }
+  if (!SPLIT || warp == 0) {   // w . w
+    double n[1] = {0.0};
+#pragma unroll
+    for (int i = 0; i < kChain; ++i) n[0] = fma(wv[i], wv[i], n[0]);
+    const double s = warp_tree<1>(n);
+    if (lane == 0) rs[a.nq] = s;
+  }
+  store_chunk<SPLIT>(a.part + (size_t)blockIdx.x * a.pstride, rowsum, a.nq + 1);
+}
+
+// pass 2 -----------------------------------------------------------------------
+// A warp with a row of its own keeps the row's w' in registers and reads the basis again for
+// the projections, from L2.  With the row split over four warps, each subtracts a quarter of the
+// entries and projects on a quarter of the vectors, w' through shared memory; a BF16 row of
+// the vectors (1 KB each) is copied there too and read from there both times.
+template <typename TB>
+__host__ __device__ inline size_t gs_tile_bytes(int nq) {
+  return std::is_same<TB, double>::value ? 0 : (size_t)nq * 32 * kChain * sizeof(TB);
+}
+
+template <typename TB, bool SPLIT>
+__global__ void __launch_bounds__(32 * warps_of(SPLIT), SPLIT ? 4 : (sizeof(TB) == 8 ? 2 : 3)) k_gs_project(Batch b, GsArgs<TB> a) {
+  constexpr bool kTile = SPLIT && !std::is_same<TB, double>::value;
+  extern __shared__ __align__(16) unsigned char gs_sm[];
+  __shared__ double rowsum[SPLIT ? 1 : kRows][kMaxRestart + 1];
+  __shared__ double wp[SPLIT ? kChain * 32 : 1];   // w' of the row, [chain index][lane]
+  __shared__ double coef[kMaxRestart];
+  const Chunk ch = b.chunks[blockIdx.x];
+  if (!case_live(b, ch.cs, a.need)) return;
+  const CaseDev cs = b.cases[ch.cs];
+  const size_t base = 4 * cs.cell_off + ch.begin;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, len = ch.len, nq = a.nq;
+  const int r = SPLIT ? blockIdx.y : warp;
+  const TB* V = a.V + base;
+  double* rs = rowsum[SPLIT ? 0 : r];
+  auto global = [&](Quad<TB>& v, int q, int m) { v.load(V + (size_t)q * a.vstride, r, m, lane, len); };
+  uint2* tile = reinterpret_cast<uint2*>(gs_sm);   // [vector][quad m][lane]
+  if constexpr (kTile) {   // this thread's quad (m = warp) of every vector
+    const int e = Quad<TB>::at(r, warp, lane);
+    const uint32_t bytes = e < len ? 8u : 0u;
+    const TB* src = V + (e < len ? e : 0);
+    uint32_t dst = static_cast<uint32_t>(__cvta_generic_to_shared(tile + warp * 32 + lane));
+#pragma unroll 4
+    for (int q = 0; q < nq; ++q) {
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+      dst += 128 * sizeof(uint2);
+      src += a.vstride;
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  }
+  Ring<TB> ring = ring_of<TB>(gs_sm, V, a, r, len);
+  if constexpr (!SPLIT) ring.start();
+  coefficients<SPLIT>(a, cs, ch.cs, b.ncases, ch.begin == 0 && (!SPLIT || r == 0), coef, false);
+  double wv[kChain];
+  if constexpr (SPLIT) {
+    double x[4];
+    load_w<TB>(a.w + base, r, warp, lane, len, x);
+    if constexpr (kTile) {
+      asm volatile("cp.async.wait_all;" ::: "memory");
+      subtract<TB>(nq, [&](Quad<TB>& v, int q) { v.raw = tile[(size_t)q * 128 + warp * 32 + lane]; }, coef, x);
+    } else {
+      subtract<TB>(nq, [&](Quad<TB>& v, int q) { global(v, q, warp); }, coef, x);
+    }
+#pragma unroll
+    for (int t = 0; t < 4; ++t) wp[(4 * warp + t) * 32 + lane] = x[t];
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < kChain; ++i) wv[i] = wp[i * 32 + lane];
+  } else {
+    double x[4][4];
+#pragma unroll
+    for (int m = 0; m < 4; ++m) load_w<TB>(a.w + base, r, m, lane, len, x[m]);
+    subtract_ring(ring, coef, x);
+#pragma unroll
+    for (int i = 0; i < kChain; ++i) wv[i] = x[i / 4][i % 4];
+    project_ring(ring, wv, rs);
+  }
+  if constexpr (kTile) {
+    project_row<TB>(
+        nq, warp, warps_of(true),
+        [&](Quad<TB>& v, int q, int m) { v.raw = tile[(size_t)q * 128 + m * 32 + lane]; }, wv, rs);
+  } else if constexpr (SPLIT) {
+    project_row<TB>(nq, warp, warps_of(true), global, wv, rs);
+  }
+  store_chunk<SPLIT>(a.part + (size_t)blockIdx.x * a.pstride, rowsum, nq);
+}
+
+// pass 3 -----------------------------------------------------------------------
+template <typename TB, bool SPLIT>
+__global__ void __launch_bounds__(32 * warps_of(SPLIT), SPLIT ? 4 : (sizeof(TB) == 8 ? 2 : 3)) k_gs_sub(Batch b, GsArgs<TB> a) {
+  extern __shared__ __align__(16) unsigned char gs_sm[];
+  __shared__ double xs[SPLIT ? kChain * 32 : 1];   // w'' of the row, [chain index][lane]
+  __shared__ double rowsum[SPLIT ? 1 : kRows][kMaxRestart + 1];
+  __shared__ double coef[kMaxRestart];
+  constexpr int NM = SPLIT ? 1 : 4;                // quads of a lane
+  const Chunk ch = b.chunks[blockIdx.x];
+  if (!case_live(b, ch.cs, a.need)) return;
+  const CaseDev cs = b.cases[ch.cs];
+  const size_t base = 4 * cs.cell_off + ch.begin;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, len = ch.len;
+  const int r = SPLIT ? blockIdx.y : warp, m0 = SPLIT ? warp : 0;
+  const TB* V = a.V + base;
+  Ring<TB> ring = ring_of<TB>(gs_sm, V, a, r, len);
+  if constexpr (!SPLIT) ring.start();
+  coefficients<SPLIT>(a, cs, ch.cs, b.ncases, ch.begin == 0 && (!SPLIT || r == 0), coef, true);
+  double x[NM][4];
+#pragma unroll
+  for (int m = 0; m < NM; ++m) load_w<TB>(a.w + base, r, m0 + m, lane, len, x[m]);
+  if constexpr (SPLIT) {
+    subtract<TB>(a.nq, [&](Quad<TB>& v, int q) { v.load(V + (size_t)q * a.vstride, r, warp, lane, len); }, coef, x[0]);
+  } else {
+    subtract_ring(ring, coef, x);
+  }
+#pragma unroll
+  for (int m = 0; m < NM; ++m) store_quad(a.Vout + base, r, m0 + m, lane, len, x[m]);
+  double n[1] = {0.0};
+  if constexpr (SPLIT) {
+#pragma unroll
+    for (int t = 0; t < 4; ++t) xs[(4 * warp + t) * 32 + lane] = x[0][t];
+    __syncthreads();
+    if (warp == 0) {
+#pragma unroll
+      for (int i = 0; i < kChain; ++i) {
+        const double y = xs[i * 32 + lane];
+        n[0] = fma(y, y, n[0]);
+      }
+    }
+  } else {
+#pragma unroll
+    for (int m = 0; m < NM; ++m)
+#pragma unroll
+      for (int t = 0; t < 4; ++t) n[0] = fma(x[m][t], x[m][t], n[0]);
+  }
+  if (!SPLIT || warp == 0) {
+    const double s = warp_tree<1>(n);
+    if (lane == 0) rowsum[SPLIT ? 0 : r][0] = s;
+  }
+  store_chunk<SPLIT>(a.part_norm + blockIdx.x, rowsum, 1);
+}
+
+// start vector: V_raw[0] = r and its squared norm ------------------------------
+constexpr int kGB = 256;                 // threads per block
+constexpr int kGE = kChunk / kGB;        // entries per thread
+
 __device__ __forceinline__ void ldv(const double* p, double (&v)[4]) {
   const double2 t0 = *reinterpret_cast<const double2*>(p);
   const double2 t1 = *reinterpret_cast<const double2*>(p + 2);
   v[0] = t0.x; v[1] = t0.y; v[2] = t1.x; v[3] = t1.y;
 }
-__device__ __forceinline__ void ldv(const float* p, double (&v)[2]) {
-  const float2 t = *reinterpret_cast<const float2*>(p);
-  v[0] = t.x; v[1] = t.y;
-}
-__device__ __forceinline__ void ldv(const double* p, double (&v)[2]) {
-  const double2 t = *reinterpret_cast<const double2*>(p);
-  v[0] = t.x; v[1] = t.y;
-}
-__device__ __forceinline__ void stv(float* p, const double (&v)[4]) {
-  *reinterpret_cast<float4*>(p) = make_float4((float)v[0], (float)v[1], (float)v[2], (float)v[3]);
-}
 __device__ __forceinline__ void stv(double* p, const double (&v)[4]) {
   *reinterpret_cast<double2*>(p) = make_double2(v[0], v[1]);
   *reinterpret_cast<double2*>(p + 2) = make_double2(v[2], v[3]);
 }
-// one basis entry in FP64, and back in its storage precision
-__device__ __forceinline__ double entry_f64(double v) { return v; }
-__device__ __forceinline__ double entry_f64(float v) { return v; }
-__device__ __forceinline__ double entry_f64(__nv_bfloat16 v) { return __bfloat162float(v); }
-template <typename TB> __device__ __forceinline__ TB to_basis(double x) { return TB(x); }
-template <> __device__ __forceinline__ __nv_bfloat16 to_basis<__nv_bfloat16>(double x) {
-  return __float2bfloat16_rn((float)x);
-}
-
 __device__ __forceinline__ void stv(__nv_bfloat16* p, const double (&v)[4]) {
   __nv_bfloat162 lo = __floats2bfloat162_rn((float)v[0], (float)v[1]);
   __nv_bfloat162 hi = __floats2bfloat162_rn((float)v[2], (float)v[3]);
-  uint2 raw;
-  raw.x = *reinterpret_cast<uint32_t*>(&lo);
-  raw.y = *reinterpret_cast<uint32_t*>(&hi);
-  *reinterpret_cast<uint2*>(p) = raw;
+  *reinterpret_cast<uint2*>(p) = make_uint2(*reinterpret_cast<uint32_t*>(&lo), *reinterpret_cast<uint32_t*>(&hi));
 }
 
-// ---------------------------------------------------------------------------
-// streaming passes.  A CTA of kGT threads owns one chunk and walks it in
-// sub-tiles of E entries; the E entries of w and of every basis vector of the
-// slice for one sub-tile (one stage) arrive by bulk copies on one mbarrier,
-// through a ring of as many stages as the shared-memory budget holds, issued
-// by thread 0 as soon as a stage is free.  The BF16 basis takes a smaller budget
-// than the others, so that more CTAs fit on an SM (measured at 64 cases: resident
-// CTAs hide the bulk copies better than a deeper ring).  Thread t works on entries
-// t*EPT .. t*EPT+EPT-1 of each sub-tile and keeps one partial sum per basis
-// vector in registers (NQ >= nq of them, a template tier); the chunk ends with
-// one fixed-order block reduction, so the result does not depend on which
-// other cases share the batch.
-// ---------------------------------------------------------------------------
-constexpr int kGT = 256;
-constexpr int kGsMaxStages = 8;
-constexpr size_t kGsSmemBudget = 74 * 1024;     // three CTAs per SM
-constexpr int kGsHeader = 128;                  // mbarriers and abort flags before the stages
-
-template <typename TB> struct GsTile;
-// 2 KB runs of every basis vector per stage (measured: larger runs beat deeper
-// rings; three CTAs per SM beat one CTA with more stages)
-template <> struct GsTile<float> { static constexpr int E = 512; };
-template <> struct GsTile<double> { static constexpr int E = 256; };
-template <> struct GsTile<__nv_bfloat16> { static constexpr int E = 1024; };
-
-template <typename TB>
-__host__ __device__ inline uint32_t gs_stage_bytes(int nq) {
-  return (uint32_t)GsTile<TB>::E * (uint32_t)(nq * sizeof(TB) + 8);
-}
-static_assert(kGsSmemBudget >= (size_t)GsTile<float>::E * (32 * 4 + 8) &&
-                  kGsSmemBudget >= (size_t)GsTile<double>::E * (32 * 8 + 8) &&
-                  kGsSmemBudget >= (size_t)GsTile<__nv_bfloat16>::E * (32 * 2 + 8),
-              "one stage of a 32-vector slice must fit the shared-memory budget");
-
-// shared-memory budget of the ring: 40 KB for the BF16 basis (slices of up to 13
-// vectors keep 2 stages or more, larger ones one stage and four or five CTAs per SM)
-template <typename TB>
-__host__ __device__ constexpr size_t gs_budget() {
-  return std::is_same<TB, __nv_bfloat16>::value ? 40 * 1024 : kGsSmemBudget;
-}
-
-template <typename TB>
-__host__ __device__ inline int gs_stages(int nq) {
-  const int s = (int)(gs_budget<TB>() / gs_stage_bytes<TB>(nq));
-  return s < 1 ? 1 : (s > kGsMaxStages ? kGsMaxStages : s);
-}
-
-// fixed-order reduction of NV values over the kGT threads; thread t < NV receives value t
-template <int NV>
-__device__ __forceinline__ double gs_block_reduce(double (&v)[NV], double* scratch /* (kGT/32)*NV */) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-  for (int q = 0; q < NV; ++q) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v[q] += __shfl_down_sync(0xffffffffu, v[q], o);
-  }
-  __syncthreads();   // the scratch may alias the last stage, still read above
-  if (lane == 0) {
-#pragma unroll
-    for (int q = 0; q < NV; ++q) scratch[warp * NV + q] = v[q];
-  }
-  __syncthreads();
-  double s = 0.0;
-  if (threadIdx.x < NV) {
-#pragma unroll
-    for (int w = 0; w < kGT / 32; ++w) s += scratch[w * NV + threadIdx.x];
-  }
-  return s;
-}
-
-// EPT consecutive entries in their storage precision, from shared memory
-template <typename TB, int EPT> struct VecOf;
-template <> struct VecOf<float, 1> { using type = float; };
-template <> struct VecOf<float, 2> { using type = float2; };
-template <> struct VecOf<float, 4> { using type = float4; };
-template <> struct VecOf<double, 1> { using type = double; };
-template <> struct VecOf<double, 2> { using type = double2; };
-struct alignas(16) Double4x { double2 lo, hi; };
-template <> struct VecOf<double, 4> { using type = Double4x; };
-template <> struct VecOf<__nv_bfloat16, 1> { using type = __nv_bfloat16; };
-template <> struct VecOf<__nv_bfloat16, 2> { using type = __nv_bfloat162; };
-struct alignas(8) Bf16x4 { __nv_bfloat162 lo, hi; };
-template <> struct VecOf<__nv_bfloat16, 4> { using type = Bf16x4; };
-
-template <typename TB, int EPT>
-struct Entries {
-  alignas(sizeof(typename VecOf<TB, EPT>::type)) TB v[EPT];
-  __device__ __forceinline__ void load(const TB* p) {
-    using V = typename VecOf<TB, EPT>::type;
-    *reinterpret_cast<V*>(v) = *reinterpret_cast<const V*>(p);
-  }
-  __device__ __forceinline__ double operator[](int u) const { return entry_f64(v[u]); }
-};
-
-// the ring of one streaming pass over a chunk
-template <typename TB>
-struct GsRing {
-  static constexpr int E = GsTile<TB>::E;
-  static constexpr int EPT = E / kGT;
-  unsigned char* stages;
-  uint64_t* full;
-  int* abort;
-  int S, nq, len, nsub;
-  uint32_t stage_bytes;
-  const TB* V;        // first vector of the slice, at the chunk's first entry
-  size_t vstride;
-  const double* w;    // at the chunk's first entry
-  uint64_t pol;       // L2 policy of the basis runs: evict first, so that w (re-read by the
-                      // three passes of an Arnoldi step) stays in L2
-
-  __device__ void init(unsigned char* smem, const GsArgs<TB>& a, const Chunk& ch, size_t base) {
-    full = reinterpret_cast<uint64_t*>(smem);
-    abort = reinterpret_cast<int*>(smem + 8 * kGsMaxStages);
-    stages = smem + kGsHeader;
-    nq = a.nq;
-    S = gs_stages<TB>(nq);
-    stage_bytes = gs_stage_bytes<TB>(nq);
-    len = ch.len;
-    nsub = (len + E - 1) / E;
-    V = a.V + (size_t)a.q0 * a.vstride + base;
-    vstride = a.vstride;
-    w = a.w + base;
-    pol = l2_evict_first();
-    if (threadIdx.x == 0) {
-      for (int s = 0; s < S; ++s) mbar_init(&full[s], 1);
-      mbar_init_fence();
-      abort[0] = abort[1] = 0;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0)
-      for (int u = 0; u < S; ++u) issue(u);
-  }
-  // sub-tile u: entries u*E .. of the chunk (len is a multiple of 4 entries, so
-  // every copy is a multiple of 16 bytes)
-  __device__ void issue(int u) const {
-    if (u >= nsub) return;
-    const int e0 = u * E;
-    const int n = min(E, len - e0);
-    const int s = u % S;
-    unsigned char* st = stages + (size_t)s * stage_bytes;
-    mbar_arrive_expect(&full[s], (uint32_t)n * (uint32_t)(nq * sizeof(TB) + 8));
-    for (int q = 0; q < nq; ++q)
-      bulk_load_hint(st + (size_t)q * E * sizeof(TB), V + (size_t)q * vstride + e0, n * sizeof(TB), &full[s], pol);
-    bulk_load(st + (size_t)nq * E * sizeof(TB), w + e0, n * 8, &full[s]);
-  }
-  __device__ const TB* vec(int u, int q) const {
-    return reinterpret_cast<const TB*>(stages + (size_t)(u % S) * stage_bytes) + (size_t)q * E;
-  }
-  __device__ const double* wvec(int u) const {
-    return reinterpret_cast<const double*>(stages + (size_t)(u % S) * stage_bytes + (size_t)nq * E * sizeof(TB));
-  }
-  __device__ void wait(int u) const {
-    if (!mbar_wait(&full[u % S], (u / S) & 1)) abort[u & 1] = 1;
-  }
-  // after consuming sub-tile u: frees its stage; false once a wait has run out
-  __device__ bool release(int u) const {
-    __syncthreads();
-    if (abort[u & 1]) return false;
-    if (threadIdx.x == 0) issue(u + S);
-    return true;
-  }
-  // error exit: record the failure and give the copies in flight a bounded time
-  __device__ void drain(int u, uint32_t* err) const {
-    if (threadIdx.x == 0) {
-      if (err != nullptr) atomicExch(err, 1u);
-      for (int v = u; v < u + S && v < nsub; ++v) (void)mbar_wait(&full[v % S], (v / S) & 1);
-    }
-    __syncthreads();
-  }
-};
-
-// pass 1 (and the re-projection of the chained path) ---------------------------
-template <typename TB, int NQ>
-__global__ void __launch_bounds__(kGT) k_gs_dots(Batch b, GsArgs<TB> a) {
-  extern __shared__ __align__(128) unsigned char smem[];
-  const Chunk ch = b.chunks[blockIdx.x];
-  if (!case_live(b, ch.cs, a.need)) return;
-  const CaseDev cs = b.cases[ch.cs];
-  GsRing<TB> ring;
-  ring.init(smem, a, ch, 4 * cs.cell_off + ch.begin);
-  constexpr int EPT = GsRing<TB>::EPT;
-  double acc[NQ + 1];
-#pragma unroll
-  for (int q = 0; q <= NQ; ++q) acc[q] = 0.0;
-  const int nq = a.nq;
-#pragma unroll 1
-  for (int u = 0; u < ring.nsub; ++u) {
-    ring.wait(u);
-    const int e = threadIdx.x * EPT;
-    if (e < ring.len - u * GsRing<TB>::E) {
-      const double* ws = ring.wvec(u) + e;
-      double w[EPT];
-#pragma unroll
-      for (int t = 0; t < EPT; ++t) w[t] = ws[t];
-#pragma unroll
-      for (int q = 0; q < NQ; ++q) {
-        Entries<TB, EPT> v;
-        v.load(ring.vec(u, q < nq ? q : nq - 1) + e);
-        if (q < nq) {
-#pragma unroll
-          for (int t = 0; t < EPT; ++t) acc[q] += v[t] * w[t];
-        }
-      }
-#pragma unroll
-      for (int t = 0; t < EPT; ++t) acc[NQ] += w[t] * w[t];
-    }
-    if (!ring.release(u)) {
-      ring.drain(u, a.err);
-      return;
-    }
-  }
-  const double r = gs_block_reduce<NQ + 1>(acc, reinterpret_cast<double*>(ring.stages));
-  double* part = a.part + (size_t)blockIdx.x * a.pstride;
-  if (threadIdx.x < nq) part[a.q0 + threadIdx.x] = r;
-  if (a.with_norm && threadIdx.x == NQ) part[a.norm_slot] = r;
-}
-
-// pass 2, fused: w' = w - V (s h1), then V . w' --------------------------------
-template <typename TB, int NQ>
-__global__ void __launch_bounds__(kGT, (NQ == 24 && std::is_same<TB, __nv_bfloat16>::value) ? 3 : 0)
-    k_gs_project(Batch b, GsArgs<TB> a) {
-  extern __shared__ __align__(128) unsigned char smem[];
-  __shared__ double coef[NQ];
-  const Chunk ch = b.chunks[blockIdx.x];
-  if (!case_live(b, ch.cs, a.need)) return;
-  const CaseDev cs = b.cases[ch.cs];
-  GsRing<TB> ring;
-  ring.init(smem, a, ch, 4 * cs.cell_off + ch.begin);   // the first bulk copies go out first
-  if (a.fold_part != nullptr) coef_folded(a, cs, ch.cs, b.ncases, ch.begin == 0, coef, false);
-  else coef_to_smem(a, ch.cs, b.ncases, coef, false);
-  constexpr int EPT = GsRing<TB>::EPT;
-  double acc[NQ];
-#pragma unroll
-  for (int q = 0; q < NQ; ++q) acc[q] = 0.0;
-  const int nq = a.nq;
-#pragma unroll 1
-  for (int u = 0; u < ring.nsub; ++u) {
-    ring.wait(u);
-    const int e = threadIdx.x * EPT;
-    if (e < ring.len - u * GsRing<TB>::E) {
-      const double* ws = ring.wvec(u) + e;
-      double sub[EPT];
-#pragma unroll
-      for (int t = 0; t < EPT; ++t) sub[t] = 0.0;
-#pragma unroll
-      for (int q = 0; q < NQ; ++q) {
-        Entries<TB, EPT> v;
-        v.load(ring.vec(u, q < nq ? q : nq - 1) + e);
-        if (q < nq) {
-#pragma unroll
-          for (int t = 0; t < EPT; ++t) sub[t] += v[t] * coef[q];
-        }
-      }
-      double wp[EPT];
-#pragma unroll
-      for (int t = 0; t < EPT; ++t) wp[t] = ws[t] - sub[t];
-#pragma unroll
-      for (int q = 0; q < NQ; ++q) {
-        Entries<TB, EPT> v;
-        v.load(ring.vec(u, q < nq ? q : nq - 1) + e);
-        if (q < nq) {
-#pragma unroll
-          for (int t = 0; t < EPT; ++t) acc[q] += v[t] * wp[t];
-        }
-      }
-    }
-    if (!ring.release(u)) {
-      ring.drain(u, a.err);
-      return;
-    }
-  }
-  const double r = gs_block_reduce<NQ>(acc, reinterpret_cast<double*>(ring.stages));
-  if (threadIdx.x < nq) a.part[(size_t)blockIdx.x * a.pstride + threadIdx.x] = r;
-}
-
-// out = in - V (s h): pass 3, and the subtraction slices of the chained path ----
-template <typename TB, int NQ>
-__global__ void __launch_bounds__(kGT) k_gs_sub(Batch b, GsArgs<TB> a) {
-  extern __shared__ __align__(128) unsigned char smem[];
-  __shared__ double coef[NQ];
-  const Chunk ch = b.chunks[blockIdx.x];
-  if (!case_live(b, ch.cs, a.need)) return;
-  const CaseDev cs = b.cases[ch.cs];
-  const size_t base = 4 * cs.cell_off + ch.begin;
-  GsRing<TB> ring;
-  ring.init(smem, a, ch, base);   // the first bulk copies go out first
-  if (a.fold_part != nullptr) coef_folded(a, cs, ch.cs, b.ncases, ch.begin == 0, coef, a.both != 0);
-  else coef_to_smem(a, ch.cs, b.ncases, coef, a.both != 0);
-  constexpr int EPT = GsRing<TB>::EPT;
-  constexpr int E = GsRing<TB>::E;
-  const int nq = a.nq;
-  double nrm = 0.0;
-#pragma unroll 1
-  for (int u = 0; u < ring.nsub; ++u) {
-    ring.wait(u);
-    const int e = threadIdx.x * EPT;
-    if (e < ring.len - u * E) {
-      const double* ws = ring.wvec(u) + e;
-      double sub[EPT];
-#pragma unroll
-      for (int t = 0; t < EPT; ++t) sub[t] = 0.0;
-#pragma unroll
-      for (int q = 0; q < NQ; ++q) {
-        Entries<TB, EPT> v;
-        v.load(ring.vec(u, q < nq ? q : nq - 1) + e);
-        if (q < nq) {
-#pragma unroll
-          for (int t = 0; t < EPT; ++t) sub[t] += v[t] * coef[q];
-        }
-      }
-      const size_t g = base + (size_t)u * E + e;
-#pragma unroll
-      for (int t = 0; t < EPT; ++t) {
-        const double x = ws[t] - sub[t];
-        nrm += x * x;
-        if (a.wout != nullptr) a.wout[g + t] = x;
-        if (a.Vout != nullptr) a.Vout[g + t] = to_basis<TB>(x);
-      }
-    }
-    if (!ring.release(u)) {
-      ring.drain(u, a.err);
-      return;
-    }
-  }
-  if (a.part_norm != nullptr) {
-    double v[1] = {nrm};
-    const double r = gs_block_reduce<1>(v, reinterpret_cast<double*>(ring.stages));
-    if (threadIdx.x == 0) a.part_norm[blockIdx.x] = r;
-  }
-}
-
-// start vector: V_raw[0] = r and its squared norm ------------------------------
 template <typename TB>
 __global__ void __launch_bounds__(kGB) k_gs_start(Batch b, GsArgs<TB> a) {
   const Chunk ch = b.chunks[blockIdx.x];
@@ -486,6 +597,7 @@ __global__ void __launch_bounds__(kGB) k_gs_start(Batch b, GsArgs<TB> a) {
   const CaseDev cs = b.cases[ch.cs];
   const size_t base = 4 * cs.cell_off + ch.begin;
   __shared__ double scratch[8];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   double nrm = 0.0;
 #pragma unroll
   for (int s = 0; s < kGE / 4; ++s) {
@@ -498,26 +610,14 @@ __global__ void __launch_bounds__(kGB) k_gs_start(Batch b, GsArgs<TB> a) {
       for (int u = 0; u < 4; ++u) nrm += x[u] * x[u];
     }
   }
-  double v[1] = {nrm};
-  const double r = gs_reduce_to_thread<1>(v, scratch);
-  if (threadIdx.x == 0) a.part_norm[blockIdx.x] = r;
-}
-
-// sum over a case's chunks of one partial, by one warp: lane c takes chunks
-// c, c+32, ... in order, then a fixed butterfly; every lane gets the total
-// per-case reduction of the chunk partials: one block per case, one warp per coefficient
-__global__ void __launch_bounds__(256) k_gs_reduce(Batch b, GsReduceArgs a) {
-  const int cs_id = blockIdx.x;
-  if (!case_live(b, cs_id, a.need)) return;
-  const CaseDev cs = b.cases[cs_id];
-  const int nred = a.nq + (a.wn0 != nullptr ? 1 : 0);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  for (int q = warp; q < nred; q += blockDim.x >> 5) {
-    const double s = warp_chunk_sum(a.part + (size_t)cs.chunk0 * a.pstride + q, a.pstride, cs.nchunks);
-    if (lane == 0) {
-      if (q < a.nq) a.h[(size_t)cs_id * kHStride + q] = s * a.scale[(size_t)q * b.ncases + cs_id];
-      else a.wn0[cs_id] = sqrt(s);
-    }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) nrm += __shfl_down_sync(0xffffffffu, nrm, o);
+  if (lane == 0) scratch[warp] = nrm;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double s = 0.0;
+    for (int w = 0; w < kGB / 32; ++w) s += scratch[w];
+    a.part_norm[blockIdx.x] = s;
   }
 }
 
@@ -558,85 +658,53 @@ __global__ void __launch_bounds__(32) k_gs_close(Batch b, GsCloseArgs a) {
 }
 
 // ---------------------------------------------------------------------------
-// host side: tier dispatch and the chained path for more than 32 vectors
+// host side
 // ---------------------------------------------------------------------------
-constexpr int kSlice = kGsSlice;
+// whether the rows of a chunk go to CTAs of their own, eight CTAs for one: with at most half the
+// SMs' number of chunks the GPU is idle otherwise (27 vectors, BF16, passes 1 / 2 / 3 in us,
+// split against whole: 48 chunks 8 / 14 / 12 against 10 / 21 / 15; 128 chunks 13 / 25 / 23
+// against 10 / 21 / 17, every CTA reducing the coefficients once more)
+static bool gs_split(int nchunks) { return nchunks <= 148 / 2; }
 
-#define A2D_GS_DISPATCH(KERNEL)                                                              \
-  template <typename TB>                                                                     \
-  static void dispatch_##KERNEL(const Batch& b, const GsArgs<TB>& a, cudaStream_t s) {       \
-    if (!b.nchunks) return;                                                                  \
-    const size_t smem = kGsHeader + (size_t)gs_stages<TB>(a.nq) * gs_stage_bytes<TB>(a.nq);  \
-    if (a.nq <= 8) KERNEL<TB, 8><<<b.nchunks, kGT, smem, s>>>(b, a);                          \
-    else if (a.nq <= 16) KERNEL<TB, 16><<<b.nchunks, kGT, smem, s>>>(b, a);                   \
-    else if (a.nq <= 24) KERNEL<TB, 24><<<b.nchunks, kGT, smem, s>>>(b, a);                   \
-    else KERNEL<TB, 32><<<b.nchunks, kGT, smem, s>>>(b, a);                                   \
-  }
-A2D_GS_DISPATCH(k_gs_dots)
-A2D_GS_DISPATCH(k_gs_project)
-A2D_GS_DISPATCH(k_gs_sub)
-#undef A2D_GS_DISPATCH
-
+// a pass over every chunk: with the chunks' rows on CTAs of their own (whole = false), the rows
+// of a chunk are a cluster
 template <typename TB>
-void launch_gs_dots(const Batch& b, const GsArgs<TB>& a0, cudaStream_t s) {
-  GsArgs<TB> a = a0;
-  a.norm_slot = a0.nq;
-  for (int q0 = 0; q0 < a0.nq; q0 += kSlice) {
-    a.q0 = q0;
-    a.nq = a0.nq - q0 < kSlice ? a0.nq - q0 : kSlice;
-    a.with_norm = a0.with_norm && q0 == 0;
-    dispatch_k_gs_dots<TB>(b, a, s);
-  }
-}
-
-template <typename TB>
-void launch_gs_project(const Batch& b, const GsArgs<TB>& a0, cudaStream_t s) {
-  if (a0.nq <= kSlice) {
-    GsArgs<TB> a = a0;
-    a.q0 = 0;
-    dispatch_k_gs_project<TB>(b, a, s);
+static void launch_pass(void (*split)(Batch, GsArgs<TB>), void (*whole)(Batch, GsArgs<TB>), size_t split_smem,
+                        const Batch& b, const GsArgs<TB>& a, cudaStream_t s) {
+  if (!b.nchunks) return;
+  if (!gs_split(b.nchunks)) {
+    whole<<<b.nchunks, 32 * warps_of(false), kRows * Ring<TB>::kBytes, s>>>(b, a);
     return;
   }
-  // chained: w' = w - V (s h1) into the scratch vector, then its projections
-  GsArgs<TB> a = a0;
-  a.both = 0;
-  a.Vout = nullptr;
-  a.part_norm = nullptr;
-  for (int q0 = 0; q0 < a0.nq; q0 += kSlice) {
-    a.q0 = q0;
-    a.nq = a0.nq - q0 < kSlice ? a0.nq - q0 : kSlice;
-    a.w = q0 == 0 ? a0.w : a0.tmp;
-    a.wout = a0.tmp;
-    dispatch_k_gs_sub<TB>(b, a, s);
-  }
-  GsArgs<TB> d = a0;
-  d.w = a0.tmp;
-  d.with_norm = 0;
-  launch_gs_dots<TB>(b, d, s);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(b.nchunks, kRows);
+  cfg.blockDim = dim3(32 * warps_of(true));
+  cfg.dynamicSmemBytes = split_smem;
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = 1;
+  at[0].val.clusterDim.y = kRows;
+  at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  (void)cudaLaunchKernelEx(&cfg, split, b, a);   // as <<<>>>: see cudaGetLastError
 }
-
 template <typename TB>
-void launch_gs_finish(const Batch& b, const GsArgs<TB>& a0, cudaStream_t s) {
-  GsArgs<TB> a = a0;
-  a.both = 1;
-  for (int q0 = 0; q0 < a0.nq; q0 += kSlice) {
-    const bool last = q0 + kSlice >= a0.nq;
-    a.q0 = q0;
-    a.nq = a0.nq - q0 < kSlice ? a0.nq - q0 : kSlice;
-    a.w = q0 == 0 ? a0.w : a0.tmp;
-    a.wout = last ? nullptr : a0.tmp;
-    a.Vout = last ? a0.Vout : nullptr;
-    a.part_norm = last ? a0.part_norm : nullptr;
-    dispatch_k_gs_sub<TB>(b, a, s);
-  }
+void launch_gs_dots(const Batch& b, const GsArgs<TB>& a, cudaStream_t s) {
+  launch_pass<TB>(k_gs_dots<TB, true>, k_gs_dots<TB, false>, 0, b, a, s);
 }
-
+template <typename TB>
+void launch_gs_project(const Batch& b, const GsArgs<TB>& a, cudaStream_t s) {
+  launch_pass<TB>(k_gs_project<TB, true>, k_gs_project<TB, false>, gs_tile_bytes<TB>(a.nq), b, a, s);
+}
+template <typename TB>
+void launch_gs_finish(const Batch& b, const GsArgs<TB>& a, cudaStream_t s) {
+  launch_pass<TB>(k_gs_sub<TB, true>, k_gs_sub<TB, false>, 0, b, a, s);
+}
 template <typename TB>
 void launch_gs_start(const Batch& b, const GsArgs<TB>& a, cudaStream_t s) {
   if (b.nchunks) k_gs_start<TB><<<b.nchunks, kGB, 0, s>>>(b, a);
-}
-void launch_gs_reduce(const Batch& b, const GsReduceArgs& a, cudaStream_t s) {
-  if (b.ncases) k_gs_reduce<<<b.ncases, 256, 0, s>>>(b, a);
 }
 void launch_gs_close(const Batch& b, const GsCloseArgs& a, cudaStream_t s) {
   if (b.ncases) k_gs_close<<<b.ncases, 32, 0, s>>>(b, a);
@@ -648,24 +716,21 @@ void launch_gs_close(const Batch& b, const GsCloseArgs& a, cudaStream_t s) {
   template void launch_gs_finish<TB>(const Batch&, const GsArgs<TB>&, cudaStream_t);   \
   template void launch_gs_start<TB>(const Batch&, const GsArgs<TB>&, cudaStream_t);
 A2D_GS_INST(double)
-A2D_GS_INST(float)
 A2D_GS_INST(__nv_bfloat16)
 #undef A2D_GS_INST
 
 cudaError_t gs_init() {
   cudaError_t e = cudaSuccess;
-  const int bytes = (int)(kGsHeader + kGsSmemBudget);
-  auto set = [&](const void* f) {
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  auto set = [&](const void* f, size_t bytes) {
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
   };
-#define A2D_GS_ATTR(TB, NQ)                                            \
-  set(reinterpret_cast<const void*>(&k_gs_dots<TB, NQ>));              \
-  set(reinterpret_cast<const void*>(&k_gs_project<TB, NQ>));           \
-  set(reinterpret_cast<const void*>(&k_gs_sub<TB, NQ>));
-  A2D_GS_ATTR(float, 8) A2D_GS_ATTR(float, 16) A2D_GS_ATTR(float, 24) A2D_GS_ATTR(float, 32)
-  A2D_GS_ATTR(double, 8) A2D_GS_ATTR(double, 16) A2D_GS_ATTR(double, 24) A2D_GS_ATTR(double, 32)
-  A2D_GS_ATTR(__nv_bfloat16, 8) A2D_GS_ATTR(__nv_bfloat16, 16) A2D_GS_ATTR(__nv_bfloat16, 24)
-  A2D_GS_ATTR(__nv_bfloat16, 32)
+  set(reinterpret_cast<const void*>(&k_gs_project<__nv_bfloat16, true>), gs_tile_bytes<__nv_bfloat16>(kMaxRestart));
+#define A2D_GS_ATTR(TB)                                                                       \
+  set(reinterpret_cast<const void*>(&k_gs_dots<TB, false>), kRows * Ring<TB>::kBytes);       \
+  set(reinterpret_cast<const void*>(&k_gs_project<TB, false>), kRows * Ring<TB>::kBytes);    \
+  set(reinterpret_cast<const void*>(&k_gs_sub<TB, false>), kRows * Ring<TB>::kBytes);
+  A2D_GS_ATTR(double)
+  A2D_GS_ATTR(__nv_bfloat16)
 #undef A2D_GS_ATTR
   return e;
 }

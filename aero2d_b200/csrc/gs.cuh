@@ -8,47 +8,26 @@
 namespace a2d {
 
 constexpr int kHStride = kMaxRestart + 2;   // per-case stride of coefficient arrays
-constexpr int kGsSlice = 32;                // basis vectors one pass handles (more: chained slices)
+constexpr int kGsRows = 8;                  // rows of a chunk (gs.cu)
 
 template <typename TB>
 struct GsArgs {
   const double* w = nullptr;      // vector being orthogonalised
   const TB* V = nullptr;          // raw basis, vector q at V + q * vstride
   size_t vstride = 0;
-  int nq = 0;                     // basis vectors taken
-  int q0 = 0;                     // first vector of the slice (set by the launchers)
-  int with_norm = 0;              // pass 1: also w . w
-  int norm_slot = 0;              // partial slot of w . w (set by the launchers)
-  double* part = nullptr;         // per-chunk partials [chunk][pstride]
+  int nq = 0;                     // basis vectors taken (at most kMaxRestart)
+  double* part = nullptr;         // pass 1, 2: partials [chunk][pstride], slot q; pass 1 also w . w in slot nq
   int pstride = 0;
-  const double* h1 = nullptr;     // [case][kHStride] coefficients of pass 1
-  const double* h2 = nullptr;     // [case][kHStride] coefficients of pass 2
-  const double* scale = nullptr;  // [q][case] scale of raw basis vector q
-  int both = 0;                   // subtraction uses h1 + h2
-  TB* Vout = nullptr;             // pass 3 / start: raw basis vector written
-  double* wout = nullptr;         // subtraction result kept in FP64 (chained path)
-  double* tmp = nullptr;          // scratch vector of the chained path (more than 32 vectors)
-  double* part_norm = nullptr;    // per-chunk squared norm of the result
-  uint32_t* err = nullptr;        // set to 1 when a bulk-copy wait runs out of time
-  uint32_t need = 0;
-  // Folded per-case reduction (one slice, nq <= 32): when fold_part is set, every CTA
-  // reduces its case's chunk partials fold_part[chunk][q] itself (the order of
-  // k_gs_reduce) into this pass's coefficients, h_q = scale_q * sum, while its first
-  // bulk copies are in flight; the case's first chunk also stores h in fold_h (and, with
-  // fold_wn0, the norm of w from the partials' slot nq).  project: the coefficients are
-  // h1; sub (both): h1 from h1 plus the folded h2.
+  // pass 2 and 3: the partials of the pass before, which every CTA reduces over its case's chunks
+  // itself into h_q = scale_q * sum; the case's first CTA stores h in fold_h (and, with
+  // fold_wn0, the norm of w from slot nq).  Pass 3 subtracts with h1 + h
   const double* fold_part = nullptr;
   double* fold_h = nullptr;
   double* fold_wn0 = nullptr;
-};
-
-struct GsReduceArgs {
-  const double* part = nullptr;
-  int pstride = 0;
-  int nq = 0;
-  const double* scale = nullptr;  // [q][case]
-  double* h = nullptr;            // [case][kHStride]
-  double* wn0 = nullptr;          // if set: sqrt of slot nq (norm of w before orthogonalisation)
+  const double* h1 = nullptr;     // [case][kHStride] coefficients of pass 1
+  const double* scale = nullptr;  // [q][case] scale of raw basis vector q
+  TB* Vout = nullptr;             // pass 3 / start: raw basis vector written
+  double* part_norm = nullptr;    // pass 3, start: squared norm per chunk
   uint32_t need = 0;
 };
 
@@ -66,12 +45,11 @@ struct GsCloseArgs {
 };
 
 template <typename TB> void launch_gs_dots(const Batch& b, const GsArgs<TB>& a, cudaStream_t s);
-void launch_gs_reduce(const Batch& b, const GsReduceArgs& a, cudaStream_t s);
 template <typename TB> void launch_gs_project(const Batch& b, const GsArgs<TB>& a, cudaStream_t s);
 template <typename TB> void launch_gs_finish(const Batch& b, const GsArgs<TB>& a, cudaStream_t s);
 template <typename TB> void launch_gs_start(const Batch& b, const GsArgs<TB>& a, cudaStream_t s);
 void launch_gs_close(const Batch& b, const GsCloseArgs& a, cudaStream_t s);
-// raises the dynamic shared-memory limit of the streaming passes (host, once per device)
+// raises the dynamic shared-memory limit of the passes (host, once per device)
 cudaError_t gs_init();
 
 }  // namespace a2d

@@ -229,7 +229,7 @@ static void layout(a2d_plan* P) {
   P->o_tpart = cv.take(8 * kTilePartStride * P->tiles.size());
   P->pstride = P->m + 2;
   P->o_cpart = cv.take(8 * (size_t)P->pstride * P->chunks.size());
-  P->o_cpart2 = cv.take(8 * (size_t)P->pstride * P->chunks.size());   // pass-2 partials of the folded path
+  P->o_cpart2 = cv.take(8 * (size_t)P->pstride * P->chunks.size());   // pass 2's, while pass 1's are read
   P->o_cpartn = cv.take(8 * P->chunks.size());
   P->o_coef = cv.take(8 * 3 * (size_t)B);
   P->o_cp = cv.take(8 * (size_t)P->total_ni);
@@ -567,53 +567,32 @@ static void newton_step_launches(a2d_plan* P, cudaStream_t s) {
     za.need = KR;
     launch_jvp<TV, TB>(P, za, s);
     precond<TJ>(P, B, z, w, KR, s);
-    // classical Gram-Schmidt run twice, three passes over the basis
+    // classical Gram-Schmidt run twice, three passes over the basis; passes 2 and 3 reduce
+    // the partials of the pass before, so pass 2 writes its own to a second buffer
     GsArgs<TB> g;
-    g.err = P->at<uint32_t>(P->o_cnt) + 1;
     g.w = w;
     g.V = V;
     g.vstride = vs;
     g.nq = k + 1;
-    g.part = cpart;
     g.pstride = P->pstride;
-    g.h1 = h1;
-    g.h2 = h2;
     g.scale = scale;
-    g.Vout = V + (size_t)(k + 1) * vs;
-    g.part_norm = cpartn;
-    g.tmp = t;
     g.need = KR;
-    g.with_norm = 1;
-    launch_gs_dots<TB>(B, g, s);
-    if (k + 1 <= kGsSlice) {
-      // one slice: the per-case reductions run inside the next pass (no reduce launches);
-      // pass 2 writes its partials to a second buffer while it reads pass 1's
-      GsArgs<TB> gp = g;
-      gp.fold_part = cpart;
-      gp.fold_h = h1;
-      gp.fold_wn0 = wn0;
-      gp.part = P->at<double>(P->o_cpart2);
-      launch_gs_project<TB>(B, gp, s);
-      GsArgs<TB> gf = g;
-      gf.fold_part = P->at<double>(P->o_cpart2);
-      gf.fold_h = h2;
-      launch_gs_finish<TB>(B, gf, s);
-    } else {
-      GsReduceArgs rd;
-      rd.part = cpart;
-      rd.pstride = P->pstride;
-      rd.nq = k + 1;
-      rd.scale = scale;
-      rd.h = h1;
-      rd.wn0 = wn0;
-      rd.need = KR;
-      launch_gs_reduce(B, rd, s);
-      launch_gs_project<TB>(B, g, s);
-      rd.h = h2;
-      rd.wn0 = nullptr;
-      launch_gs_reduce(B, rd, s);
-      launch_gs_finish<TB>(B, g, s);
-    }
+    GsArgs<TB> gd = g;
+    gd.part = cpart;
+    launch_gs_dots<TB>(B, gd, s);
+    GsArgs<TB> gp = g;
+    gp.fold_part = cpart;
+    gp.fold_h = h1;
+    gp.fold_wn0 = wn0;
+    gp.part = P->at<double>(P->o_cpart2);
+    launch_gs_project<TB>(B, gp, s);
+    GsArgs<TB> gf = g;
+    gf.fold_part = P->at<double>(P->o_cpart2);
+    gf.fold_h = h2;
+    gf.h1 = h1;
+    gf.Vout = V + (size_t)(k + 1) * vs;
+    gf.part_norm = cpartn;
+    launch_gs_finish<TB>(B, gf, s);
     GsCloseArgs ck;
     ck.part_norm = cpartn;
     ck.wn0 = wn0;
@@ -1246,20 +1225,18 @@ int a2d_time_kernel(a2d_plan* P, int which, int reps, float* ms, void* stream) {
         auto run = [&](auto* Vb) {
           using TB = std::remove_pointer_t<decltype(Vb)>;
           GsArgs<TB> g;
-          g.err = P->at<uint32_t>(P->o_cnt) + 1;
           g.w = P->vec(kW);
           g.V = Vb;
           g.vstride = vs;
           g.nq = half;
-          g.with_norm = 1;
-          g.part = P->at<double>(P->o_cpart);
+                g.part = P->at<double>(which == A2D_K_PROJECT ? P->o_cpart2 : P->o_cpart);
           g.pstride = P->pstride;
+          g.fold_part = P->at<double>(which == A2D_K_PROJECT ? P->o_cpart : P->o_cpart2);
+          g.fold_h = P->at<double>(P->o_h2);
           g.h1 = P->at<double>(P->o_h1);
-          g.h2 = P->at<double>(P->o_h2);
           g.scale = P->at<double>(P->o_scale);
           g.Vout = Vb + (size_t)P->m * vs;
           g.part_norm = P->at<double>(P->o_cpartn);
-          g.tmp = P->vec(kPB);
           if (which == A2D_K_DOTS) launch_gs_dots<TB>(B, g, s);
           else if (which == A2D_K_PROJECT) launch_gs_project<TB>(B, g, s);
           else launch_gs_finish<TB>(B, g, s);

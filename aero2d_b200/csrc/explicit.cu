@@ -9,6 +9,7 @@
 // 1e-18 of the diagonal are dropped, so results equal the FFT's to rounding.
 // Smoothing along j is a Thomas solve of (-e, 1+2e, -e) with end diagonals 1+e.
 #include <algorithm>
+#include <cmath>
 
 #include "batch.cuh"
 #include "explicit.cuh"
@@ -34,10 +35,11 @@ __device__ __forceinline__ T local_dt_cell(const GridDev& g, const State4<T>& W,
   return cfl * m.vol(j, i) / (li + lj);
 }
 
-// local time steps of every case from its conserved state (the RK iteration)
+// local time steps of every case from its conserved state, which is kept as the
+// iteration's start state U0 (the RK iteration)
 template <typename T>
-__global__ void __launch_bounds__(256) k_local_dt(Batch b, const double* __restrict__ U, double* __restrict__ dt,
-                                                  double cfl) {
+__global__ void __launch_bounds__(256) k_local_dt(Batch b, const double* __restrict__ U, double* __restrict__ U0,
+                                                  double* __restrict__ dt, double cfl) {
   const Tile t = b.tiles[blockIdx.x];
   const CaseDev cs = b.cases[t.cs];
   const GridDev& g = cs.g;
@@ -46,7 +48,11 @@ __global__ void __launch_bounds__(256) k_local_dt(Batch b, const double* __restr
     const int j = t.j0 + c / t.ti, i = t.i0 + c % t.ti;
     State4<T> u;
 #pragma unroll
-    for (int k = 0; k < 4; ++k) u.c[k] = T(Uc[vidx(g, k, j, i)]);
+    for (int k = 0; k < 4; ++k) {
+      const double v = Uc[vidx(g, k, j, i)];
+      U0[4 * cs.cell_off + vidx(g, k, j, i)] = v;
+      u.c[k] = T(v);
+    }
     dt[cs.cell_off + (size_t)j * g.ni + i] = (double)local_dt_cell<T>(g, cons_to_prim<T, T>(u), j, i, T(cfl));
   }
 }
@@ -159,6 +165,251 @@ __global__ void __launch_bounds__(128) k_irs_j(Batch b, double* __restrict__ R, 
   }
 }
 
+// ---------------------------------------------------------------------------
+// smoothing and stage update in one kernel
+// ---------------------------------------------------------------------------
+// A CTA takes 32 columns of one component of one case: the rows of R with a halo of M columns
+// (the Green's function's reach, 35 at e = 0.6) into shared memory, the smoothing along i from
+// there (four outputs of a row per thread, each value read once per four terms as a 16-byte
+// vector), the Thomas solves along j (a thread per column, rows in shared memory) and the
+// stage update U = U0 - a (dt / vol) R of euler.py:344 -- or, without STAGE, the smoothed R.
+//
+// What bounded the three kernels this replaces: the Green's function's pow calls in every
+// block, two shared-memory reads per term, and along j a global load and a division in
+// every step of the recurrence.  The tables (irs_table) are now made once per plan, and
+// the division by the step's constant pivot is one multiplication by its reciprocal with
+// Markstein's correction (P. Markstein, IBM J. Res. Dev. 34, 1990: with y = RN(1/b), q = RN(a y)
+// and r = RN(a - q b), RN(q + r y) is RN(a/b)), the quotient itself.  The FP32 iteration is
+// bitwise what it was.
+// Measured (B200, per stage): FP32, 32 cases of 256 x 64, 120 -> 31 us; FP64, 3 cases of
+// 128 x 48, 31 -> 13 us.  Left: the Thomas recurrence's length, one warp of a CTA.
+constexpr int kIrsCols = 32;
+
+// entries of a shape's table: M, g_0 .. g_{ni/2}, then per row the pivot, its reciprocal and c'
+__host__ __device__ inline int irs_gm_entries(int ni) { return ni / 2 + 2; }
+
+// reach of the Green's function: terms below 1e-18 of the diagonal are dropped
+int irs_reach(double e, int ni) {
+  const double lam = ((1.0 + 2.0 * e) - std::sqrt(1.0 + 4.0 * e)) / (2.0 * e);
+  const int M = (int)std::ceil(std::log(1e-18) / std::log(lam));
+  return M > ni / 2 ? ni / 2 : M;
+}
+size_t irs_table_entries(int ni, int nc) { return (size_t)irs_gm_entries(ni) + 3 * (size_t)nc; }
+
+// tables of every case's shape (cases of one shape share a table and write the same values)
+template <typename T>
+__global__ void __launch_bounds__(64) k_irs_table(Batch b, double* __restrict__ tab, double e_) {
+  const CaseDev cs = b.cases[blockIdx.x];
+  const int ni = cs.g.ni, nc = cs.g.nc;
+  double* t = tab + cs.irs_off;
+  const double e = e_;
+  const double lam = ((1.0 + 2.0 * e) - sqrt(1.0 + 4.0 * e)) / (2.0 * e);
+  const double G0 = 1.0 / (e * (1.0 / lam - lam));
+  int M = (int)ceil(log(1e-18) / log(lam));
+  if (M > ni / 2) M = ni / 2;
+  const double ln = pow(lam, (double)ni);
+  for (int m = threadIdx.x; m <= M; m += blockDim.x)
+    t[1 + m] = (double)T(G0 * (pow(lam, (double)m) + pow(lam, (double)(ni - m))) / (1.0 - ln));
+  if (threadIdx.x == 0) {
+    t[0] = M;
+    double* piv = t + irs_gm_entries(ni);
+    const T ee = T(e_);
+    T cp = T(0);
+    for (int j = 0; j < nc; ++j) {
+      const T dj = (j == 0 || j == nc - 1) ? T(1) + ee : T(1) + T(2) * ee;
+      const T lj = (j == 0) ? T(0) : -ee;
+      const T uj = (j == nc - 1) ? T(0) : -ee;
+      const T den = dj - lj * cp;
+      cp = uj / den;
+      piv[j] = (double)den;
+      piv[nc + j] = (double)(T(1) / den);
+      piv[2 * nc + j] = (double)cp;
+    }
+  }
+}
+
+__device__ __forceinline__ void ld4(const float* p, float (&v)[4]) {
+  const float4 t = *reinterpret_cast<const float4*>(p);
+  v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
+}
+__device__ __forceinline__ void ld4(const double* p, double (&v)[4]) {
+  const double2 t = reinterpret_cast<const double2*>(p)[0], u = reinterpret_cast<const double2*>(p)[1];
+  v[0] = t.x; v[1] = t.y; v[2] = u.x; v[3] = u.y;
+}
+
+// a / b for a normal b with y = RN(1/b); an infinite or NaN quotient stays what a y is
+template <typename T>
+__device__ __forceinline__ T quotient(T a, T b, T y) {
+  const T q = a * y;
+  const T r = fma(-q, b, a);
+  return fabs(q) <= T(1e30) ? fma(r, y, q) : a / b;
+}
+
+struct IrsShape {
+  int halo, width;      // columns of a row in shared memory: halo + 32 + halo, or the whole ring
+  bool full;
+};
+// full: the reach covers the ring, every column is summed
+__host__ __device__ inline IrsShape irs_shape(int M, int ni) {
+  IrsShape s;
+  s.full = 2 * M + 1 >= ni;
+  s.halo = s.full ? 0 : (M + 3) & ~3;
+  s.width = s.full ? (ni + 3) & ~3 : kIrsCols + 2 * s.halo;
+  return s;
+}
+// shared memory of a CTA for shapes up to these: the rows, the smoothed columns, the tables
+template <typename T>
+static size_t irs_smem(int width, int nc, int reach) {
+  return sizeof(T) * ((size_t)nc * (width + kIrsCols + 1) + 3 * (size_t)nc + ((reach + 8) & ~3));
+}
+
+template <typename T, bool STAGE>
+__global__ void __launch_bounds__(256) k_irs(Batch b, const double* __restrict__ R, const double* __restrict__ U0,
+                                             const double* __restrict__ dt, double* __restrict__ out,
+                                             const double* __restrict__ tab, double e_, double a) {
+  const CaseDev cs = b.cases[blockIdx.z];
+  const GridDev& g = cs.g;
+  const int ni = g.ni, nc = g.nc, c0 = blockIdx.x * kIrsCols, comp = blockIdx.y;
+  if (c0 >= ni) return;
+  const double* t = tab + cs.irs_off;
+  const int M = (int)t[0];
+  const IrsShape sh = irs_shape(M, ni);
+  extern __shared__ __align__(16) unsigned char irs_sm[];
+  T* raw = reinterpret_cast<T*>(irs_sm);             // [nc][width]
+  T* gm = raw + (size_t)nc * sh.width;               // g_0 .., and room to read past M in vectors
+  T* piv = gm + ((M + 8) & ~3);                      // pivots, reciprocals, c' [nc] each
+  T* sm = piv + 3 * nc;                              // smoothed columns [nc][33]
+  const size_t base = 4 * (size_t)cs.cell_off + vidx(g, comp, 0, 0);
+  // rows to warps, columns to lanes; four rows' values on the way at a time
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  constexpr int kWarps = 8, kRowsAtOnce = 4;
+  for (int x = lane; x < sh.width; x += 32) {
+    int i = sh.full ? x : c0 - sh.halo + x;
+    i += i < 0 ? ni : 0;
+    i -= i >= ni ? ni : 0;     // the last CTA's columns past the ring (full: past ni, not used) wrap
+    i -= i >= ni ? ni : 0;
+    const double* src = R + base + i;
+    for (int j0 = warp; j0 < nc; j0 += kWarps * kRowsAtOnce) {
+      double v[kRowsAtOnce];
+#pragma unroll
+      for (int u = 0; u < kRowsAtOnce; ++u) {
+        const int j = j0 + u * kWarps;
+        v[u] = j < nc ? src[(size_t)j * ni] : 0.0;
+      }
+#pragma unroll
+      for (int u = 0; u < kRowsAtOnce; ++u) {
+        const int j = j0 + u * kWarps;
+        if (j < nc) raw[j * sh.width + x] = T(v[u]);
+      }
+    }
+  }
+  for (int m = threadIdx.x; m < ((M + 8) & ~3); m += blockDim.x) gm[m] = m <= M ? T(t[1 + m]) : T(0);
+  for (int q = threadIdx.x; q < 3 * nc; q += blockDim.x) piv[q] = T(t[irs_gm_entries(ni) + q]);
+  __syncthreads();
+  if (sh.full) {
+    for (int q = threadIdx.x; q < nc * kIrsCols; q += blockDim.x) {
+      const int j = q / kIrsCols, c = q % kIrsCols, i = c0 + c;
+      if (i >= ni) continue;
+      const T* r = raw + (size_t)j * sh.width;
+      T s = gm[0] * r[i];
+      for (int d = 1; d < ni; ++d) {
+        const int m = d <= ni / 2 ? d : ni - d;
+        int p = i - d;
+        if (p < 0) p += ni;
+        s += gm[m] * r[p];
+      }
+      sm[j * (kIrsCols + 1) + c] = s;
+    }
+  } else {
+    for (int q = threadIdx.x; q < nc * (kIrsCols / 4); q += blockDim.x) {
+      const int j = q / (kIrsCols / 4), c = q % (kIrsCols / 4) * 4;
+      const T* r = raw + (size_t)j * sh.width + sh.halo + c;
+      // terms m = 4 h + 1 .. 4 h + 4 of the four outputs c .. c + 3: the columns from 4 h + 4
+      // before to 4 h + 7 after are two vectors on either side, one of them new
+      T s[4], L[4], P[4], Ln[4], Pn[4];
+      ld4(r, L);
+#pragma unroll
+      for (int v = 0; v < 4; ++v) {
+        P[v] = L[v];
+        s[v] = gm[0] * L[v];
+      }
+      for (int h = 0; 4 * h < M; ++h) {
+        ld4(r - 4 * (h + 1), Ln);
+        ld4(r + 4 * (h + 1), Pn);
+#pragma unroll
+        for (int k = 1; k <= 4; ++k) {
+          if (4 * h + k <= M) {
+            const T w = gm[4 * h + k];
+#pragma unroll
+            for (int v = 0; v < 4; ++v) {
+              const T lo = v - k >= 0 ? L[(v - k) & 3] : Ln[(4 + v - k) & 3];
+              const T hi = v + k < 4 ? P[(v + k) & 3] : Pn[(v + k) & 3];
+              s[v] += w * (lo + hi);
+            }
+          }
+        }
+#pragma unroll
+        for (int v = 0; v < 4; ++v) {
+          L[v] = Ln[v];
+          P[v] = Pn[v];
+        }
+      }
+#pragma unroll
+      for (int v = 0; v < 4; ++v) sm[j * (kIrsCols + 1) + c + v] = s[v];
+    }
+  }
+  __syncthreads();
+  // Thomas solves by one warp; the others fetch what the stage update needs meanwhile, into the
+  // raw rows, which are done with (two values a cell: rings of fewer columns fetch it after)
+  const bool ahead = STAGE && sh.width >= 2 * kIrsCols;
+  const int n = min(kIrsCols, ni - c0);
+  const Metric<T> m{g};
+  T* fs = raw;
+  T* us = raw + nc * kIrsCols;
+  auto factor = [&](int j, int i) { return T(a) * (T(dt[cs.cell_off + (size_t)j * ni + i]) / m.vol(j, i)); };
+  if (warp == 0) {
+    T* col = sm + lane;
+    constexpr int st = kIrsCols + 1;
+    const T e = T(e_);
+    T prev = T(0), x = col[0];
+    for (int j = 0; j < nc; ++j) {
+      const T xn = j + 1 < nc ? col[(j + 1) * st] : T(0);
+      const T v = quotient(j == 0 ? x : fma(e, prev, x), piv[j], piv[nc + j]);
+      col[j * st] = v;
+      prev = v;
+      x = xn;
+    }
+    T xn = T(0), y = col[(nc - 1) * st];
+    for (int j = nc - 1; j >= 0; --j) {
+      const T yn = j > 0 ? col[(j - 1) * st] : T(0);
+      const T v = y - piv[2 * nc + j] * xn;
+      col[j * st] = v;
+      xn = v;
+      y = yn;
+    }
+  } else if (ahead && lane < n) {
+#pragma unroll 4
+    for (int j = warp - 1; j < nc; j += kWarps - 1) {
+      fs[j * kIrsCols + lane] = factor(j, c0 + lane);
+      us[j * kIrsCols + lane] = T(U0[base + (size_t)j * ni + c0 + lane]);
+    }
+  }
+  __syncthreads();
+  if (lane >= n) return;
+#pragma unroll 4
+  for (int j = warp; j < nc; j += kWarps) {
+    const T v = sm[j * (kIrsCols + 1) + lane];
+    const size_t o = base + (size_t)j * ni + c0 + lane;
+    if constexpr (STAGE) {
+      const T f = ahead ? fs[j * kIrsCols + lane] : factor(j, c0 + lane);
+      const T u = ahead ? us[j * kIrsCols + lane] : T(U0[o]);
+      out[o] = (double)(u - f * v);
+    } else {
+      out[o] = (double)v;
+    }
+  }
+}
+
 // U = U0 - a (dt / vol) R   (euler.py:344), in the compute type T (with FP32
 // the state is rounded to FP32 at every stage, as the reference's float32 run keeps it)
 template <typename T>
@@ -210,13 +461,25 @@ __global__ void __launch_bounds__(256) k_rk_res(Batch b, const double* __restric
   }
 }
 
-// res = sqrt(mean(...)) per case; circ = 1/2 Cl M from the forces   (euler.py:345, :401-403)
-__global__ void k_rk_finish(Batch b, const double* tpart, const double* coef, double* res, double* circ) {
-  const int cs = blockIdx.x * blockDim.x + threadIdx.x;
-  if (cs >= b.ncases) return;
+// res = sqrt(mean(...)) per case; circ = 1/2 Cl M from the forces   (euler.py:345, :401-403); a
+// block per case, the tiles' sums fetched together and added in order
+__global__ void __launch_bounds__(128) k_rk_finish(Batch b, const double* tpart, const double* coef, double* res,
+                                                   double* circ) {
+  __shared__ double part[128];
+  const int cs = blockIdx.x;
   const CaseDev c = b.cases[cs];
   double s = 0.0;
-  for (int q = 0; q < c.ntiles; ++q) s += tpart[(size_t)(c.tile0 + q) * kTilePartStride + 3];
+  if (res != nullptr) {
+    for (int q0 = 0; q0 < c.ntiles; q0 += 128) {
+      if (q0 + (int)threadIdx.x < c.ntiles)
+        part[threadIdx.x] = tpart[(size_t)(c.tile0 + q0 + threadIdx.x) * kTilePartStride + 3];
+      __syncthreads();
+      if (threadIdx.x == 0)
+        for (int q = 0; q < min(128, c.ntiles - q0); ++q) s += part[q];
+      __syncthreads();
+    }
+  }
+  if (threadIdx.x != 0) return;
   const double N = (double)c.g.ni * (double)c.g.nc;
   if (res != nullptr) res[cs] = sqrt(s / N);
   const double mach = sqrt(c.winf[1] * c.winf[1] + c.winf[2] * c.winf[2]);
@@ -333,10 +596,10 @@ __global__ void __launch_bounds__(256) k_fas_prolong(Batch fb, Batch cb, double*
   }
 }
 
-void launch_local_dt(const Batch& b, const double* U, double* dt, double cfl, bool fp32, cudaStream_t s) {
+void launch_local_dt(const Batch& b, const double* U, double* U0, double* dt, double cfl, bool fp32, cudaStream_t s) {
   if (b.ntiles == 0) return;
-  if (fp32) k_local_dt<float><<<b.ntiles, 256, 0, s>>>(b, U, dt, cfl);
-  else k_local_dt<double><<<b.ntiles, 256, 0, s>>>(b, U, dt, cfl);
+  if (fp32) k_local_dt<float><<<b.ntiles, 256, 0, s>>>(b, U, U0, dt, cfl);
+  else k_local_dt<double><<<b.ntiles, 256, 0, s>>>(b, U, U0, dt, cfl);
 }
 void launch_local_dt_prim(const GridDev& g, const double* W, double* dt, double cfl, cudaStream_t s) {
   const size_t N = (size_t)g.ni * g.nc;
@@ -357,6 +620,43 @@ void launch_irs(const Batch& b, double* R, double* tmp, double e, int max_ni, in
     k_irs_j<double><<<gj, 128, (size_t)max_nc * sizeof(double), s>>>(b, tmp, e);
   }
 }
+void launch_irs_table(const Batch& b, double* tab, double e, bool fp32, cudaStream_t s) {
+  if (b.ncases == 0) return;
+  if (fp32) k_irs_table<float><<<b.ncases, 64, 0, s>>>(b, tab, e);
+  else k_irs_table<double><<<b.ncases, 64, 0, s>>>(b, tab, e);
+}
+template <typename T, bool STAGE>
+static void irs_launch(const Batch& b, const IrsArgs& p, size_t smem, cudaStream_t s) {
+  k_irs<T, STAGE><<<dim3((p.max_ni + kIrsCols - 1) / kIrsCols, 4, b.ncases), 256, smem, s>>>(b, p.R, p.U0, p.dt, p.out,
+                                                                                            p.tab, p.e, p.a);
+}
+void launch_irs_fused(const Batch& b, const IrsArgs& p, bool fp32, cudaStream_t s) {
+  if (b.ncases == 0) return;
+  const size_t smem = p.smem;
+  if (p.U0 != nullptr) {
+    if (fp32) irs_launch<float, true>(b, p, smem, s);
+    else irs_launch<double, true>(b, p, smem, s);
+  } else {
+    if (fp32) irs_launch<float, false>(b, p, smem, s);
+    else irs_launch<double, false>(b, p, smem, s);
+  }
+}
+size_t irs_smem_bytes(int ni, int nc, double e, bool fp32) {
+  const int M = irs_reach(e, ni);
+  const IrsShape sh = irs_shape(M, ni);
+  return fp32 ? irs_smem<float>(sh.width, nc, M) : irs_smem<double>(sh.width, nc, M);
+}
+cudaError_t irs_init() {
+  cudaError_t e = cudaSuccess;
+  auto set = [&](const void* f) {
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kIrsMaxSmem);
+  };
+  set(reinterpret_cast<const void*>(&k_irs<float, true>));
+  set(reinterpret_cast<const void*>(&k_irs<float, false>));
+  set(reinterpret_cast<const void*>(&k_irs<double, true>));
+  set(reinterpret_cast<const void*>(&k_irs<double, false>));
+  return e;
+}
 void launch_rk_stage(const Batch& b, const double* U0, const double* R, const double* dt, double* U, double a,
                      bool fp32, cudaStream_t s) {
   if (b.ntiles == 0) return;
@@ -369,7 +669,7 @@ void launch_rk_res(const Batch& b, const double* U0, const double* U, const doub
 }
 void launch_rk_finish(const Batch& b, const double* tpart, const double* coef, double* res, double* circ,
                       cudaStream_t s) {
-  k_rk_finish<<<(b.ncases + 63) / 64, 64, 0, s>>>(b, tpart, coef, res, circ);
+  if (b.ncases) k_rk_finish<<<b.ncases, 128, 0, s>>>(b, tpart, coef, res, circ);
 }
 
 void launch_add_forcing(const Batch& b, double* R, const double* P, cudaStream_t s) {

@@ -95,6 +95,8 @@ struct a2d_plan {
   std::vector<LineClass> line_classes;
   std::vector<int> line_cases;
   bool lines_fit = false;      // every class runs on the device bound to (set at bind)
+  size_t irs_entries = 0, irs_smem = 0, o_irs = 0;   // smoothing tables (explicit.cu), a shape's once
+  bool irs_ready = false;      // filled since bind
   size_t o_lcases = 0, o_E0 = 0;   // o_E0: inv r of the lines, kept between the sweeps of an application
   long long C = 0, rows_nc = 0, rows_nc1 = 0, total_ni = 0;
   size_t tj = 8, tb = 8;   // bytes of face-Jacobian and basis storage entries
@@ -184,6 +186,15 @@ static void build_tables(a2d_plan* P, const int* ni, const int* nc, const void* 
   P->total_ni = cpo;
   for (int sh = 0; sh < kNumTileShapes; ++sh) P->max_jtiles = std::max(P->max_jtiles, (int)tile_list(P, sh).size());
   P->jtiles = tile_list(P, P->jvp_tile);
+  std::map<std::pair<int, int>, int> irs_at;
+  for (int k = 0; k < P->ncases; ++k) {
+    const auto it = irs_at.emplace(std::make_pair(ni[k], nc[k]), (int)P->irs_entries);
+    P->cases[k].irs_off = it.first->second;
+    if (!it.second) continue;
+    P->irs_entries += irs_table_entries(ni[k], nc[k]);
+    if (P->p.irs_eps > 0)
+      P->irs_smem = std::max(P->irs_smem, irs_smem_bytes(ni[k], nc[k], P->p.irs_eps, P->p.precision == A2D_MIXED));
+  }
   std::map<int, std::vector<int>> by_groups;
   for (int k = 0; k < P->ncases; ++k) by_groups[P->cases[k].ngroups].push_back(k);
   for (const auto& g : by_groups) {
@@ -239,6 +250,7 @@ static void layout(a2d_plan* P) {
   P->o_idx = cv.take(sizeof(int) * (size_t)B);   // case index lists of a2d_case_restart / _retire
   P->o_sat = cv.take(sizeof(unsigned long long));
   P->o_jtiles = cv.take(sizeof(Tile) * (size_t)P->max_jtiles);
+  P->o_irs = cv.take(8 * P->irs_entries);
   P->o_lcases = cv.take(sizeof(int) * (size_t)B);
   P->bytes = cv.off + 256;
 }
@@ -461,6 +473,34 @@ static void precond_setup(a2d_plan* P, const Batch& B, uint32_t need, cudaStream
   ja.need = need;
   launch_face_jac<TJ>(B, ja, s);
   launch_factor<TJ, typename FactorStore<TJ>::type>(B, factor_args(P, need), s);
+}
+
+// one smoothing of R by the plan's coefficient: the stage update U = U0 - a (dt / vol) R~, or
+// (U0 null) out = R~; false where the fused kernel does not run
+static bool irs_fused(a2d_plan* P, const Batch& B, const double* R, const double* U0, double* out, double a,
+                      cudaStream_t s) {
+  if (P->p.irs_eps <= 0 || P->irs_smem > kIrsMaxSmem) return false;
+  const bool fp32 = P->p.precision == A2D_MIXED;
+  if (!P->irs_ready) {
+    launch_irs_table(B, P->at<double>(P->o_irs), P->p.irs_eps, fp32, s);
+    P->irs_ready = true;
+  }
+  IrsArgs p;
+  p.R = R;
+  p.U0 = U0;
+  p.dt = P->at<double>(P->o_dt);
+  p.out = out;
+  p.tab = P->at<double>(P->o_irs);
+  p.e = P->p.irs_eps;
+  p.a = a;
+  p.max_ni = P->max_ni;
+  p.smem = P->irs_smem;
+  launch_irs_fused(B, p, fp32, s);
+  return true;
+}
+static void smoothed(a2d_plan* P, const Batch& B, double* R, double* out, cudaStream_t s) {
+  if (!irs_fused(P, B, R, nullptr, out, 0.0, s))
+    launch_irs(B, R, out, P->p.irs_eps, P->max_ni, P->max_nc, P->p.precision == A2D_MIXED, s);
 }
 
 static StencilArgs<double> residual_args(a2d_plan* P) {
@@ -853,6 +893,8 @@ int a2d_plan_bind(a2d_plan* P, void* workspace, size_t bytes, void* stream) {
     P->lines_fit = P->lines_fit && (mixed ? n > 0 : n >= c.count);
   }
   A2D_CK(gs_init());
+  A2D_CK(irs_init());
+  P->irs_ready = false;
   stencil_init_fp64();
   stencil_init_fp32();
   k_reset<<<(P->ncases + 63) / 64, 64, 0, s>>>(P->ncases, P->ctl(), P->live(), P->p.cfl0);
@@ -1360,7 +1402,7 @@ int a2d_smooth(a2d_plan* P, void* stream) {
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   Batch B = P->batch;
   B.live = nullptr;
-  launch_irs(B, P->vec(kR), P->vec(kPA), P->p.irs_eps, P->max_ni, P->max_nc, P->p.precision == A2D_MIXED, s);
+  smoothed(P, B, P->vec(kR), P->vec(kPA), s);
   if (P->p.irs_eps > 0)
     A2D_CK(cudaMemcpyAsync(P->vec(kR), P->vec(kPA), 8 * 4 * (size_t)P->C, cudaMemcpyDeviceToDevice, s));
   A2D_CK(cudaGetLastError());
@@ -1403,8 +1445,7 @@ static cudaError_t rk_iter(a2d_plan* P, const double* circ, const double* forcin
   // (the reference casts its whole explicit iteration to the solver dtype,
   // aero2d/euler.py:222-234); the state keeps FP32-rounded values in FP64 storage
   const bool fp32 = P->p.precision == A2D_MIXED;
-  if (cudaError_t e = cudaMemcpyAsync(U0, U, 8 * 4 * (size_t)P->C, cudaMemcpyDeviceToDevice, s)) return e;
-  launch_local_dt(B, U, dt, P->p.cfl, fp32, s);
+  launch_local_dt(B, U, U0, dt, P->p.cfl, fp32, s);
   for (int st = 0; st < 4; ++st) {
     StencilArgs<double> a = residual_args(P);
     a.circ_in = circ;
@@ -1413,6 +1454,7 @@ static cudaError_t rk_iter(a2d_plan* P, const double* circ, const double* forcin
     if (fp32) launch_stencil<float, false, double>(B, a, s);
     else launch_stencil<double, false, double>(B, a, s);
     if (forcing != nullptr) launch_add_forcing(B, R, forcing, s);
+    if (irs_fused(P, B, R, U0, U, alphas[st], s)) continue;
     const double* Ruse = R;
     if (P->p.irs_eps > 0) {
       launch_irs(B, R, Rs, P->p.irs_eps, P->max_ni, P->max_nc, fp32, s);

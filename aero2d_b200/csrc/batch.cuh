@@ -156,6 +156,9 @@ template <> struct Metric<double> {
   __device__ __forceinline__ double sj(int k, int j, int i) const {
     return g.Sj[((size_t)k * (g.nc + 1) + j) * g.ni + i];
   }
+  // component k of the i- (j-) faces of row j
+  __device__ __forceinline__ const double* si_row(int k, int j) const { return g.Si + ((size_t)k * g.nc + j) * g.ni; }
+  __device__ __forceinline__ const double* sj_row(int k, int j) const { return g.Sj + ((size_t)k * (g.nc + 1) + j) * g.ni; }
   __device__ __forceinline__ double xf(int i) const { return g.xf[i]; }
   __device__ __forceinline__ double yf(int i) const { return g.yf[i]; }
 };
@@ -168,6 +171,8 @@ template <> struct Metric<float> {
   __device__ __forceinline__ float sj(int k, int j, int i) const {
     return g.Sj_f[((size_t)k * (g.nc + 1) + j) * g.ni + i];
   }
+  __device__ __forceinline__ const float* si_row(int k, int j) const { return g.Si_f + ((size_t)k * g.nc + j) * g.ni; }
+  __device__ __forceinline__ const float* sj_row(int k, int j) const { return g.Sj_f + ((size_t)k * (g.nc + 1) + j) * g.ni; }
   __device__ __forceinline__ float xf(int i) const { return g.xf_f[i]; }
   __device__ __forceinline__ float yf(int i) const { return g.yf_f[i]; }
 };

@@ -116,6 +116,13 @@ __device__ void block_circulation(const CaseDev& cs, const double* U, const VT* 
   }
 }
 
+// division of the small numbers of a tile's index arithmetic (n < 2048, d < 70: exact)
+struct SmallDiv {
+  uint32_t magic;
+  __device__ __forceinline__ explicit SmallDiv(int d) : magic((1u << 18) / (uint32_t)d + 1u) {}
+  __device__ __forceinline__ int operator()(int n) const { return (int)(((uint32_t)n * magic) >> 18); }
+};
+
 // ---------------------------------------------------------------------------
 // the fused residual / JVP tile kernel
 // ---------------------------------------------------------------------------
@@ -173,8 +180,9 @@ __device__ __forceinline__ void stencil_tile(const Batch& b, const StencilArgs<V
 
   // stage primitive states with halo and ghosts
   const int wr = t.tj + 4, wc = t.ti + 4;
+  const SmallDiv by_wc(wc);
   for (int idx = threadIdx.x; idx < wr * wc; idx += blockDim.x) {
-    const int r = idx / wc, c = idx % wc;
+    const int r = by_wc(idx), c = idx - r * wc;
     const int gj = t.j0 + r - 2;
     int gi = t.i0 + c - 2;
     gi = gi < 0 ? gi + ni : (gi >= ni ? gi - ni : gi);
@@ -206,56 +214,56 @@ __device__ __forceinline__ void stencil_tile(const Batch& b, const StencilArgs<V
   }
   __syncthreads();
 
-  // face fluxes: i-faces (tj rows x ti+1 faces), then j-faces (tj+1 faces x ti columns)
+  // face fluxes: i-faces (tj rows x ti+1 faces), then j-faces (tj+1 faces x ti columns), all by
+  // one copy of the code: two, one per direction, are 32 KB of instructions in the dual case
   const int nfi = t.tj * (t.ti + 1);
   const int nfj = (t.tj + 1) * t.ti;
   const bool second = a.order == 2;
+  const SmallDiv by_ti1(t.ti + 1), by_ti(t.ti);
+  const S* sWf = &sW[0][0][0];
+  const T* Si = m.si_row(0, 0);
+  const T* Sj = m.sj_row(0, 0);
   for (int f = threadIdx.x; f < nfi + nfj; f += blockDim.x) {
-    State4<S> Wm, W0, Wp, Wpp;
+    int w0, st, dst_stride;   // the four states of the face: w0, w0 + st, ..
+    T* dst;
     T sx, sy;
     if (f < nfi) {
-      const int jl = f / (t.ti + 1), fl = f % (t.ti + 1);
-      const int r = jl + 2;
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        Wm.c[k] = sW[k][r][fl];
-        W0.c[k] = sW[k][r][fl + 1];
-        Wp.c[k] = sW[k][r][fl + 2];
-        Wpp.c[k] = sW[k][r][fl + 3];
-      }
+      const int jl = by_ti1(f), fl = f - jl * (t.ti + 1);
+      w0 = (jl + 2) * WI + fl;
+      st = 1;
       int fi = t.i0 + fl;
       if (fi >= ni) fi -= ni;
-      sx = m.si(0, t.j0 + jl, fi);
-      sy = m.si(1, t.j0 + jl, fi);
-      State4<S> WL, WR;
-      recon<S, T>(Wm, W0, Wp, Wpp, eps, second, WL, WR);
-      const State4<S> F = hllc<S, T>(WL, WR, sx, sy);
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        if constexpr (LIN) sFi[k][jl][fl] = F.c[k].d[0];
-        else sFi[k][jl][fl] = F.c[k];
-      }
+      const int q = (t.j0 + jl) * ni + fi;
+      sx = Si[q];
+      sy = Si[q + nc * ni];
+      dst = &sFi[0][jl][fl];
+      dst_stride = TJ * (TI + 1);
     } else {
       const int f2 = f - nfi;
-      const int fl = f2 / t.ti, il = f2 % t.ti;
-      const int c = il + 2;
+      const int fl = by_ti(f2), il = f2 - fl * t.ti;
+      w0 = fl * WI + il + 2;
+      st = WI;
+      const int q = (t.j0 + fl) * ni + t.i0 + il;
+      sx = Sj[q];
+      sy = Sj[q + (nc + 1) * ni];
+      dst = &sFj[0][fl][il];
+      dst_stride = (TJ + 1) * TI;
+    }
+    State4<S> Wm, W0, Wp, Wpp, WL, WR;
 #pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        Wm.c[k] = sW[k][fl][c];
-        W0.c[k] = sW[k][fl + 1][c];
-        Wp.c[k] = sW[k][fl + 2][c];
-        Wpp.c[k] = sW[k][fl + 3][c];
-      }
-      sx = m.sj(0, t.j0 + fl, t.i0 + il);
-      sy = m.sj(1, t.j0 + fl, t.i0 + il);
-      State4<S> WL, WR;
-      recon<S, T>(Wm, W0, Wp, Wpp, eps, second, WL, WR);
-      const State4<S> F = hllc<S, T>(WL, WR, sx, sy);
+    for (int k = 0; k < 4; ++k) {
+      const S* w = sWf + k * (WJ * WI) + w0;
+      Wm.c[k] = w[0];
+      W0.c[k] = w[st];
+      Wp.c[k] = w[2 * st];
+      Wpp.c[k] = w[3 * st];
+    }
+    recon<S, T>(Wm, W0, Wp, Wpp, eps, second, WL, WR);
+    const State4<S> F = hllc<S, T>(WL, WR, sx, sy);
 #pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        if constexpr (LIN) sFj[k][fl][il] = F.c[k].d[0];
-        else sFj[k][fl][il] = F.c[k];
-      }
+    for (int k = 0; k < 4; ++k) {
+      if constexpr (LIN) dst[k * dst_stride] = F.c[k].d[0];
+      else dst[k * dst_stride] = F.c[k];
     }
   }
   __syncthreads();
@@ -264,7 +272,7 @@ __device__ __forceinline__ void stencil_tile(const Batch& b, const StencilArgs<V
   double part = 0.0;
   const size_t base = 4 * cs.cell_off;
   for (int c = threadIdx.x; c < t.ti * t.tj; c += blockDim.x) {
-    const int jl = c / t.ti, il = c % t.ti;
+    const int jl = by_ti(c), il = c - jl * t.ti;
     const int gj = t.j0 + jl, gi = t.i0 + il;
     T R[4];
 #pragma unroll
@@ -301,8 +309,15 @@ __device__ __forceinline__ void stencil_tile(const Batch& b, const StencilArgs<V
 // Persistent: the grid is at most the CTAs resident on the GPU, and each CTA
 // walks the batch's tile list (every case's tiles, whatever their grid size)
 // with a stride of the grid size.  TI x TJ is the tile shape of that list.
+//
+// The divides, square roots and their dependent chains bound it, so what counts is the warps
+// in flight: FP32 runs at 64 registers, 4 CTAs per SM.  FP64 left alone takes 150 (residual)
+// and 168 (JVP) registers, one CTA; held to 128 it runs two, the residual without a spill,
+// the JVP with 92 bytes of them.  On 64 cases of 256x64 cells: residual 402 -> 193 us
+// (320 MB compulsory, 48 us), FP64 JVP 602 -> 300; one 128x48 case 20.6 -> 18.5 and
+// 28.8 -> 25.7.
 template <typename T, bool LIN, typename VT, int TI, int TJ>
-__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 1) k_stencil(Batch b, StencilArgs<VT> a) {
+__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 2) k_stencil(Batch b, StencilArgs<VT> a) {
   for (int tile = blockIdx.x; tile < b.ntiles; tile += gridDim.x) {
     if (tile != (int)blockIdx.x) __syncthreads();   // the previous tile is done with shared memory
     stencil_tile<T, LIN, VT, TI, TJ>(b, a, tile);

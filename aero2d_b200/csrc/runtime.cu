@@ -70,6 +70,10 @@ enum VecSlot { kU = 0, kR, kVin, kJV, kDU, kB, kX0, kT, kRr, kZ, kW, kPA, kPB, k
 
 using namespace a2d;
 
+// the most 16x4 tiles that one wave of the FP64 and of the FP32 stencils takes: 2 and 4 CTAs on
+// each of 148 SMs (tile_stencil)
+constexpr int kFineTiles64 = 2 * 148, kFineTiles32 = 4 * 148;
+
 struct a2d_plan {
   a2d_params p{};
   int ncases = 0;
@@ -109,8 +113,10 @@ struct a2d_plan {
   size_t o_tpart = 0, o_cpart = 0, o_cpart2 = 0, o_cpartn = 0, o_coef = 0, o_cp = 0, o_hrn = 0, o_hcl = 0,
          o_cnt = 0, o_idx = 0;
   size_t o_sat = 0;        // saturated FP16 factor entries since bind (a2d_factor_saturations)
-  size_t o_jtiles = 0;
+  size_t o_jtiles = 0, o_ftiles = 0;
   Batch jbatch{};          // the batch with the JVP's tile list
+  std::vector<Tile> ftiles;    // 16x4 tiles, none when they would be more than kFineTiles32
+  Batch fbatch{};          // the batch with these
   int pstride = 0;
   size_t bytes = 0;
   char* ws = nullptr;
@@ -186,6 +192,8 @@ static void build_tables(a2d_plan* P, const int* ni, const int* nc, const void* 
   P->total_ni = cpo;
   for (int sh = 0; sh < kNumTileShapes; ++sh) P->max_jtiles = std::max(P->max_jtiles, (int)tile_list(P, sh).size());
   P->jtiles = tile_list(P, P->jvp_tile);
+  P->ftiles = tile_list(P, kTile16x4);
+  if ((int)P->ftiles.size() > kFineTiles32) P->ftiles.clear();
   std::map<std::pair<int, int>, int> irs_at;
   for (int k = 0; k < P->ncases; ++k) {
     const auto it = irs_at.emplace(std::make_pair(ni[k], nc[k]), (int)P->irs_entries);
@@ -250,6 +258,7 @@ static void layout(a2d_plan* P) {
   P->o_idx = cv.take(sizeof(int) * (size_t)B);   // case index lists of a2d_case_restart / _retire
   P->o_sat = cv.take(sizeof(unsigned long long));
   P->o_jtiles = cv.take(sizeof(Tile) * (size_t)P->max_jtiles);
+  P->o_ftiles = cv.take(sizeof(Tile) * P->ftiles.size());
   P->o_irs = cv.take(8 * P->irs_entries);
   P->o_lcases = cv.take(sizeof(int) * (size_t)B);
   P->bytes = cv.off + 256;
@@ -512,17 +521,27 @@ static StencilArgs<double> residual_args(a2d_plan* P) {
   return a;
 }
 
-// the linearised stencil (J v): in FP32 on the plan's JVP tile list and shape,
-// in FP64 on the standard tiles
-template <typename TV, typename VT>
-static void launch_jvp(const a2d_plan* P, const StencilArgs<VT>& a, cudaStream_t s) {
-  if constexpr (sizeof(TV) == 4) {
-    Batch jb = P->jbatch;
-    jb.live = P->batch.live;
-    launch_stencil<TV, true, VT>(jb, a, s, P->jvp_tile);
-  } else {
-    launch_stencil<TV, true, VT>(P->batch, a, s);
+// The stencil on the tile list that suits the plan.  A batch whose 16x4 tiles all run at once
+// takes these: a small batch is bound by the latency of one tile, whose 148 faces are one round
+// of the CTA's 256 threads and the 552 of a 32x8 tile three, while the chip has SMs to spare.
+// One 128x48 case: FP32 JVP 14.4 -> 8.4 us, FP64 JVP 25.7 -> 18.4, explicit FP64 residual of
+// three 16.1 -> 10.9.  From the second wave on the wider halo costs more than the latency saved:
+// 8 cases of 128x48 are 14.4 on either in FP32 and 30.8 on 32x8, 32.8 on 16x4 in FP64; 8 of
+// 256x64 are 18.5 and 24.7.  The squared residual sums of a Newton step are per 32x8 tile, so
+// its residual keeps these, and a JVP shape that was asked for stays.
+template <typename T, bool LIN, typename VT>
+static void tile_stencil(const a2d_plan* P, const uint32_t* live, const StencilArgs<VT>& a, cudaStream_t s) {
+  constexpr bool knob = LIN && sizeof(T) == 4;
+  int shape = knob ? P->jvp_tile : kTile32x8;
+  Batch b = knob ? P->jbatch : P->batch;
+  const size_t limit = sizeof(T) == 4 ? kFineTiles32 : kFineTiles64;
+  if (!P->ftiles.empty() && P->ftiles.size() <= limit && a.tile_part == nullptr &&
+      (!knob || P->jvp_tile == kTile32x16)) {
+    shape = kTile16x4;
+    b = P->fbatch;
   }
+  b.live = live;
+  launch_stencil<T, LIN, VT>(b, a, s, shape);
 }
 
 template <typename TV, typename TJ, typename TB>
@@ -555,7 +574,7 @@ static void newton_step_launches(a2d_plan* P, cudaStream_t s) {
   ra.circ_out = P->at<double>(P->o_circ);
   ra.tile_part = tpart;
   ra.need = NW;
-  launch_stencil<double, false, double>(B, ra, s);
+  tile_stencil<double, false>(P, live, ra, s);
   // line preconditioner at U
   precond_setup<TJ>(P, B, NW, s);
   nvtxRangePop();
@@ -571,7 +590,7 @@ static void newton_step_launches(a2d_plan* P, cudaStream_t s) {
   ta.bvec = b;
   ta.out = t;
   ta.need = NW;
-  launch_jvp<TV, double>(P, ta, s);
+  tile_stencil<TV, true>(P, live, ta, s);
   // r = M t, v0 = r / ||r||
   precond<TJ>(P, B, t, r, NW, s);
   double* h1 = P->at<double>(P->o_h1);
@@ -605,7 +624,7 @@ static void newton_step_launches(a2d_plan* P, cudaStream_t s) {
     za.order = P->p.order;
     za.vortex = P->p.vortex_correction;
     za.need = KR;
-    launch_jvp<TV, TB>(P, za, s);
+    tile_stencil<TV, true>(P, live, za, s);
     precond<TJ>(P, B, z, w, KR, s);
     // classical Gram-Schmidt run twice, three passes over the basis; passes 2 and 3 reduce
     // the partials of the pass before, so pass 2 writes its own to a second buffer
@@ -876,6 +895,11 @@ int a2d_plan_bind(a2d_plan* P, void* workspace, size_t bytes, void* stream) {
   P->jbatch = B;
   P->jbatch.tiles = P->at<Tile>(P->o_jtiles);
   P->jbatch.ntiles = (int)P->jtiles.size();
+  A2D_CK(cudaMemcpyAsync(P->ws + P->o_ftiles, P->ftiles.data(), sizeof(Tile) * P->ftiles.size(),
+                         cudaMemcpyHostToDevice, s));
+  P->fbatch = B;
+  P->fbatch.tiles = P->at<Tile>(P->o_ftiles);
+  P->fbatch.ntiles = (int)P->ftiles.size();
   A2D_CK(cudaMemcpyAsync(P->ws + P->o_lcases, P->line_cases.data(), sizeof(int) * P->line_cases.size(),
                          cudaMemcpyHostToDevice, s));
   if (P->host_count == nullptr) A2D_CK(cudaMallocHost(&P->host_count, 2 * sizeof(int)));
@@ -1054,9 +1078,7 @@ int a2d_residual(a2d_plan* P, const double* circ, void* stream) {
   a.sign = 1.0;
   a.circ_out = P->at<double>(P->o_circ);
   a.tile_part = P->at<double>(P->o_tpart);
-  Batch B = P->batch;
-  B.live = nullptr;
-  launch_stencil<double, false, double>(B, a, static_cast<cudaStream_t>(stream));
+  tile_stencil<double, false>(P, nullptr, a, static_cast<cudaStream_t>(stream));
   A2D_CK(cudaGetLastError());
   return A2D_OK;
 }
@@ -1066,15 +1088,9 @@ int a2d_jvp(a2d_plan* P, void* stream) {
   StencilArgs<double> a = residual_args(P);
   a.V = P->vec(kVin);
   a.out = P->vec(kJV);
-  Batch B = P->batch;
-  B.live = nullptr;
-  if (P->p.precision == A2D_MIXED) {
-    Batch jb = P->jbatch;
-    jb.live = nullptr;
-    launch_stencil<float, true, double>(jb, a, static_cast<cudaStream_t>(stream), P->jvp_tile);
-  } else {
-    launch_stencil<double, true, double>(B, a, static_cast<cudaStream_t>(stream));
-  }
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  if (P->p.precision == A2D_MIXED) tile_stencil<float, true>(P, nullptr, a, s);
+  else tile_stencil<double, true>(P, nullptr, a, s);
   A2D_CK(cudaGetLastError());
   return A2D_OK;
 }
@@ -1219,15 +1235,13 @@ int a2d_time_kernel(a2d_plan* P, int which, int reps, float* ms, void* stream) {
           a.lim_k = P->p.lim_k;
           a.order = P->p.order;
           a.vortex = P->p.vortex_correction;
-          Batch jb = P->jbatch;
-          jb.live = nullptr;
-          launch_stencil<float, true, Basis16>(jb, a, s, P->jvp_tile);
+          tile_stencil<float, true>(P, nullptr, a, s);
         } else {
           StencilArgs<double> a = residual_args(P);
           a.V = P->at<double>(P->o_V);
           a.diag = P->at<double>(P->o_diag);
           a.out = P->vec(kZ);
-          launch_stencil<double, true, double>(B, a, s);
+          tile_stencil<double, true>(P, nullptr, a, s);
         }
         break;
       }
@@ -1451,8 +1465,8 @@ static cudaError_t rk_iter(a2d_plan* P, const double* circ, const double* forcin
     a.circ_in = circ;
     a.out = R;
     a.sign = 1.0;
-    if (fp32) launch_stencil<float, false, double>(B, a, s);
-    else launch_stencil<double, false, double>(B, a, s);
+    if (fp32) tile_stencil<float, false>(P, nullptr, a, s);
+    else tile_stencil<double, false>(P, nullptr, a, s);
     if (forcing != nullptr) launch_add_forcing(B, R, forcing, s);
     if (irs_fused(P, B, R, U0, U, alphas[st], s)) continue;
     const double* Ruse = R;
@@ -1481,8 +1495,8 @@ static cudaError_t fas_cycle(a2d_plan* P, const double* circ, const double* forc
   a.circ_in = circ;
   a.out = P->vec(kR);
   a.sign = 1.0;
-  if (P->p.precision == A2D_MIXED) launch_stencil<float, false, double>(B, a, s);
-  else launch_stencil<double, false, double>(B, a, s);
+  if (P->p.precision == A2D_MIXED) tile_stencil<float, false>(P, nullptr, a, s);
+  else tile_stencil<double, false>(P, nullptr, a, s);
   if (forcing != nullptr) launch_add_forcing(B, P->vec(kR), forcing, s);
   // coarse start state Uc0 (kept in the coarse plan's JV slot) and forcing (its V slot)
   double* Uc = Cp->vec(kU);
@@ -1493,8 +1507,8 @@ static cudaError_t fas_cycle(a2d_plan* P, const double* circ, const double* forc
   ca.circ_in = circ;
   ca.out = Pc;
   ca.sign = 1.0;
-  if (Cp->p.precision == A2D_MIXED) launch_stencil<float, false, double>(CB, ca, s);
-  else launch_stencil<double, false, double>(CB, ca, s);
+  if (Cp->p.precision == A2D_MIXED) tile_stencil<float, false>(Cp, nullptr, ca, s);
+  else tile_stencil<double, false>(Cp, nullptr, ca, s);
   launch_fas_forcing(B, CB, P->vec(kR), Pc, s);
   if (cudaError_t e = fas_cycle(Cp, circ, Pc, false, s)) return e;
   launch_fas_prolong(B, CB, P->vec(kU), Uc, Uc0, s);

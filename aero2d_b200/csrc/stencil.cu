@@ -143,6 +143,8 @@ template void launch_stencil<double, true, double>(const Batch&, const StencilAr
 void stencil_init_fp64() {
   stencil_cap<double, false, double, kTI, kTJ>();
   stencil_cap<double, true, double, kTI, kTJ>();
+  stencil_cap<double, false, double, 16, 4>();
+  stencil_cap<double, true, double, 16, 4>();
 }
 
 void launch_forces(const Batch& b, const double* U, double* coef, double* cp, const long long* cp_off,

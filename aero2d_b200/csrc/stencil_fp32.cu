@@ -24,10 +24,12 @@ static void caps_of() {
   stencil_cap<float, true, VT, 32, 16>();
   stencil_cap<float, true, VT, 64, 4>();
   stencil_cap<float, true, VT, 16, 16>();
+  stencil_cap<float, true, VT, 16, 4>();
 }
 
 void stencil_init_fp32() {
   stencil_cap<float, false, double, kTI, kTJ>();
+  stencil_cap<float, false, double, 16, 4>();
   caps_of<double>();
   caps_of<float>();
   caps_of<__nv_bfloat16>();

@@ -363,7 +363,8 @@ void launch_stencil(const Batch& b, const StencilArgs<VT>& a, cudaStream_t s, in
       default: break;
     }
   }
-  launch_stencil_shape<T, LIN, VT, kTI, kTJ>(b, a, s);
+  if (shape == kTile16x4) launch_stencil_shape<T, LIN, VT, 16, 4>(b, a, s);
+  else launch_stencil_shape<T, LIN, VT, kTI, kTJ>(b, a, s);
 }
 
 }  // namespace a2d

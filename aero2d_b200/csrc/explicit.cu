@@ -13,6 +13,7 @@
 
 #include "batch.cuh"
 #include "explicit.cuh"
+#include "launch.cuh"
 #include "physics.cuh"
 
 namespace a2d {
@@ -40,6 +41,7 @@ __device__ __forceinline__ T local_dt_cell(const GridDev& g, const State4<T>& W,
 template <typename T>
 __global__ void __launch_bounds__(256) k_local_dt(Batch b, const double* __restrict__ U, double* __restrict__ U0,
                                                   double* __restrict__ dt, double cfl) {
+  grid_wait();
   const Tile t = b.tiles[blockIdx.x];
   const CaseDev cs = b.cases[t.cs];
   const GridDev& g = cs.g;
@@ -76,6 +78,7 @@ __global__ void __launch_bounds__(256) k_local_dt_prim(GridDev g, const double* 
 template <typename T>
 __global__ void __launch_bounds__(256) k_irs_i(Batch b, const double* __restrict__ R, double* __restrict__ out,
                                                double e_) {
+  grid_wait();
   const int row = blockIdx.x;   // rows enumerated as (case, k, j) via the row table below
   const int cs_id = blockIdx.y;
   const CaseDev cs = b.cases[cs_id];
@@ -126,6 +129,7 @@ __global__ void __launch_bounds__(256) k_irs_i(Batch b, const double* __restrict
 // The elimination coefficients depend on j only and are formed once per block.
 template <typename T>
 __global__ void __launch_bounds__(128) k_irs_j(Batch b, double* __restrict__ R, double e_) {
+  grid_wait();
   const int cs_id = blockIdx.y;
   const CaseDev cs = b.cases[cs_id];
   const GridDev& g = cs.g;
@@ -267,6 +271,7 @@ template <typename T, bool STAGE>
 __global__ void __launch_bounds__(256) k_irs(Batch b, const double* __restrict__ R, const double* __restrict__ U0,
                                              const double* __restrict__ dt, double* __restrict__ out,
                                              const double* __restrict__ tab, double e_, double a) {
+  grid_wait();
   const CaseDev cs = b.cases[blockIdx.z];
   const GridDev& g = cs.g;
   const int ni = g.ni, nc = g.nc, c0 = blockIdx.x * kIrsCols, comp = blockIdx.y;
@@ -416,6 +421,7 @@ template <typename T>
 __global__ void __launch_bounds__(256) k_rk_stage(Batch b, const double* __restrict__ U0,
                                                   const double* __restrict__ R, const double* __restrict__ dt,
                                                   double* __restrict__ U, double a) {
+  grid_wait();
   const Tile t = b.tiles[blockIdx.x];
   const CaseDev cs = b.cases[t.cs];
   const GridDev& g = cs.g;
@@ -437,6 +443,7 @@ __global__ void __launch_bounds__(256) k_rk_stage(Batch b, const double* __restr
 __global__ void __launch_bounds__(256) k_rk_res(Batch b, const double* __restrict__ U0,
                                                 const double* __restrict__ U, const double* __restrict__ dt,
                                                 double* __restrict__ tpart) {
+  grid_wait();
   const Tile t = b.tiles[blockIdx.x];
   const CaseDev cs = b.cases[t.cs];
   const GridDev& g = cs.g;
@@ -465,6 +472,7 @@ __global__ void __launch_bounds__(256) k_rk_res(Batch b, const double* __restric
 // block per case, the tiles' sums fetched together and added in order
 __global__ void __launch_bounds__(128) k_rk_finish(Batch b, const double* tpart, const double* coef, double* res,
                                                    double* circ) {
+  grid_wait();
   __shared__ double part[128];
   const int cs = blockIdx.x;
   const CaseDev c = b.cases[cs];
@@ -494,6 +502,7 @@ __global__ void __launch_bounds__(128) k_rk_finish(Batch b, const double* tpart,
 // ---------------------------------------------------------------------------
 // R += P over the cells of every case (the forcing term of a coarse level)
 __global__ void __launch_bounds__(256) k_add_forcing(Batch b, double* __restrict__ R, const double* __restrict__ P) {
+  grid_wait();
   const Tile t = b.tiles[blockIdx.x];
   const CaseDev cs = b.cases[t.cs];
   const size_t base = 4 * cs.cell_off;
@@ -517,6 +526,7 @@ __device__ __forceinline__ double sum4(double a00, double a10, double a01, doubl
 // residual at Uc0) and P (nullable) is the fine level's own forcing
 __global__ void __launch_bounds__(256) k_fas_restrict(Batch fb, Batch cb, const double* __restrict__ Uf,
                                                      double* __restrict__ Uc, double* __restrict__ Uc0) {
+  grid_wait();
   const Tile t = cb.tiles[blockIdx.x];
   const CaseDev cc = cb.cases[t.cs];
   const CaseDev cf = fb.cases[t.cs];
@@ -546,6 +556,7 @@ __global__ void __launch_bounds__(256) k_fas_restrict(Batch fb, Batch cb, const 
 // the fine level's forcing
 __global__ void __launch_bounds__(256) k_fas_forcing(Batch fb, Batch cb, const double* __restrict__ Rf,
                                                     double* __restrict__ Pc) {
+  grid_wait();
   const Tile t = cb.tiles[blockIdx.x];
   const CaseDev cc = cb.cases[t.cs];
   const CaseDev cf = fb.cases[t.cs];
@@ -571,6 +582,7 @@ __global__ void __launch_bounds__(256) k_fas_forcing(Batch fb, Batch cb, const d
 __global__ void __launch_bounds__(256) k_fas_prolong(Batch fb, Batch cb, double* __restrict__ Uf,
                                                     const double* __restrict__ Uc,
                                                     const double* __restrict__ Uc0) {
+  grid_wait();
   const Tile t = fb.tiles[blockIdx.x];
   const CaseDev cf = fb.cases[t.cs];
   const CaseDev cc = cb.cases[t.cs];
@@ -598,8 +610,8 @@ __global__ void __launch_bounds__(256) k_fas_prolong(Batch fb, Batch cb, double*
 
 void launch_local_dt(const Batch& b, const double* U, double* U0, double* dt, double cfl, bool fp32, cudaStream_t s) {
   if (b.ntiles == 0) return;
-  if (fp32) k_local_dt<float><<<b.ntiles, 256, 0, s>>>(b, U, U0, dt, cfl);
-  else k_local_dt<double><<<b.ntiles, 256, 0, s>>>(b, U, U0, dt, cfl);
+  if (fp32) launch(k_local_dt<float>, b.ntiles, 256, 0, s, b, U, U0, dt, cfl);
+  else launch(k_local_dt<double>, b.ntiles, 256, 0, s, b, U, U0, dt, cfl);
 }
 void launch_local_dt_prim(const GridDev& g, const double* W, double* dt, double cfl, cudaStream_t s) {
   const size_t N = (size_t)g.ni * g.nc;
@@ -613,11 +625,11 @@ void launch_irs(const Batch& b, double* R, double* tmp, double e, int max_ni, in
   const size_t sm = (size_t)(max_ni + max_ni / 2 + 2) * sizeof(double);
   dim3 gj((4 * max_ni + 127) / 128, b.ncases);
   if (fp32) {
-    k_irs_i<float><<<gi, 256, sm, s>>>(b, R, tmp, e);
-    k_irs_j<float><<<gj, 128, (size_t)max_nc * sizeof(double), s>>>(b, tmp, e);
+    launch(k_irs_i<float>, gi, 256, sm, s, b, R, tmp, e);
+    launch(k_irs_j<float>, gj, 128, (size_t)max_nc * sizeof(double), s, b, tmp, e);
   } else {
-    k_irs_i<double><<<gi, 256, sm, s>>>(b, R, tmp, e);
-    k_irs_j<double><<<gj, 128, (size_t)max_nc * sizeof(double), s>>>(b, tmp, e);
+    launch(k_irs_i<double>, gi, 256, sm, s, b, R, tmp, e);
+    launch(k_irs_j<double>, gj, 128, (size_t)max_nc * sizeof(double), s, b, tmp, e);
   }
 }
 void launch_irs_table(const Batch& b, double* tab, double e, bool fp32, cudaStream_t s) {
@@ -627,7 +639,7 @@ void launch_irs_table(const Batch& b, double* tab, double e, bool fp32, cudaStre
 }
 template <typename T, bool STAGE>
 static void irs_launch(const Batch& b, const IrsArgs& p, size_t smem, cudaStream_t s) {
-  k_irs<T, STAGE><<<dim3((p.max_ni + kIrsCols - 1) / kIrsCols, 4, b.ncases), 256, smem, s>>>(b, p.R, p.U0, p.dt, p.out,
+  launch(k_irs<T, STAGE>, dim3((p.max_ni + kIrsCols - 1) / kIrsCols, 4, b.ncases), 256, smem, s, b, p.R, p.U0, p.dt, p.out,
                                                                                             p.tab, p.e, p.a);
 }
 void launch_irs_fused(const Batch& b, const IrsArgs& p, bool fp32, cudaStream_t s) {
@@ -660,31 +672,31 @@ cudaError_t irs_init() {
 void launch_rk_stage(const Batch& b, const double* U0, const double* R, const double* dt, double* U, double a,
                      bool fp32, cudaStream_t s) {
   if (b.ntiles == 0) return;
-  if (fp32) k_rk_stage<float><<<b.ntiles, 256, 0, s>>>(b, U0, R, dt, U, a);
-  else k_rk_stage<double><<<b.ntiles, 256, 0, s>>>(b, U0, R, dt, U, a);
+  if (fp32) launch(k_rk_stage<float>, b.ntiles, 256, 0, s, b, U0, R, dt, U, a);
+  else launch(k_rk_stage<double>, b.ntiles, 256, 0, s, b, U0, R, dt, U, a);
 }
 void launch_rk_res(const Batch& b, const double* U0, const double* U, const double* dt, double* tpart,
                    cudaStream_t s) {
-  if (b.ntiles) k_rk_res<<<b.ntiles, 256, 0, s>>>(b, U0, U, dt, tpart);
+  if (b.ntiles) launch(k_rk_res, b.ntiles, 256, 0, s, b, U0, U, dt, tpart);
 }
 void launch_rk_finish(const Batch& b, const double* tpart, const double* coef, double* res, double* circ,
                       cudaStream_t s) {
-  if (b.ncases) k_rk_finish<<<b.ncases, 128, 0, s>>>(b, tpart, coef, res, circ);
+  if (b.ncases) launch(k_rk_finish, b.ncases, 128, 0, s, b, tpart, coef, res, circ);
 }
 
 void launch_add_forcing(const Batch& b, double* R, const double* P, cudaStream_t s) {
-  if (b.ntiles) k_add_forcing<<<b.ntiles, 256, 0, s>>>(b, R, P);
+  if (b.ntiles) launch(k_add_forcing, b.ntiles, 256, 0, s, b, R, P);
 }
 void launch_fas_restrict(const Batch& fine, const Batch& coarse, const double* Uf, double* Uc, double* Uc0,
                          cudaStream_t s) {
-  if (coarse.ntiles) k_fas_restrict<<<coarse.ntiles, 256, 0, s>>>(fine, coarse, Uf, Uc, Uc0);
+  if (coarse.ntiles) launch(k_fas_restrict, coarse.ntiles, 256, 0, s, fine, coarse, Uf, Uc, Uc0);
 }
 void launch_fas_forcing(const Batch& fine, const Batch& coarse, const double* Rf, double* Pc, cudaStream_t s) {
-  if (coarse.ntiles) k_fas_forcing<<<coarse.ntiles, 256, 0, s>>>(fine, coarse, Rf, Pc);
+  if (coarse.ntiles) launch(k_fas_forcing, coarse.ntiles, 256, 0, s, fine, coarse, Rf, Pc);
 }
 void launch_fas_prolong(const Batch& fine, const Batch& coarse, double* Uf, const double* Uc, const double* Uc0,
                         cudaStream_t s) {
-  if (fine.ntiles) k_fas_prolong<<<fine.ntiles, 256, 0, s>>>(fine, coarse, Uf, Uc, Uc0);
+  if (fine.ntiles) launch(k_fas_prolong, fine.ntiles, 256, 0, s, fine, coarse, Uf, Uc, Uc0);
 }
 
 }  // namespace a2d

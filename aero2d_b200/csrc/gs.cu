@@ -43,6 +43,7 @@
 
 #include "batch.cuh"
 #include "gs.cuh"
+#include "launch.cuh"
 
 namespace a2d {
 
@@ -406,6 +407,7 @@ __device__ __forceinline__ void subtract_ring(Ring<TB>& ring, const double* coef
 // pass 1 -----------------------------------------------------------------------
 template <typename TB, bool SPLIT>
 __global__ void __launch_bounds__(32 * warps_of(SPLIT), SPLIT ? 4 : (sizeof(TB) == 8 ? 2 : 3)) k_gs_dots(Batch b, GsArgs<TB> a) {
+  grid_wait();
   extern __shared__ __align__(16) unsigned char gs_sm[];
   __shared__ double rowsum[SPLIT ? 1 : kRows][kMaxRestart + 1];
   const Chunk ch = b.chunks[blockIdx.x];
@@ -453,6 +455,7 @@ __host__ __device__ inline size_t gs_tile_bytes(int nq) {
 
 template <typename TB, bool SPLIT>
 __global__ void __launch_bounds__(32 * warps_of(SPLIT), SPLIT ? 4 : (sizeof(TB) == 8 ? 2 : 3)) k_gs_project(Batch b, GsArgs<TB> a) {
+  grid_wait();
   constexpr bool kTile = SPLIT && !std::is_same<TB, double>::value;
   extern __shared__ __align__(16) unsigned char gs_sm[];
   __shared__ double rowsum[SPLIT ? 1 : kRows][kMaxRestart + 1];
@@ -521,6 +524,7 @@ __global__ void __launch_bounds__(32 * warps_of(SPLIT), SPLIT ? 4 : (sizeof(TB) 
 // pass 3 -----------------------------------------------------------------------
 template <typename TB, bool SPLIT>
 __global__ void __launch_bounds__(32 * warps_of(SPLIT), SPLIT ? 4 : (sizeof(TB) == 8 ? 2 : 3)) k_gs_sub(Batch b, GsArgs<TB> a) {
+  grid_wait();
   extern __shared__ __align__(16) unsigned char gs_sm[];
   __shared__ double xs[SPLIT ? kChain * 32 : 1];   // w'' of the row, [chain index][lane]
   __shared__ double rowsum[SPLIT ? 1 : kRows][kMaxRestart + 1];
@@ -592,6 +596,7 @@ __device__ __forceinline__ void stv(__nv_bfloat16* p, const double (&v)[4]) {
 
 template <typename TB>
 __global__ void __launch_bounds__(kGB) k_gs_start(Batch b, GsArgs<TB> a) {
+  grid_wait();
   const Chunk ch = b.chunks[blockIdx.x];
   if (!case_live(b, ch.cs, a.need)) return;
   const CaseDev cs = b.cases[ch.cs];
@@ -624,6 +629,7 @@ __global__ void __launch_bounds__(kGB) k_gs_start(Batch b, GsArgs<TB> a) {
 // per-case close of an Arnoldi step (k >= 0) or of the start vector (k = -1),
 // one warp per case ----
 __global__ void __launch_bounds__(32) k_gs_close(Batch b, GsCloseArgs a) {
+  grid_wait();
   const int cs_id = blockIdx.x;
   if ((a.live[cs_id] & a.need) != a.need) return;
   const CaseDev cs = b.cases[cs_id];
@@ -673,7 +679,7 @@ static void launch_pass(void (*split)(Batch, GsArgs<TB>), void (*whole)(Batch, G
                         const Batch& b, const GsArgs<TB>& a, cudaStream_t s) {
   if (!b.nchunks) return;
   if (!gs_split(b.nchunks)) {
-    whole<<<b.nchunks, 32 * warps_of(false), kRows * Ring<TB>::kBytes, s>>>(b, a);
+    launch(whole, b.nchunks, 32 * warps_of(false), kRows * Ring<TB>::kBytes, s, b, a);
     return;
   }
   cudaLaunchConfig_t cfg = {};
@@ -681,13 +687,14 @@ static void launch_pass(void (*split)(Batch, GsArgs<TB>), void (*whole)(Batch, G
   cfg.blockDim = dim3(32 * warps_of(true));
   cfg.dynamicSmemBytes = split_smem;
   cfg.stream = s;
-  cudaLaunchAttribute at[1];
+  cudaLaunchAttribute at[2];
   at[0].id = cudaLaunchAttributeClusterDimension;
   at[0].val.clusterDim.x = 1;
   at[0].val.clusterDim.y = kRows;
   at[0].val.clusterDim.z = 1;
+  at[1] = dependent_launch();
   cfg.attrs = at;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = 2;
   (void)cudaLaunchKernelEx(&cfg, split, b, a);   // as <<<>>>: see cudaGetLastError
 }
 template <typename TB>
@@ -704,10 +711,10 @@ void launch_gs_finish(const Batch& b, const GsArgs<TB>& a, cudaStream_t s) {
 }
 template <typename TB>
 void launch_gs_start(const Batch& b, const GsArgs<TB>& a, cudaStream_t s) {
-  if (b.nchunks) k_gs_start<TB><<<b.nchunks, kGB, 0, s>>>(b, a);
+  if (b.nchunks) launch(k_gs_start<TB>, b.nchunks, kGB, 0, s, b, a);
 }
 void launch_gs_close(const Batch& b, const GsCloseArgs& a, cudaStream_t s) {
-  if (b.ncases) k_gs_close<<<b.ncases, 32, 0, s>>>(b, a);
+  if (b.ncases) launch(k_gs_close, b.ncases, 32, 0, s, b, a);
 }
 
 #define A2D_GS_INST(TB)                                                                 \

@@ -13,6 +13,7 @@
 
 #include "batch.cuh"
 #include "krylov.cuh"
+#include "launch.cuh"
 #include "physics.cuh"
 
 namespace a2d {
@@ -72,6 +73,7 @@ constexpr int kPer = kChunk / kVB;       // entries per thread
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(32) k_lstsq(int ncases, const uint32_t* live, CaseCtl* ctl, const double* Hall,
                                               double* yall) {
+  grid_wait();
   const int cs = blockIdx.x;
   if (!(live[cs] & kLiveNewton)) return;
   const int k = ctl[cs].k_used;
@@ -124,6 +126,7 @@ __device__ __forceinline__ double basis_f64(__nv_bfloat16 v) { return __bfloat16
 
 template <typename TB>
 __global__ void __launch_bounds__(kVB) k_combine(Batch b, CombineArgs<TB> a) {
+  grid_wait();
   const Chunk ch = b.chunks[blockIdx.x];
   if (!case_live(b, ch.cs, a.need)) return;
   const CaseDev cs = b.cases[ch.cs];
@@ -147,6 +150,7 @@ __global__ void __launch_bounds__(kVB) k_combine(Batch b, CombineArgs<TB> a) {
 
 // per-case norms of b and x0 -> ptol (jax gmres: ptol = ||M b|| * min(1, tol ||b|| / ||b||))
 __global__ void k_gm_setup(Batch b, const double* part, int pstride, CaseCtl* ctl, double gtol) {
+  grid_wait();
   const int cs = blockIdx.x * blockDim.x + threadIdx.x;
   if (cs >= b.ncases) return;
   if (!case_live(b, cs, kLiveNewton)) return;
@@ -166,6 +170,7 @@ __global__ void k_gm_setup(Batch b, const double* part, int pstride, CaseCtl* ct
 // two squared norms per chunk (||b||^2, ||x0||^2)
 __global__ void __launch_bounds__(kVB) k_norms2(Batch b, const double* x, const double* y, double* part,
                                                 int pstride, uint32_t need) {
+  grid_wait();
   const Chunk ch = b.chunks[blockIdx.x];
   if (!case_live(b, ch.cs, need)) return;
   const CaseDev cs = b.cases[ch.cs];
@@ -186,6 +191,7 @@ __global__ void __launch_bounds__(kVB) k_norms2(Batch b, const double* x, const 
 
 // squared norm per chunk
 __global__ void __launch_bounds__(kVB) k_norm1(Batch b, const double* x, double* part, uint32_t need) {
+  grid_wait();
   const Chunk ch = b.chunks[blockIdx.x];
   if (!case_live(b, ch.cs, need)) return;
   const CaseDev cs = b.cases[ch.cs];
@@ -203,6 +209,7 @@ __global__ void __launch_bounds__(kVB) k_norm1(Batch b, const double* x, double*
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(256) k_update_rel(Batch b, const double* U, const double* dU,
                                                     double* tpart, uint32_t need) {
+  grid_wait();
   const Tile t = b.tiles[blockIdx.x];
   if (!case_live(b, t.cs, need)) return;
   const CaseDev cs = b.cases[t.cs];
@@ -231,6 +238,7 @@ __global__ void __launch_bounds__(256) k_update_rel(Batch b, const double* U, co
 __global__ void __launch_bounds__(256) k_update_check(Batch b, const double* U, const double* dU,
                                                       double* tpart, CaseCtl* ctl, double max_update,
                                                       uint32_t need) {
+  grid_wait();
   const Tile t = b.tiles[blockIdx.x];
   if (!case_live(b, t.cs, need)) return;
   const CaseDev cs = b.cases[t.cs];
@@ -264,6 +272,7 @@ __global__ void __launch_bounds__(256) k_update_check(Batch b, const double* U, 
 
 __global__ void k_controller(Batch b, const double* tpart, CaseCtl* ctl, uint32_t* live, double* hist_rn,
                              int hist_cap, CtlParams p) {
+  grid_wait();
   const int cs = blockIdx.x * blockDim.x + threadIdx.x;
   if (cs >= b.ncases) return;
   if (!(live[cs] & kLiveNewton)) return;
@@ -300,6 +309,7 @@ __global__ void k_controller(Batch b, const double* tpart, CaseCtl* ctl, uint32_
 
 __global__ void __launch_bounds__(256) k_commit(Batch b, double* U, const double* dU, const CaseCtl* ctl,
                                                 uint32_t need_mask_unused) {
+  grid_wait();
   const Tile t = b.tiles[blockIdx.x];
   const CaseCtl& s = ctl[t.cs];
   if (!s.commit || !s.stepped) return;
@@ -319,6 +329,7 @@ __global__ void __launch_bounds__(256) k_commit(Batch b, double* U, const double
 
 // marks which cases take this step (before the controller may retire them)
 __global__ void k_mark_stepped(int ncases, const uint32_t* live, CaseCtl* ctl) {
+  grid_wait();
   const int cs = blockIdx.x * blockDim.x + threadIdx.x;
   if (cs >= ncases) return;
   ctl[cs].stepped = (live[cs] & kLiveNewton) ? 1 : 0;
@@ -329,39 +340,39 @@ __global__ void k_mark_stepped(int ncases, const uint32_t* live, CaseCtl* ctl) {
 // launchers
 template <typename TB>
 void launch_combine(const Batch& b, const CombineArgs<TB>& a, cudaStream_t s) {
-  if (b.nchunks) k_combine<TB><<<b.nchunks, kVB, 0, s>>>(b, a);
+  if (b.nchunks) launch(k_combine<TB>, b.nchunks, kVB, 0, s, b, a);
 }
 void launch_lstsq(const Batch& b, const uint32_t* live, CaseCtl* ctl, double* H, double* y, cudaStream_t s) {
-  k_lstsq<<<b.ncases, 32, 0, s>>>(b.ncases, live, ctl, H, y);
+  launch(k_lstsq, b.ncases, 32, 0, s, b.ncases, live, ctl, H, y);
 }
 void launch_gm_setup(const Batch& b, const double* part, int pstride, CaseCtl* ctl, double gtol,
                      cudaStream_t s) {
-  k_gm_setup<<<(b.ncases + 63) / 64, 64, 0, s>>>(b, part, pstride, ctl, gtol);
+  launch(k_gm_setup, (b.ncases + 63) / 64, 64, 0, s, b, part, pstride, ctl, gtol);
 }
 void launch_norms2(const Batch& b, const double* x, const double* y, double* part, int pstride,
                    uint32_t need, cudaStream_t s) {
-  if (b.nchunks) k_norms2<<<b.nchunks, kVB, 0, s>>>(b, x, y, part, pstride, need);
+  if (b.nchunks) launch(k_norms2, b.nchunks, kVB, 0, s, b, x, y, part, pstride, need);
 }
 void launch_norm1(const Batch& b, const double* x, double* part, uint32_t need, cudaStream_t s) {
-  if (b.nchunks) k_norm1<<<b.nchunks, kVB, 0, s>>>(b, x, part, need);
+  if (b.nchunks) launch(k_norm1, b.nchunks, kVB, 0, s, b, x, part, need);
 }
 void launch_update_rel(const Batch& b, const double* U, const double* dU, double* tpart, uint32_t need,
                        cudaStream_t s) {
-  if (b.ntiles) k_update_rel<<<b.ntiles, 256, 0, s>>>(b, U, dU, tpart, need);
+  if (b.ntiles) launch(k_update_rel, b.ntiles, 256, 0, s, b, U, dU, tpart, need);
 }
 void launch_update_check(const Batch& b, const double* U, const double* dU, double* tpart, CaseCtl* ctl,
                          double max_update, uint32_t need, cudaStream_t s) {
-  if (b.ntiles) k_update_check<<<b.ntiles, 256, 0, s>>>(b, U, dU, tpart, ctl, max_update, need);
+  if (b.ntiles) launch(k_update_check, b.ntiles, 256, 0, s, b, U, dU, tpart, ctl, max_update, need);
 }
 void launch_controller(const Batch& b, const double* tpart, CaseCtl* ctl, uint32_t* live, double* hist_rn,
                        int hist_cap, const CtlParams& p, cudaStream_t s) {
-  k_controller<<<(b.ncases + 63) / 64, 64, 0, s>>>(b, tpart, ctl, live, hist_rn, hist_cap, p);
+  launch(k_controller, (b.ncases + 63) / 64, 64, 0, s, b, tpart, ctl, live, hist_rn, hist_cap, p);
 }
 void launch_commit(const Batch& b, double* U, const double* dU, const CaseCtl* ctl, cudaStream_t s) {
-  if (b.ntiles) k_commit<<<b.ntiles, 256, 0, s>>>(b, U, dU, ctl, 0);
+  if (b.ntiles) launch(k_commit, b.ntiles, 256, 0, s, b, U, dU, ctl, 0);
 }
 void launch_mark_stepped(const Batch& b, const uint32_t* live, CaseCtl* ctl, cudaStream_t s) {
-  k_mark_stepped<<<(b.ncases + 63) / 64, 64, 0, s>>>(b.ncases, live, ctl);
+  launch(k_mark_stepped, (b.ncases + 63) / 64, 64, 0, s, b.ncases, live, ctl);
 }
 
 template void launch_combine<double>(const Batch&, const CombineArgs<double>&, cudaStream_t);

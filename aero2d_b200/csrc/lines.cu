@@ -35,6 +35,7 @@
 
 #include "batch.cuh"
 #include "kernels.cuh"
+#include "launch.cuh"
 #include "tma.cuh"
 
 namespace a2d {
@@ -665,6 +666,7 @@ __device__ __forceinline__ bool recur(const Cta<TI> c, const SweepArgs& a, size_
 template <typename TI>
 __global__ void __launch_bounds__(kThreads, Types<TI>::kCtas) k_lines(Batch b, SweepArgs a, const int* cases, int sweeps,
                                                        int rows_cap) {
+  grid_wait();
   using SM = Smem<TI>;
   constexpr int S = Types<TI>::kStages;
   const uint32_t size = cluster_size(), rank = cluster_rank();
@@ -723,7 +725,7 @@ __global__ void __launch_bounds__(kThreads, Types<TI>::kCtas) k_lines(Batch b, S
 template <typename TI>
 struct LinesLaunch {
   cudaLaunchConfig_t cfg = {};
-  cudaLaunchAttribute at[1];
+  cudaLaunchAttribute at[2];
   LinesLaunch(int count, int groups, int rows, cudaStream_t s) {
     cfg.gridDim = dim3((unsigned)(count * groups));
     cfg.blockDim = dim3(lines::kThreads);
@@ -732,8 +734,9 @@ struct LinesLaunch {
     at[0].id = cudaLaunchAttributeClusterDimension;
     at[0].val.clusterDim.x = (unsigned)groups;
     at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    at[1] = dependent_launch();
     cfg.attrs = at;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = 2;
   }
 };
 

@@ -18,6 +18,7 @@
 // kernel streams with bulk copies.
 #include "batch.cuh"
 #include "kernels.cuh"
+#include "launch.cuh"
 #include "physics.cuh"
 
 namespace a2d {
@@ -76,6 +77,7 @@ __device__ __forceinline__ void store_block(TS* base, long long row0, int rows, 
 
 template <typename T>
 __global__ void __launch_bounds__(256) k_face_jac(Batch b, JacArgs a) {
+  grid_wait();
   const Tile t = b.tiles[blockIdx.x];
   if (!case_live(b, t.cs, a.need)) return;
   const CaseDev cs = b.cases[t.cs];
@@ -221,6 +223,7 @@ __device__ __forceinline__ void mul4_store(const double A[16], const double B[16
 // eliminations after each other.
 template <typename TJ, typename TF>
 __global__ void __launch_bounds__(128) k_factor(Batch b, FactorArgs a) {
+  grid_wait();
   __shared__ double cfar[2][16][kLanes];   // per group of the CTA: c'_{k+1} of each line
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int pair = warp >> 1;              // group slot of the CTA
@@ -403,12 +406,12 @@ __global__ void __launch_bounds__(128) k_factor(Batch b, FactorArgs a) {
 template <typename T>
 void launch_face_jac(const Batch& b, const JacArgs& a, cudaStream_t s) {
   if (b.ntiles == 0) return;
-  k_face_jac<T><<<b.ntiles, 256, 0, s>>>(b, a);
+  launch(k_face_jac<T>, b.ntiles, 256, 0, s, b, a);
 }
 template <typename TJ, typename TF>
 void launch_factor(const Batch& b, const FactorArgs& a, cudaStream_t s) {
   if (b.ngroups == 0) return;
-  k_factor<TJ, TF><<<(b.ngroups + 1) / 2, 128, 0, s>>>(b, a);
+  launch(k_factor<TJ, TF>, (b.ngroups + 1) / 2, 128, 0, s, b, a);
 }
 
 template void launch_face_jac<double>(const Batch&, const JacArgs&, cudaStream_t);

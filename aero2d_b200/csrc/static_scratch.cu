@@ -21,6 +21,7 @@
 #include "aero2d_b200.h"
 #include "batch.cuh"
 #include "kernels.cuh"
+#include "launch.cuh"
 
 namespace a2d {
 
@@ -45,6 +46,7 @@ static __device__ __align__(256) unsigned char g_scratch[kStaticScratchBytes];
 // case and tile tables of a uniform batch (every case on one grid), built on the device
 __global__ void k_static_tables(unsigned char* scratch, const void* metrics, int ni, int nc, int ncases,
                                 const double* winf) {
+  grid_wait();
   CaseDev* cases = reinterpret_cast<CaseDev*>(scratch + kOffCases);
   Tile* tiles = reinterpret_cast<Tile*>(scratch + kOffTiles);
   const int nti = (ni + kTI - 1) / kTI, ntj = (nc + kTJ - 1) / kTJ;
@@ -68,6 +70,7 @@ __global__ void k_static_tables(unsigned char* scratch, const void* metrics, int
 
 // rn = sqrt(mean((R_rho / vol)^2)) per case from its tile partials, in tile order
 __global__ void k_static_norms(const unsigned char* scratch, int ncases, int cells, double* rnorm) {
+  grid_wait();
   const CaseDev* cases = reinterpret_cast<const CaseDev*>(scratch + kOffCases);
   const double* part = reinterpret_cast<const double*>(scratch + kOffPart);
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
@@ -160,7 +163,7 @@ extern "C" int a2d_residual_norms_static(const void* metrics, int ni, int nj, in
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const int tpc = ((ni + kTI - 1) / kTI) * ((nc + kTJ - 1) / kTJ);
   const int ntiles = ncases * tpc;
-  k_static_tables<<<(ntiles + 255) / 256, 256, 0, s>>>(scratch, metrics, ni, nc, ncases, winf);
+  launch(k_static_tables, (ntiles + 255) / 256, 256, 0, s, scratch, metrics, ni, nc, ncases, winf);
   Batch b{};
   b.cases = reinterpret_cast<const CaseDev*>(scratch + kOffCases);
   b.tiles = reinterpret_cast<const Tile*>(scratch + kOffTiles);
@@ -177,7 +180,7 @@ extern "C" int a2d_residual_norms_static(const void* metrics, int ni, int nj, in
   a.order = p.order;
   a.vortex = p.vortex_correction;
   launch_stencil<double, false, double>(b, a, s);
-  k_static_norms<<<(ncases + 63) / 64, 64, 0, s>>>(scratch, ncases, ni * nc, rnorm);
+  launch(k_static_norms, (ncases + 63) / 64, 64, 0, s, scratch, ncases, ni * nc, rnorm);
   const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return fail(A2D_ERR_CUDA, std::string("residual_norms_static: ") + cudaGetErrorString(e));
   return A2D_OK;

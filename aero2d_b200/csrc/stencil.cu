@@ -17,6 +17,7 @@
 
 #include "batch.cuh"
 #include "kernels.cuh"
+#include "launch.cuh"
 #include "physics.cuh"
 #include "stencil_impl.cuh"
 
@@ -92,6 +93,7 @@ __global__ void __launch_bounds__(256) k_forces(Batch b, const double* __restric
                                                 double* __restrict__ coef /* [ncases][3] */,
                                                 double* __restrict__ cp_out, const long long* cp_off,
                                                 const CaseCtl* ctl, double* hist_cl, int hist_cap) {
+  grid_wait();
   const int cs_id = blockIdx.x;
   if (!case_live(b, cs_id, 0)) return;
   const CaseDev cs = b.cases[cs_id];
@@ -150,7 +152,7 @@ void stencil_init_fp64() {
 void launch_forces(const Batch& b, const double* U, double* coef, double* cp, const long long* cp_off,
                    const CaseCtl* ctl, double* hist_cl, int hist_cap, cudaStream_t s) {
   if (b.ncases == 0) return;
-  k_forces<<<b.ncases, 256, 0, s>>>(b, U, coef, cp, cp_off, ctl, hist_cl, hist_cap);
+  launch(k_forces, b.ncases, 256, 0, s, b, U, coef, cp, cp_off, ctl, hist_cl, hist_cap);
 }
 
 }  // namespace a2d

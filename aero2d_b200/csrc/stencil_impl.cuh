@@ -8,6 +8,7 @@
 
 #include "batch.cuh"
 #include "kernels.cuh"
+#include "launch.cuh"
 #include "physics.cuh"
 
 namespace a2d {
@@ -318,6 +319,7 @@ __device__ __forceinline__ void stencil_tile(const Batch& b, const StencilArgs<V
 // 28.8 -> 25.7.
 template <typename T, bool LIN, typename VT, int TI, int TJ>
 __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 2) k_stencil(Batch b, StencilArgs<VT> a) {
+  grid_wait();
   for (int tile = blockIdx.x; tile < b.ntiles; tile += gridDim.x) {
     if (tile != (int)blockIdx.x) __syncthreads();   // the previous tile is done with shared memory
     stencil_tile<T, LIN, VT, TI, TJ>(b, a, tile);
@@ -349,7 +351,7 @@ int stencil_cap() {
 template <typename T, bool LIN, typename VT, int TI, int TJ>
 void launch_stencil_shape(const Batch& b, const StencilArgs<VT>& a, cudaStream_t s) {
   const int cap = stencil_cap<T, LIN, VT, TI, TJ>();
-  k_stencil<T, LIN, VT, TI, TJ><<<b.ntiles < cap ? b.ntiles : cap, 256, 0, s>>>(b, a);
+  launch(k_stencil<T, LIN, VT, TI, TJ>, b.ntiles < cap ? b.ntiles : cap, 256, 0, s, b, a);
 }
 
 template <typename T, bool LIN, typename VT>

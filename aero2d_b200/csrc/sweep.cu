@@ -44,6 +44,7 @@
 
 #include "batch.cuh"
 #include "kernels.cuh"
+#include "launch.cuh"
 #include "tma.cuh"
 
 namespace a2d {
@@ -118,6 +119,7 @@ __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.
 
 template <typename TI, bool FIRST, bool LAST>
 __global__ void __launch_bounds__(kSweepThreads) k_sweep(Batch b, SweepArgs a) {
+  grid_wait();
   using SM = SweepSmem<TI>;
   using TF = typename SM::TF;
   using TC = typename SM::TC;
@@ -462,8 +464,8 @@ void launch_sweep(const Batch& b, const SweepArgs& a, bool last, cudaStream_t s,
     launch_sweep_pairs<TI, FIRST>(b, a, last, s);
     return;
   }
-  if (last) k_sweep<TI, FIRST, true><<<b.ngroups, kSweepThreads, sizeof(SweepSmem<TI>), s>>>(b, a);
-  else k_sweep<TI, FIRST, false><<<b.ngroups, kSweepThreads, sizeof(SweepSmem<TI>), s>>>(b, a);
+  if (last) launch(k_sweep<TI, FIRST, true>, b.ngroups, kSweepThreads, sizeof(SweepSmem<TI>), s, b, a);
+  else launch(k_sweep<TI, FIRST, false>, b.ngroups, kSweepThreads, sizeof(SweepSmem<TI>), s, b, a);
 }
 
 cudaError_t sweep_init() {

@@ -24,6 +24,7 @@
 
 #include "batch.cuh"
 #include "kernels.cuh"
+#include "launch.cuh"
 #include "tma.cuh"
 
 namespace a2d {
@@ -106,6 +107,7 @@ __device__ __forceinline__ void full4(int p, const TC (&own)[2], TC (&v)[4]) {
 
 template <typename TI, bool FIRST, bool LAST>
 __global__ void __launch_bounds__(kSweepThreads) k_sweep(Batch b, SweepArgs a) {
+  grid_wait();
   using SM = SweepSmem<TI>;
   using TF = typename SM::TF;
   using TC = typename SM::TC;
@@ -456,8 +458,8 @@ template <typename TI, bool FIRST>
 void launch_sweep_pairs(const Batch& b, const SweepArgs& a, bool last, cudaStream_t s) {
   using namespace pairs;
   if (b.ngroups == 0) return;
-  if (last) k_sweep<TI, FIRST, true><<<b.ngroups, kSweepThreads, sizeof(SweepSmem<TI>), s>>>(b, a);
-  else k_sweep<TI, FIRST, false><<<b.ngroups, kSweepThreads, sizeof(SweepSmem<TI>), s>>>(b, a);
+  if (last) launch(k_sweep<TI, FIRST, true>, b.ngroups, kSweepThreads, sizeof(SweepSmem<TI>), s, b, a);
+  else launch(k_sweep<TI, FIRST, false>, b.ngroups, kSweepThreads, sizeof(SweepSmem<TI>), s, b, a);
 }
 
 cudaError_t sweep_pairs_init() {

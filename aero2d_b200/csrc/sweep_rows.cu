@@ -24,6 +24,7 @@
 
 #include "batch.cuh"
 #include "kernels.cuh"
+#include "launch.cuh"
 #include "tma.cuh"
 
 namespace a2d {
@@ -113,6 +114,7 @@ __device__ __forceinline__ void consumers_sync() {
 
 template <typename TI, bool FIRST, bool LAST>
 __global__ void __launch_bounds__(kSweepThreads, 4) k_sweep(Batch b, SweepArgs a) {
+  grid_wait();
   using SM = SweepSmem<TI>;
   using TF = typename SM::TF;
   using TC = typename SM::TC;
@@ -469,8 +471,8 @@ template <typename TI, bool FIRST>
 void launch_sweep_rows(const Batch& b, const SweepArgs& a, bool last, cudaStream_t s) {
   using namespace rows;
   if (b.ngroups == 0) return;
-  if (last) k_sweep<TI, FIRST, true><<<b.ngroups, kSweepThreads, sizeof(SweepSmem<TI>), s>>>(b, a);
-  else k_sweep<TI, FIRST, false><<<b.ngroups, kSweepThreads, sizeof(SweepSmem<TI>), s>>>(b, a);
+  if (last) launch(k_sweep<TI, FIRST, true>, b.ngroups, kSweepThreads, sizeof(SweepSmem<TI>), s, b, a);
+  else launch(k_sweep<TI, FIRST, false>, b.ngroups, kSweepThreads, sizeof(SweepSmem<TI>), s, b, a);
 }
 
 cudaError_t sweep_rows_init() {

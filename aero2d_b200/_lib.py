@@ -87,6 +87,8 @@ SIGNATURES = {
     "a2d_vec_set": (_I, [_P, _I, _I, _P, _P]),
     "a2d_vec_get": (_I, [_P, _I, _I, _P, _P]),
     "a2d_vec_get_prim": (_I, [_P, _I, _I, _P, _P]),
+    "a2d_batch_set": (_I, [_P, _I, _P, _P]),
+    "a2d_batch_get": (_I, [_P, _I, _P, _P]),
     "a2d_local_dt": (_I, [_P, _I, _P, _P, _P]),
     "a2d_init_freestream": (_I, [_P, _P]),
     "a2d_reset": (_I, [_P, _P]),

@@ -176,11 +176,24 @@ class Plan:
             _lib.check(self.lib.a2d_local_dt(self.handle, k, _ptr(W), _ptr(dt), self.stream))
         return dt
 
+    def _uniform(self) -> bool:
+        return len(set(self.shapes)) == 1
+
     def set_batch(self, slot: int, U: torch.Tensor) -> None:
+        # a tensor that is the cases' vectors one after another goes in with one launch
+        if (isinstance(U, torch.Tensor) and U.dtype == torch.float64 and U.device == self.device and U.is_contiguous()
+                and self._uniform() and tuple(U.shape) == (self.B, 4, *self.shapes[0])):
+            self.call("a2d_batch_set", slot, _ptr(U))
+            self._keep = U
+            return
         for k in range(self.B):
             self.set_vec(slot, k, U[k])
 
     def get_batch(self, slot: int) -> torch.Tensor:
+        if self._uniform():
+            out = torch.empty((self.B, 4, *self.shapes[0]), dtype=torch.float64, device=self.device)
+            self.call("a2d_batch_get", slot, _ptr(out))
+            return out
         return torch.stack([self.get_vec(slot, k) for k in range(self.B)])
 
     # -- operations ------------------------------------------------------------

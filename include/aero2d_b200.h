@@ -103,7 +103,7 @@ int a2d_plan_ncases(const a2d_plan* plan);
  * (aero2d_b200.autotune); no counterpart in the reference.  Results do not depend on
  * them: every variant computes the same arithmetic in the same order. ---- */
 #define A2D_JVP_TILE_32x8 0     /* tile shape (i x j cells) of the FP32 JVP stencil; FP64 plans */
-#define A2D_JVP_TILE_32x16 1    /* always use 32 x 8 */
+#define A2D_JVP_TILE_32x16 1    /* use 32 x 8; small batches, FP64 or at 32x16, use 16 x 4  */
 #define A2D_JVP_TILE_64x4 2
 #define A2D_JVP_TILE_16x16 3
 #define A2D_SWEEP_LANES 0       /* a launch per sweep: one warp per half line group, a lane per line;   */
@@ -122,6 +122,9 @@ int a2d_plan_get_tuning(const a2d_plan* plan, int* jvp_tile, int* sweep_variant)
 /* vector I/O in the reference layout [4][ni][nc] of one case (device pointers) */
 int a2d_vec_set(a2d_plan* plan, int slot, int case_index, const double* src, void* stream);
 int a2d_vec_get(const a2d_plan* plan, int slot, int case_index, double* dst, void* stream);
+/* the vectors of all cases, one after another, each in the reference layout: one launch */
+int a2d_batch_set(a2d_plan* plan, int slot, const double* src, void* stream);
+int a2d_batch_get(const a2d_plan* plan, int slot, double* dst, void* stream);
 /* primitives (rho, u, v, p) = cons_to_prim of a slot's vector of one case (euler.py:66-71),
  * in the reference layout [4][ni][nc]: the W that EulerSolver.residual returns (euler.py:260) */
 int a2d_vec_get_prim(const a2d_plan* plan, int slot, int case_index, double* dst, void* stream);

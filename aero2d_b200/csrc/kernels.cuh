@@ -76,6 +76,7 @@ struct FactorArgs {
   double* diag = nullptr;          // per-cell vol / dtau
   double cfl_base = 2.5;           // EulerSolver.cfl, which local_dt multiplies and step() divides out
   unsigned long long* sat = nullptr; // counts factor entries saturated by the FP16 store
+  uint32_t* err = nullptr;         // set when a bounded wait inside the kernel runs out
   uint32_t need = 0;
 };
 
@@ -116,6 +117,7 @@ void launch_forces(const Batch& b, const double* U, double* coef, double* cp, co
 template <typename T>
 void launch_face_jac(const Batch& b, const JacArgs& a, cudaStream_t s);
 
+cudaError_t factor_init();   // once, before the first launch_factor
 template <typename TJ, typename TF>
 void launch_factor(const Batch& b, const FactorArgs& a, cudaStream_t s);
 

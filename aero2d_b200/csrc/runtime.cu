@@ -255,7 +255,7 @@ static void layout(a2d_plan* P) {
   P->o_cp = cv.take(8 * (size_t)P->total_ni);
   P->o_hrn = cv.take(8 * (size_t)B * P->p.max_iter);
   P->o_hcl = cv.take(8 * (size_t)B * P->p.max_iter);
-  P->o_cnt = cv.take(8);   // [0] live-case count, [1] sweep copy-wait failure flag
+  P->o_cnt = cv.take(8);   // [0] live-case count, [1] failure flag of the bounded waits of the sweeps and the factors
   P->o_idx = cv.take(sizeof(int) * (size_t)B);   // case index lists of a2d_case_restart / _retire
   P->o_sat = cv.take(sizeof(unsigned long long));
   P->o_jtiles = cv.take(sizeof(Tile) * (size_t)P->max_jtiles);
@@ -448,6 +448,7 @@ static FactorArgs factor_args(const a2d_plan* P, uint32_t need) {
   fa.diag = P->at<double>(P->o_diag);
   fa.cfl_base = P->p.cfl;
   fa.sat = P->at<unsigned long long>(P->o_sat);
+  fa.err = P->at<uint32_t>(P->o_cnt) + 1;
   fa.need = need;
   return fa;
 }
@@ -940,6 +941,7 @@ int a2d_plan_bind(a2d_plan* P, void* workspace, size_t bytes, void* stream) {
   }
   A2D_CK(gs_init());
   A2D_CK(irs_init());
+  A2D_CK(factor_init());
   P->irs_ready = false;
   stencil_init_fp64();
   stencil_init_fp32();

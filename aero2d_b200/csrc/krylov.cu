@@ -67,9 +67,10 @@ constexpr int kPer = kChunk / kVB;       // entries per thread
 // ---------------------------------------------------------------------------
 // Hessenberg least squares min || beta e1 - H y || by Givens rotations (H
 // column k = Arnoldi step k).  One warp per case copies the case's columns
-// into shared memory; its first lane then rotates and back-substitutes there
-// (a sequential chain of dependent updates: in shared memory each costs a few
-// tens of cycles instead of a global-memory round trip).
+// into shared memory; rotation q, formed from column q by every lane, turns the
+// columns beyond it side by side, a lane per column.  What is left in sequence
+// is the k rotations and the back substitution, whose sums keep their order:
+// 50 columns 93 us with one lane doing all, 44 this way, 30 columns 48 and 25.
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(32) k_lstsq(int ncases, const uint32_t* live, CaseCtl* ctl, const double* Hall,
                                               double* yall) {
@@ -80,75 +81,105 @@ __global__ void __launch_bounds__(32) k_lstsq(int ncases, const uint32_t* live, 
   if (k == 0) return;
   constexpr int L = kMaxRestart + 1;
   __shared__ double Hc[kMaxRestart * L];   // column j at Hc[j * L + q]; rotated in place
-  __shared__ double g[L], cr[L], sr[L];
+  __shared__ double g[L], ys[L];
+  const int lane = threadIdx.x;
   const double* Hg = Hall + (size_t)cs * kMaxRestart * L;
-  for (int e = threadIdx.x; e < k * L; e += blockDim.x) Hc[e] = Hg[e];
-  __syncthreads();
-  if (threadIdx.x != 0) return;
-  double* y = yall + (size_t)cs * kMaxRestart;
-  for (int q = 0; q <= k; ++q) g[q] = 0.0;
-  g[0] = ctl[cs].beta;
-  for (int j = 0; j < k; ++j) {
-    double* col = Hc + (size_t)j * L;
-    for (int q = 0; q < j; ++q) {
-      const double t = cr[q] * col[q] + sr[q] * col[q + 1];
-      col[q + 1] = -sr[q] * col[q] + cr[q] * col[q + 1];
-      col[q] = t;
-    }
-    const double a = col[j], c = col[j + 1];
+#pragma unroll 4
+  for (int e = lane; e < k * L; e += 32) Hc[e] = Hg[e];
+  for (int q = lane; q <= k; q += 32) g[q] = q == 0 ? ctl[cs].beta : 0.0;
+  for (int q = 0; q < k; ++q) {
+    __syncwarp();
+    const double* piv = Hc + (size_t)q * L;
+    const double a = piv[q], c = piv[q + 1];
+    const double gj = g[q], gj1 = g[q + 1];
     const double d = hypot(a, c);
     double cc = 1.0, ss = 0.0;
     if (d != 0.0) {
       cc = a / d;
       ss = c / d;
     }
-    cr[j] = cc;
-    sr[j] = ss;
-    col[j] = cc * a + ss * c;
-    col[j + 1] = 0.0;
-    const double gj = g[j], gj1 = g[j + 1];
-    g[j] = cc * gj + ss * gj1;
-    g[j + 1] = -ss * gj + cc * gj1;
+    __syncwarp();                            // every lane has read the pivot column and g
+    for (int j = q + 1 + lane; j < k; j += 32) {
+      double* col = Hc + (size_t)j * L;
+      const double t = cc * col[q] + ss * col[q + 1];
+      col[q + 1] = -ss * col[q] + cc * col[q + 1];
+      col[q] = t;
+    }
+    if (lane == 0) {
+      Hc[(size_t)q * L + q] = cc * a + ss * c;
+      g[q] = cc * gj + ss * gj1;
+      g[q + 1] = -ss * gj + cc * gj1;
+    }
   }
-  for (int i = k - 1; i >= 0; --i) {
-    double s = g[i];
-    for (int j = i + 1; j < k; ++j) s -= Hc[(size_t)j * L + i] * y[j];
-    const double rii = Hc[(size_t)i * L + i];
-    y[i] = rii != 0.0 ? s / rii : 0.0;
+  __syncwarp();
+  if (lane == 0) {
+    for (int i = k - 1; i >= 0; --i) {
+      double s = g[i];
+#pragma unroll 8
+      for (int j = i + 1; j < k; ++j) s -= Hc[(size_t)j * L + i] * ys[j];
+      const double rii = Hc[(size_t)i * L + i];
+      ys[i] = rii != 0.0 ? s / rii : 0.0;
+    }
   }
+  __syncwarp();
+  for (int q = lane; q < k; q += 32) yall[(size_t)cs * kMaxRestart + q] = ys[q];
 }
 
-// dU = x0 + V y
-// one basis entry in FP64
-__device__ __forceinline__ double basis_f64(double v) { return v; }
-__device__ __forceinline__ double basis_f64(float v) { return v; }
-__device__ __forceinline__ double basis_f64(__nv_bfloat16 v) { return __bfloat162float(v); }
+// consecutive basis entries of one vector load, in FP64
+__device__ __forceinline__ void basis_f64(const double* v, double o[2]) {
+  const double2 t = *reinterpret_cast<const double2*>(v);
+  o[0] = t.x;
+  o[1] = t.y;
+}
+__device__ __forceinline__ void basis_f64(const __nv_bfloat16* v, double o[4]) {
+  const uint2 t = *reinterpret_cast<const uint2*>(v);
+  const float2 lo = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&t.x));
+  const float2 hi = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&t.y));
+  o[0] = lo.x;
+  o[1] = lo.y;
+  o[2] = hi.x;
+  o[3] = hi.y;
+}
 
+// dU = x0 + V y.  Reads the basis once, so memory bounds it: a thread takes the entries of one
+// 8-byte (BF16) or 16-byte load and keeps eight vectors' loads in flight, and a chunk is several
+// CTAs so that small cases spread.  50 vectors of one 128x48 case 43 -> 11 us, 30 of 64 256x64 cases
+// 79 -> 59 (252 MB) against a thread walking 16 entries one after another.
+template <typename TB>
+constexpr int combine_width() { return sizeof(TB) == 2 ? 4 : 2; }
 template <typename TB>
 __global__ void __launch_bounds__(kVB) k_combine(Batch b, CombineArgs<TB> a) {
   grid_wait();
   const Chunk ch = b.chunks[blockIdx.x];
   if (!case_live(b, ch.cs, a.need)) return;
-  const CaseDev cs = b.cases[ch.cs];
-  const size_t base = 4 * cs.cell_off + ch.begin;
+  const CaseDev& cs = b.cases[ch.cs];
+  constexpr int W = combine_width<TB>();
+  const int e = (blockIdx.y * kVB + threadIdx.x) * W;   // chunks are a multiple of 4 entries
+  const size_t base = 4 * cs.cell_off + ch.begin + e;
   const int k = a.ctl[ch.cs].k_used;
   const double* y = a.y + (size_t)ch.cs * kMaxRestart;
   __shared__ double ys[kMaxRestart];
   // raw basis vectors carry their normalisation in scale[q][case]
   for (int q = threadIdx.x; q < k; q += blockDim.x) ys[q] = y[q] * a.scale[(size_t)q * b.ncases + ch.cs];
   __syncthreads();
+  if (e >= ch.len) return;
+  double acc[W];
 #pragma unroll
-  for (int s = 0; s < kPer; ++s) {
-    const int e = threadIdx.x + s * kVB;
-    if (e < ch.len) {
-      double acc = 0.0;
-      for (int q = 0; q < k; ++q) acc += basis_f64(a.V[(size_t)q * a.vstride + base + e]) * ys[q];
-      a.out[base + e] = a.x0[base + e] + acc;
-    }
+  for (int w = 0; w < W; ++w) acc[w] = 0.0;
+#pragma unroll 8
+  for (int q = 0; q < k; ++q) {
+    double v[W];
+    basis_f64(a.V + (size_t)q * a.vstride + base, v);
+#pragma unroll
+    for (int w = 0; w < W; ++w) acc[w] += v[w] * ys[q];
+  }
+#pragma unroll
+  for (int w = 0; w < W; w += 2) {
+    const double2 x = *reinterpret_cast<const double2*>(a.x0 + base + w);
+    *reinterpret_cast<double2*>(a.out + base + w) = make_double2(x.x + acc[w], x.y + acc[w + 1]);
   }
 }
 
-// per-case norms of b and x0 -> ptol (jax gmres: ptol = ||M b|| * min(1, tol ||b|| / ||b||))
 __global__ void k_gm_setup(Batch b, const double* part, int pstride, CaseCtl* ctl, double gtol) {
   grid_wait();
   const int cs = blockIdx.x * blockDim.x + threadIdx.x;
@@ -243,11 +274,11 @@ __global__ void __launch_bounds__(256) k_update_check(Batch b, const double* U, 
   if (!case_live(b, t.cs, need)) return;
   const CaseDev cs = b.cases[t.cs];
   const GridDev& g = cs.g;
+  __shared__ double scratch[32];
   double rel = 0.0;
-  for (int q = 0; q < cs.ntiles; ++q) {
-    const double v = tpart[(size_t)(cs.tile0 + q) * kTilePartStride + 1];
-    rel = q == 0 ? v : nmax(rel, v);
-  }
+  for (int q = threadIdx.x; q < cs.ntiles; q += blockDim.x)
+    rel = nmax(rel, tpart[(size_t)(cs.tile0 + q) * kTilePartStride + 1]);
+  block_max(rel, scratch);
   double omega = max_update / (rel + 1e-30);
   omega = (omega != omega) ? omega : (omega < 1.0 ? omega : 1.0);
   const size_t base = 4 * cs.cell_off;
@@ -262,7 +293,6 @@ __global__ void __launch_bounds__(256) k_update_check(Batch b, const double* U, 
     }
   }
   double v[1] = {bad};
-  __shared__ double scratch[32];
   block_sum_k<double, 1>(v, scratch);
   if (threadIdx.x == 0) {
     tpart[(size_t)blockIdx.x * kTilePartStride + 2] = v[0];
@@ -340,7 +370,7 @@ __global__ void k_mark_stepped(int ncases, const uint32_t* live, CaseCtl* ctl) {
 // launchers
 template <typename TB>
 void launch_combine(const Batch& b, const CombineArgs<TB>& a, cudaStream_t s) {
-  if (b.nchunks) launch(k_combine<TB>, b.nchunks, kVB, 0, s, b, a);
+  if (b.nchunks) launch(k_combine<TB>, dim3(b.nchunks, kChunk / (kVB * combine_width<TB>())), kVB, 0, s, b, a);
 }
 void launch_lstsq(const Batch& b, const uint32_t* live, CaseCtl* ctl, double* H, double* y, cudaStream_t s) {
   launch(k_lstsq, b.ncases, 32, 0, s, b.ncases, live, ctl, H, y);
@@ -376,7 +406,6 @@ void launch_mark_stepped(const Batch& b, const uint32_t* live, CaseCtl* ctl, cud
 }
 
 template void launch_combine<double>(const Batch&, const CombineArgs<double>&, cudaStream_t);
-template void launch_combine<float>(const Batch&, const CombineArgs<float>&, cudaStream_t);
 template void launch_combine<__nv_bfloat16>(const Batch&, const CombineArgs<__nv_bfloat16>&, cudaStream_t);
 
 }  // namespace a2d

@@ -93,6 +93,7 @@ SIGNATURES = {
     "a2d_init_freestream": (_I, [_P, _P]),
     "a2d_reset": (_I, [_P, _P]),
     "a2d_residual": (_I, [_P, _P, _P]),
+    "a2d_residual_of": (_I, [_P, _I, _P, _P, _P, _P, _P]),
     "a2d_jvp": (_I, [_P, _P]),
     "a2d_forces": (_I, [_P, _P, _P, _P]),
     "a2d_precond_setup": (_I, [_P, _P]),

@@ -353,9 +353,8 @@ __global__ void k_count(int ncases, const CaseCtl* ctl, const uint32_t* live, in
 // case with one side strided was 64 times 2.4 us, and the host behind with the launches).
 enum { kLayoutIn, kLayoutOut, kLayoutPrim };
 template <int MODE>
-__global__ void __launch_bounds__(256) k_layout(Batch b, int tile0, long long off0, const double* __restrict__ src,
-                                                double* __restrict__ dst) {
-  grid_wait();
+__device__ __forceinline__ void layout_tile(const Batch& b, int tile0, long long off0, const double* __restrict__ src,
+                                            double* __restrict__ dst) {
   __shared__ double sm[4][kTI][kTJ + 1];
   const Tile t = b.tiles[tile0 + blockIdx.x];
   const CaseDev& cs = b.cases[t.cs];
@@ -391,6 +390,22 @@ __global__ void __launch_bounds__(256) k_layout(Batch b, int tile0, long long of
       for (int k = 0; k < 4; ++k) dst[qr + k * N] = sm[k][ir][jr];
     }
   }
+}
+
+template <int MODE>
+__global__ void __launch_bounds__(256) k_layout(Batch b, int tile0, long long off0, const double* __restrict__ src,
+                                                double* __restrict__ dst) {
+  grid_wait();
+  layout_tile<MODE>(b, tile0, off0, src, dst);
+}
+
+// a residual and the primitives of its state out together, one launch for both
+__global__ void __launch_bounds__(256) k_layout_residual(Batch b, int tile0, long long off0,
+                                                         const double* __restrict__ R, double* __restrict__ Rout,
+                                                         const double* __restrict__ U, double* __restrict__ Wout) {
+  grid_wait();
+  if (blockIdx.y == 0) layout_tile<kLayoutOut>(b, tile0, off0, R, Rout);
+  else layout_tile<kLayoutPrim>(b, tile0, off0, U, Wout);
 }
 
 __global__ void k_point_flux(int n, const double* WL, const double* WR, const double* S, double* F) {
@@ -1114,6 +1129,18 @@ int a2d_residual(a2d_plan* P, const double* circ, void* stream) {
   a.sign = 1.0;
   a.circ_out = P->at<double>(P->o_circ);
   tile_stencil<double, false>(P, nullptr, a, static_cast<cudaStream_t>(stream));
+  A2D_CK(cudaGetLastError());
+  return A2D_OK;
+}
+
+int a2d_residual_of(a2d_plan* P, int k, const double* U, const double* circ, double* R, double* W, void* stream) {
+  A2D_BOUND(P);
+  if (U == nullptr || R == nullptr || W == nullptr) return fail(A2D_ERR_ARG, "residual_of: null pointer");
+  if (int e = a2d_vec_set(P, A2D_VEC_U, k, U, stream)) return e;
+  if (int e = a2d_residual(P, circ, stream)) return e;
+  const CaseDev& c = P->cases[k];
+  launch(k_layout_residual, dim3(c.ntiles, 2), 256, 0, static_cast<cudaStream_t>(stream), P->batch, c.tile0, c.cell_off,
+         P->vec(kR), R, P->vec(kU), W);
   A2D_CK(cudaGetLastError());
   return A2D_OK;
 }

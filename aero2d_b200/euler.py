@@ -203,12 +203,10 @@ class EulerSolver:
         """(R, W) for one case (aero2d/euler.py:259-287).  circ=None takes the
         circulation from U itself (Gamma = Cl M / 2, as ImplicitEuler does)."""
         pl = self._plan(winf)
-        pl.set_vec(_lib.VEC_U, 0, U)
         c = None
         if circ is not None:
             c = torch.full((1,), float(circ), dtype=torch.float64, device=self.device)
-        pl.residual(c)
-        return pl.get_vec(_lib.VEC_R, 0), pl.get_prim(_lib.VEC_U, 0)
+        return pl.residual_of(0, U, c)
 
     def local_dt(self, W):
         """Local time steps (ni, nc) of one case from its primitives W (4, ni, nc):

@@ -210,6 +210,18 @@ class Plan:
     def residual(self, circ: torch.Tensor | None = None):
         self.call("a2d_residual", None if circ is None else _ptr(circ))
 
+    def residual_of(self, k: int, U: torch.Tensor, circ: torch.Tensor | None = None):
+        """(R, W) of case k at the state U: set_vec, residual, get_vec and get_prim in one call."""
+        g = self.grids[k]
+        U = torch.as_tensor(U, dtype=torch.float64, device=self.device).contiguous()
+        if tuple(U.shape) != (4, g.ni, g.nc):
+            raise ValueError(f"state of case {k} must have shape (4, {g.ni}, {g.nc}), got {tuple(U.shape)}")
+        R = torch.empty((4, g.ni, g.nc), dtype=torch.float64, device=self.device)
+        W = torch.empty((4, g.ni, g.nc), dtype=torch.float64, device=self.device)
+        self.call("a2d_residual_of", k, _ptr(U), None if circ is None else _ptr(circ), _ptr(R), _ptr(W))
+        self._keep = U
+        return R, W
+
     def jvp(self):
         self.call("a2d_jvp")
 

@@ -137,6 +137,10 @@ int a2d_reset(a2d_plan* plan, void* stream);
 /* R := residual(U, winf, circ) (euler.py:259-287); circ: device [ncases] or NULL for
  * Gamma(U) = Cl(U) M / 2 as ImplicitEuler._res does (implicit.py:160-167) */
 int a2d_residual(a2d_plan* plan, const double* circ, void* stream);
+/* the same at the state U of one case, with a2d_vec_set before and a2d_vec_get and a2d_vec_get_prim
+ * after: U, R and W = cons_to_prim(U) are device arrays in the reference layout [4][ni][nc] */
+int a2d_residual_of(a2d_plan* plan, int case_index, const double* U, const double* circ, double* R, double* W,
+                    void* stream);
 /* JV := d residual(U, winf, Gamma(U)) / dU . V  (implicit.py:179-181, jax.jvp) */
 int a2d_jvp(a2d_plan* plan, void* stream);
 /* forces (euler.py:318-331): coef [ncases][3] = Cl, Cd, Cm; cp: wall Cp of all cases

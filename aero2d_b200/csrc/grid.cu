@@ -33,29 +33,58 @@ __device__ __forceinline__ double smooth1(double am, double a, double ap, double
   return __dadd_rn(a, __dmul_rn(eps, t));
 }
 
-// `passes` smoothing passes of the 2-vector field (vx, vy) of node i; buf is
-// [2][2][ni] ping-pong storage in shared memory; returns the smoothed value
-__device__ void smooth_ring(double& vx, double& vy, double eps, int passes, int i, int im, int ip, int ni,
-                            double* buf, bool on) {
-  int b = 0;
-  if (on) {
-    buf[i] = vx;
-    buf[ni + i] = vy;
-  }
-  __syncthreads();
-  for (int p = 0; p < passes; ++p) {
-    const double* src = buf + b * 2 * ni;
-    double* dst = buf + (b ^ 1) * 2 * ni;
-    if (on) {
-      vx = smooth1(src[im], src[i], src[ip], eps);
-      vy = smooth1(src[ni + im], src[ni + i], src[ni + ip], eps);
-      dst[i] = vx;
-      dst[ni + i] = vy;
+// A warp smooths a window of the ring in registers, two points a lane: kHalo passes need no more
+// than shuffles when the window reaches kHalo points past those it owns on either side.
+constexpr int kHalo = 10;
+constexpr int kWindow = 64;
+constexpr int kOwned = kWindow - 2 * kHalo;
+constexpr int kMaxWarps = (kMaxRing + kOwned - 1) / kOwned;
+
+struct Ring {
+  double* buf;        // [2][2][ni]: what the warps exchange, two copies in turn
+  int ni, copy;
+  int at[2];          // the lane's ring points
+  bool own[2];
+
+  // the owned points of every warp into the ring's next copy, this warp's window out of it; one
+  // barrier: a copy is written again only after the next exchange's
+  __device__ __forceinline__ void exchange(double (&vx)[2], double (&vy)[2]) {
+    double* c = buf + copy * 2 * ni;
+    copy ^= 1;
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      if (own[q]) {
+        c[at[q]] = vx[q];
+        c[ni + at[q]] = vy[q];
+      }
     }
-    b ^= 1;
     __syncthreads();
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      vx[q] = c[at[q]];
+      vy[q] = c[ni + at[q]];
+    }
   }
-}
+
+  // `passes` smoothing passes of a 2-vector field whose window is valid; then its owned points are
+  __device__ __forceinline__ void smooth(double (&vx)[2], double (&vy)[2], double eps, int passes) {
+    while (true) {
+      const int n = passes < kHalo ? passes : kHalo;
+      for (int p = 0; p < n; ++p) {
+        const double lx = __shfl_up_sync(0xffffffffu, vx[1], 1), ly = __shfl_up_sync(0xffffffffu, vy[1], 1);
+        const double rx = __shfl_down_sync(0xffffffffu, vx[0], 1), ry = __shfl_down_sync(0xffffffffu, vy[0], 1);
+        const double x0 = smooth1(lx, vx[0], vx[1], eps), y0 = smooth1(ly, vy[0], vy[1], eps);
+        vx[1] = smooth1(vx[0], vx[1], rx, eps);
+        vy[1] = smooth1(vy[0], vy[1], ry, eps);
+        vx[0] = x0;
+        vy[0] = y0;
+      }
+      passes -= n;
+      if (passes == 0) return;
+      exchange(vx, vy);
+    }
+  }
+};
 
 // NumPy's pairwise summation of a contiguous float64 array (blocks of 8
 // partial sums up to 128 entries, halves at multiples of 8 above): the order of
@@ -109,110 +138,127 @@ __device__ double pairwise_sum(const double* a, int n) {
   }
 }
 
-// one grid per CTA; ring [n][ni][2], spacing [n][nj-1], x/y [n][ni][nj], min_area [n]
-__global__ void __launch_bounds__(kMaxRing) k_ogrid(int ni, int nj, const double* __restrict__ ring,
-                                                    const double* __restrict__ spacing, int normal_smoothing,
-                                                    double* __restrict__ x, double* __restrict__ y,
-                                                    double* __restrict__ min_area) {
+// one grid per CTA; ring [n][ni][2], spacing [n][nj-1], x/y [n][ni][nj], min_area [n].
+// A chain of some 26 smoothing passes a layer, each four dependent FP64 operations and a shuffle,
+// is what bounds it: 16 grids of 256x65 points take 214 us.  A point per thread with a barrier per
+// pass took 246, the cell areas read back at the end included; in windows (Ring) a layer
+// has three barriers, and the areas are taken from the layers in shared memory.
+__global__ void __launch_bounds__(32 * kMaxWarps) k_ogrid(int ni, int nj, const double* __restrict__ ring,
+                                                          const double* __restrict__ spacing, int normal_smoothing,
+                                                          double* __restrict__ x, double* __restrict__ y,
+                                                          double* __restrict__ min_area) {
   extern __shared__ double sm[];
-  double* cur = sm;             // [2][ni] current layer
-  double* buf = sm + 2 * ni;    // [2][2][ni] smoothing ping-pong
+  double* layer[2] = {sm, sm + 2 * ni};   // [2][ni]: the last layer and the one being formed
+  Ring r;
+  r.buf = sm + 4 * ni;
+  r.ni = ni;
+  r.copy = 0;
   const int g = blockIdx.x;
-  const int i = threadIdx.x;
-  const bool on = i < ni;
-  const int im = on ? (i == 0 ? ni - 1 : i - 1) : 0;
-  const int ip = on ? (i == ni - 1 ? 0 : i + 1) : 0;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int im[2], ip[2];
+#pragma unroll
+  for (int q = 0; q < 2; ++q) {
+    const int w = 2 * lane + q - kHalo;   // from the warp's first owned point
+    const int i = ((warp * kOwned + w) % ni + ni) % ni;
+    r.at[q] = i;
+    r.own[q] = w >= 0 && w < kOwned && warp * kOwned + w < ni;
+    im[q] = i == 0 ? ni - 1 : i - 1;
+    ip[q] = i == ni - 1 ? 0 : i + 1;
+  }
   const double* rg = ring + 2 * (size_t)ni * g;
   const double* sp = spacing + (size_t)(nj - 1) * g;
   double* xg = x + (size_t)ni * nj * g;
   double* yg = y + (size_t)ni * nj * g;
+  // the points of layer j that this warp owns
+  auto put = [&](int j, const double (&cx)[2], const double (&cy)[2]) {
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      if (!r.own[q]) continue;
+      const int i = r.at[q];
+      layer[1][i] = cx[q];
+      layer[1][ni + i] = cy[q];
+      xg[(size_t)i * nj + j] = cx[q];
+      yg[(size_t)i * nj + j] = cy[q];
+    }
+  };
 
-  double cx = 0.0, cy = 0.0;
-  if (on) {
-    cx = rg[2 * i];
-    cy = rg[2 * i + 1];
-    cur[i] = cx;
-    cur[ni + i] = cy;
-    xg[(size_t)i * nj] = cx;
-    yg[(size_t)i * nj] = cy;
+  double cx[2], cy[2];
+#pragma unroll
+  for (int q = 0; q < 2; ++q) {
+    cx[q] = rg[2 * r.at[q]];
+    cy[q] = rg[2 * r.at[q] + 1];
   }
+  put(0, cx, cy);
   __syncthreads();
+  double amin = INFINITY;
   for (int j = 1; j < nj; ++j) {
+    double* t = layer[0];
+    layer[0] = layer[1];
+    layer[1] = t;
+    const double* cur = layer[0];
     // unit tangent from the neighbours, normal = (t_y, -t_x) (aero2d/grid.py:58-60)
-    double nx = 0.0, ny = 0.0;
-    if (on) {
-      const double tx = __dsub_rn(cur[ip], cur[im]);
-      const double ty = __dsub_rn(cur[ni + ip], cur[ni + im]);
+    double nx[2], ny[2];
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      const double tx = __dsub_rn(cur[ip[q]], cur[im[q]]);
+      const double ty = __dsub_rn(cur[ni + ip[q]], cur[ni + im[q]]);
       const double len = __dsqrt_rn(__dadd_rn(__dmul_rn(tx, tx), __dmul_rn(ty, ty)));
-      nx = __ddiv_rn(ty, len);
-      ny = -__ddiv_rn(tx, len);
+      nx[q] = __ddiv_rn(ty, len);
+      ny[q] = -__ddiv_rn(tx, len);
     }
-    smooth_ring(nx, ny, 0.25, j > 1 ? normal_smoothing : 2, i, im, ip, ni, buf, on);
-    if (on) {
-      const double len = __dsqrt_rn(__dadd_rn(__dmul_rn(nx, nx), __dmul_rn(ny, ny)));
-      nx = __ddiv_rn(nx, len);
-      ny = __ddiv_rn(ny, len);
-    }
+    r.smooth(nx, ny, 0.25, j > 1 ? normal_smoothing : 2);
     // step out by this layer's spacing, then smooth along the layer (:62-64)
     const double frac = __ddiv_rn((double)j, (double)(nj - 1));
     const double s = sp[j - 1];
-    double px = 0.0, py = 0.0;
-    if (on) {
-      px = __dadd_rn(cx, __dmul_rn(s, nx));
-      py = __dadd_rn(cy, __dmul_rn(s, ny));
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      const double len = __dsqrt_rn(__dadd_rn(__dmul_rn(nx[q], nx[q]), __dmul_rn(ny[q], ny[q])));
+      cx[q] = __dadd_rn(cur[r.at[q]], __dmul_rn(s, __ddiv_rn(nx[q], len)));
+      cy[q] = __dadd_rn(cur[ni + r.at[q]], __dmul_rn(s, __ddiv_rn(ny[q], len)));
     }
     const double eps = __dadd_rn(0.1, __dmul_rn(0.3, frac));
     const int passes = 2 + (int)__dmul_rn(8.0, frac);
-    smooth_ring(px, py, eps, passes, i, im, ip, ni, buf, on);
-    cx = px;
-    cy = py;
-    if (on) {
-      cur[i] = cx;
-      cur[ni + i] = cy;
-      if (j < nj - 1) {
-        xg[(size_t)i * nj + j] = cx;
-        yg[(size_t)i * nj + j] = cy;
+    r.exchange(cx, cy);
+    r.smooth(cx, cy, eps, passes);
+    if (j == nj - 1) {
+      // outer layer on a circle of the mean radius about (0.5, 0) (:65-69)
+      double* rad = r.buf + r.copy * 2 * ni;
+      double rx[2], ry[2];
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        rx[q] = __dsub_rn(cx[q], 0.5);
+        ry[q] = __dsub_rn(cy[q], 0.0);
+        if (r.own[q]) rad[r.at[q]] = __dsqrt_rn(__dadd_rn(__dmul_rn(rx[q], rx[q]), __dmul_rn(ry[q], ry[q])));
+      }
+      __syncthreads();
+      __shared__ double rmean;
+      if (threadIdx.x == 0) rmean = __ddiv_rn(pairwise_sum(rad, ni), (double)ni);
+      __syncthreads();
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        const double ang = atan2(ry[q], rx[q]);
+        cx[q] = __dadd_rn(0.5, __dmul_rn(rmean, cos(ang)));
+        cy[q] = __dadd_rn(0.0, __dmul_rn(rmean, sin(ang)));
       }
     }
+    put(j, cx, cy);
     __syncthreads();
-  }
-  // outer layer on a circle of the mean radius about (0.5, 0) (:65-69)
-  double rx = 0.0, ry = 0.0;
-  if (on) {
-    rx = __dsub_rn(cx, 0.5);
-    ry = __dsub_rn(cy, 0.0);
-    buf[i] = __dsqrt_rn(__dadd_rn(__dmul_rn(rx, rx), __dmul_rn(ry, ry)));
-  }
-  __syncthreads();
-  __shared__ double rmean;
-  if (i == 0) rmean = __ddiv_rn(pairwise_sum(buf, ni), (double)ni);
-  __syncthreads();
-  if (on) {
-    const double ang = atan2(ry, rx);
-    cx = __dadd_rn(0.5, __dmul_rn(rmean, cos(ang)));
-    cy = __dadd_rn(0.0, __dmul_rn(rmean, sin(ang)));
-    xg[(size_t)i * nj + nj - 1] = cx;
-    yg[(size_t)i * nj + nj - 1] = cy;
-  }
-  __syncthreads();
-  // smallest cell area from the two diagonals (aero2d/grid.py:24-31, :78-80)
-  double amin = INFINITY;
-  if (on) {
-    const double* x0 = xg + (size_t)i * nj;
-    const double* y0 = yg + (size_t)i * nj;
-    const double* x1 = xg + (size_t)ip * nj;
-    const double* y1 = yg + (size_t)ip * nj;
-    for (int j = 0; j < nj - 1; ++j) {
-      const double d1x = x1[j + 1] - x0[j], d1y = y1[j + 1] - y0[j];
-      const double d2x = x0[j + 1] - x1[j], d2y = y0[j + 1] - y1[j];
+    // smallest cell area from the two diagonals (aero2d/grid.py:24-31, :78-80)
+    const double* now = layer[1];
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      if (!r.own[q]) continue;
+      const int i = r.at[q], n = ip[q];
+      const double d1x = now[n] - cur[i], d1y = now[ni + n] - cur[ni + i];
+      const double d2x = now[i] - cur[n], d2y = now[ni + i] - cur[ni + n];
       amin = fmin(amin, -0.5 * (d1x * d2y - d1y * d2x));
     }
   }
   for (int o = 16; o > 0; o >>= 1) amin = fmin(amin, __shfl_xor_sync(0xffffffffu, amin, o));
-  __shared__ double wmin[kMaxRing / 32];
-  if ((i & 31) == 0) wmin[i >> 5] = amin;
+  __shared__ double wmin[kMaxWarps];
+  if (lane == 0) wmin[warp] = amin;
   __syncthreads();
-  if (i == 0) {
+  if (threadIdx.x == 0) {
     double m = INFINITY;
     for (int w = 0; w < (int)(blockDim.x >> 5); ++w) m = fmin(m, wmin[w]);
     min_area[g] = m;
@@ -250,9 +296,9 @@ int a2d_grid_build(int n, int ni, int nj, const double* ring, const double* spac
   if (n == 0) return A2D_OK;
   if (ring == nullptr || spacing == nullptr || x == nullptr || y == nullptr || min_area == nullptr)
     return fail(A2D_ERR_ARG, "grid_build: null pointer");
-  const int threads = (ni + 31) / 32 * 32;
-  const size_t smem = sizeof(double) * 6 * (size_t)ni;
-  cudaFuncSetAttribute(k_ogrid, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(sizeof(double) * 6 * kMaxRing));
+  const int threads = 32 * ((ni + kOwned - 1) / kOwned);
+  const size_t smem = sizeof(double) * 8 * (size_t)ni;
+  cudaFuncSetAttribute(k_ogrid, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(sizeof(double) * 8 * kMaxRing));
   k_ogrid<<<n, threads, smem, static_cast<cudaStream_t>(stream)>>>(ni, nj, ring, spacing, normal_smoothing, x,
                                                                    y, min_area);
   const cudaError_t e = cudaGetLastError();

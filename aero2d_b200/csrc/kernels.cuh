@@ -100,8 +100,8 @@ struct SweepArgs {
   uint32_t need = 0;
 };
 
-void launch_metrics(int ni, int nc, const double* x, const double* y, double* md, float* mf,
-                    cudaStream_t s);
+void launch_metrics(int n, int ni, int nc, const double* x, const double* y, void* metrics, size_t stride,
+                    size_t float_off, cudaStream_t s);
 
 // shape: the tile shape of b's tile list (kTile*; only the FP32 linearised
 // stencil has shapes other than kTile32x8)

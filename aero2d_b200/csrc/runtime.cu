@@ -815,12 +815,16 @@ int a2d_metrics_bytes(int ni, int nj, size_t* bytes) {
 }
 
 int a2d_metrics_build(int ni, int nj, const double* x, const double* y, void* metrics, void* stream) {
-  if (x == nullptr || y == nullptr || metrics == nullptr || ni < 4 || nj < 3)
+  return a2d_metrics_build_batch(1, ni, nj, x, y, metrics, 0, stream);
+}
+
+int a2d_metrics_build_batch(int n, int ni, int nj, const double* x, const double* y, void* metrics, size_t stride,
+                            void* stream) {
+  if (x == nullptr || y == nullptr || metrics == nullptr || ni < 4 || nj < 3 || n < 1 || n > 65535 || stride % 8 != 0 ||
+      (n > 1 && stride < metrics_total_bytes(ni, nj - 1)))
     return fail(A2D_ERR_ARG, "metrics: bad arguments");
-  const int nc = nj - 1;
-  double* md = static_cast<double*>(metrics);
-  float* mf = reinterpret_cast<float*>(static_cast<char*>(metrics) + metrics_float_offset(ni, nc));
-  launch_metrics(ni, nc, x, y, md, mf, static_cast<cudaStream_t>(stream));
+  launch_metrics(n, ni, nj - 1, x, y, metrics, stride, metrics_float_offset(ni, nj - 1),
+                 static_cast<cudaStream_t>(stream));
   A2D_CK(cudaGetLastError());
   return A2D_OK;
 }

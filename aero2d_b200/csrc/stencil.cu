@@ -26,8 +26,14 @@ namespace a2d {
 // ---------------------------------------------------------------------------
 // metrics from node coordinates (reference layout x[i][j], nj = nc + 1)
 // ---------------------------------------------------------------------------
+// a grid per blockIdx.y: nodes one grid after another, metrics `stride` bytes apart
 __global__ void k_metrics(int ni, int nc, const double* __restrict__ x, const double* __restrict__ y,
-                          double* __restrict__ md, float* __restrict__ mf) {
+                          char* __restrict__ metrics, size_t stride, size_t float_off) {
+  metrics += stride * blockIdx.y;
+  double* __restrict__ md = reinterpret_cast<double*>(metrics);
+  float* __restrict__ mf = reinterpret_cast<float*>(metrics + float_off);
+  x += (size_t)ni * (nc + 1) * blockIdx.y;
+  y += (size_t)ni * (nc + 1) * blockIdx.y;
   const int nj = nc + 1;
   const size_t N = (size_t)ni * nc;
   double* vol = md;
@@ -132,11 +138,11 @@ __global__ void __launch_bounds__(256) k_forces(Batch b, const double* __restric
 // ---------------------------------------------------------------------------
 // host launchers
 // ---------------------------------------------------------------------------
-void launch_metrics(int ni, int nc, const double* x, const double* y, double* md, float* mf,
-                    cudaStream_t s) {
+void launch_metrics(int n, int ni, int nc, const double* x, const double* y, void* metrics, size_t stride,
+                    size_t float_off, cudaStream_t s) {
   const size_t total = (size_t)ni * (nc + 1);
   const int blocks = (int)((total + 255) / 256);
-  k_metrics<<<blocks, 256, 0, s>>>(ni, nc, x, y, md, mf);
+  k_metrics<<<dim3(blocks, n), 256, 0, s>>>(ni, nc, x, y, static_cast<char*>(metrics), stride, float_off);
 }
 
 template void launch_stencil<double, false, double>(const Batch&, const StencilArgs<double>&, cudaStream_t, int);

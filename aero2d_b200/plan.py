@@ -38,10 +38,11 @@ class DeviceGrid:
     """An O-grid resident on the device: node coordinates and the metrics blob
     (cell areas, face vectors, wall and far-field face midpoints, FP64 and FP32)."""
 
-    def __init__(self, grid: OGrid | None = None, device=None, *, nodes: tuple | None = None):
+    def __init__(self, grid: OGrid | None = None, device=None, *, nodes: tuple | None = None,
+                 metrics: torch.Tensor | None = None):
         """From a host OGrid, or from node coordinates already on the device
         (`nodes=(x, y)`, contiguous FP64 tensors (ni, nj), as the device grid
-        generator writes them)."""
+        generator writes them; `metrics` is their blob where it has built that too)."""
         lib = _lib.load()
         if nodes is not None:
             self.x, self.y = nodes
@@ -56,6 +57,9 @@ class DeviceGrid:
             self.x = torch.as_tensor(np.ascontiguousarray(grid.x, np.float64), device=self.device)
             self.y = torch.as_tensor(np.ascontiguousarray(grid.y, np.float64), device=self.device)
         self.ni, self.nj, self.nc = ni, nj, nj - 1
+        if metrics is not None:
+            self.metrics = metrics
+            return
         n = C.c_size_t()
         _lib.check(lib.a2d_metrics_bytes(ni, nj, C.byref(n)))
         self.metrics = torch.empty(n.value, dtype=torch.uint8, device=self.device)

@@ -89,6 +89,10 @@ int a2d_grid_build(int n, int ni, int nj, const double* ring, const double* spac
 int a2d_metrics_bytes(int ni, int nj, size_t* bytes);
 /* x, y: device FP64 node coordinates [ni][nj]; metrics: device blob of a2d_metrics_bytes */
 int a2d_metrics_build(int ni, int nj, const double* x, const double* y, void* metrics, void* stream);
+/* the metrics of n grids of one size, their nodes one after another, `stride` bytes (a multiple of
+ * 8, at least a2d_metrics_bytes) apart: one launch */
+int a2d_metrics_build_batch(int n, int ni, int nj, const double* x, const double* y, void* metrics, size_t stride,
+                            void* stream);
 
 /* ---- plans: a batch of cases (the vmap axis of euler.py:393 / implicit.py:204-210) ---- */
 /* ni[k], nc[k]: cells of case k; metrics[k]: its metrics blob; winf: [ncases][4] host FP64 */

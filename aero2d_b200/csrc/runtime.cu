@@ -743,6 +743,15 @@ static int newton_step(a2d_plan* P, cudaStream_t s) {
     return A2D_OK;
   }
   if (P->graph == nullptr) {
+    // a plan's first step goes out kernel by kernel, and the graph of the later ones is captured
+    // and instantiated while it runs
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    A2D_CK(cudaStreamIsCapturing(s, &status));
+    const bool first = status == cudaStreamCaptureStatusNone;
+    if (first) {
+      newton_dispatch(P, s);
+      A2D_CK(cudaGetLastError());
+    }
     cudaStream_t cap;
     A2D_CK(cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking));
     cudaGraph_t g;
@@ -766,6 +775,7 @@ static int newton_step(a2d_plan* P, cudaStream_t s) {
     e = cudaGraphInstantiate(&P->graph, g, 0);
     cudaGraphDestroy(g);
     if (e != cudaSuccess) return fail(A2D_ERR_CUDA, std::string("graph instantiate: ") + cudaGetErrorString(e));
+    if (first) return A2D_OK;
   }
   A2D_CK(cudaGraphLaunch(P->graph, s));
   return A2D_OK;

@@ -78,8 +78,11 @@ __device__ __forceinline__ void store_block(TS* base, long long row0, int rows, 
   for (int e = 0; e < 16; ++e) base[lbidx(row0, rows, g, j, e, lane)] = TS(A[e]);
 }
 
+// Bound by the dual flux's instructions and their latency.  FP32 left alone takes 174 registers, one
+// CTA per SM; held to 128 (28 bytes of spills) it runs two: 64 cases of 256x64 350 -> 238 us.  Three
+// are slower (263), and FP64 fills its 255.
 template <typename T>
-__global__ void __launch_bounds__(256) k_face_jac(Batch b, JacArgs a) {
+__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 2 : 1) k_face_jac(Batch b, JacArgs a) {
   grid_wait();
   const Tile t = b.tiles[blockIdx.x];
   if (!case_live(b, t.cs, a.need)) return;

@@ -1,0 +1,54 @@
+// Thread-block clusters: ranks, the barrier, another CTA's shared memory and bounded waits for
+// what others store here.
+#pragma once
+#include <cstdint>
+
+#include "tma.cuh"
+
+namespace a2d {
+
+__device__ __forceinline__ uint32_t cluster_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ uint32_t cluster_size() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
+  return r;
+}
+// every thread of the cluster that has not exited (whole warps)
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ uint32_t peer_addr(const void* p, uint32_t rank) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_u32(p)), "r"(rank));
+  return r;
+}
+// bounded wait that acquires other CTAs' stores
+__device__ __forceinline__ bool wait_cluster(uint64_t* bar, uint32_t parity) {
+  auto try_once = [&]() {
+    uint32_t ok;
+    asm volatile(
+        "{\n"
+        " .reg .pred p;\n"
+        " mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2, %3;\n"
+        " selp.u32 %0, 1, 0, p;\n"
+        "}\n"
+        : "=r"(ok)
+        : "r"(smem_u32(bar)), "r"(parity), "r"(kSuspendNs)
+        : "memory");
+    return ok != 0;
+  };
+#pragma unroll 1
+  for (int q = 0; q < kWaitTries; ++q)
+    if (try_once()) return true;
+  const unsigned long long t0 = global_ns();
+  while (!try_once()) {
+    if (global_ns() - t0 > kWaitLimitNs) return false;
+  }
+  return true;
+}
+
+}  // namespace a2d

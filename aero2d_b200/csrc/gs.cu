@@ -25,6 +25,8 @@
 // and differences are not, spelled out, so that no unrolling changes a bit: h2 is made of w's
 // rounding, and a marginal case's path follows it.
 //
+// Small mixed-precision cases run a whole step, passes and close, in one launch: k_gs_case.
+//
 // What bounds the passes: the basis from HBM (each pass reads it once from there), with few
 // chunks the latency of one CTA.  A warp owns a row (in split launches a quarter of one)
 // and runs it through alone: the row's entries of w stay in registers from the subtraction to
@@ -42,6 +44,7 @@
 #include <type_traits>
 
 #include "batch.cuh"
+#include "cluster.cuh"
 #include "gs.cuh"
 #include "launch.cuh"
 
@@ -241,9 +244,6 @@ struct Ring {
 // ---- a chunk's sums from its rows', added in order ----
 // split: the rows are CTAs of one cluster (rank = row), whose sums the first one reads from
 // their shared memory
-__device__ __forceinline__ void cluster_sync() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
 __device__ __forceinline__ double peer_value(const double* p, int rank) {
   uint32_t addr;
   double v;
@@ -575,6 +575,238 @@ __global__ void __launch_bounds__(32 * warps_of(SPLIT), SPLIT ? 4 : (sizeof(TB) 
   store_chunk<SPLIT>(a.part_norm + blockIdx.x, rowsum, 1);
 }
 
+// the end of Arnoldi step a.k, by one warp: the Hessenberg column and the new vector's scale
+__device__ __forceinline__ void close_step(const GsCloseArgs& a, int ncases, int cs_id, double hn, double wn0,
+                                           const double* h1, const double* h2) {
+  const int lane = threadIdx.x & 31, k = a.k;
+  CaseCtl& c = a.ctl[cs_id];
+  const bool use = hn > DBL_EPSILON * wn0;
+  double* H = a.H + (size_t)cs_id * kMaxRestart * (kMaxRestart + 1) + (size_t)k * (kMaxRestart + 1);
+  for (int q = lane; q <= k; q += 32) H[q] = h1[q] + h2[q];
+  if (lane == 0) {
+    H[k + 1] = use ? hn : 0.0;
+    a.scale[(size_t)(k + 1) * ncases + cs_id] = use ? 1.0 / hn : 0.0;
+    c.k_used = k + 1;
+    if (!use) a.live[cs_id] &= ~kLiveKrylov;
+  }
+}
+
+// a whole Arnoldi step of a small case --------------------------------------------
+// With few rows the four launches are latency: each starts up, fetches the basis or the sums of the
+// last, reduces.  Here a case is a cluster.  A row of a chunk belongs to a team of four warps,
+// which copies its entries of every vector (1 KB each) into shared memory once and runs all three
+// passes from there; a row's sums go to every CTA of the cluster as they are formed (st.async,
+// counted on an mbarrier there), and each CTA adds them up itself, in the order of the passes
+// above, so the results are theirs to the bit.  What is left is latency, and the conversions of the
+// entries to FP64.  One 128x48 case, 25 vectors on average: the four launches 29.5 us, this 17;
+// 16 cases of 128x32, 13 vectors: 24 and 14.  FP64 rows are too large for the shared memory.
+using CaseBasis = __nv_bfloat16;
+constexpr int kTeams = 5;                // rows of a CTA at most
+struct CaseSmem {
+  int tile, wp, msg, norm, rowsum, coef, scale, h1, h2, wn0, bar, bytes;   // offsets
+  __host__ __device__ CaseSmem(int teams, int rows, int nq) {
+    int o = 0;
+    auto take = [&](int n) {
+      const int at = o;
+      o += n;
+      return at;
+    };
+    tile = take(teams * nq * 1024);                     // [team][vector][quad m][lane]
+    wp = take(teams * kChain * 32 * 8);                 // [team][chain index][lane]
+    msg = take(2 * rows * (nq + 1) * 8);                // [pass][row][vector]
+    norm = take(rows * 8);
+    rowsum = take(teams * (kMaxRestart + 1) * 8);
+    coef = take(kMaxRestart * 8);
+    scale = take(kMaxRestart * 8);
+    h1 = take(kMaxRestart * 8);
+    h2 = take(kMaxRestart * 8);
+    wn0 = take(8);
+    bar = take(3 * 8);
+    bytes = o;
+  }
+};
+constexpr int kCaseMaxSmem = 227 * 1024;
+
+__device__ __forceinline__ void team_sync(int team) {
+  asm volatile("bar.sync %0, 128;" ::"r"(1 + team) : "memory");
+}
+__device__ __forceinline__ void peer_store1(uint32_t addr, double v, uint32_t bar) {
+  asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.f64 [%0], %1, [%2];" ::"r"(addr), "d"(v),
+               "r"(bar)
+               : "memory");
+}
+
+template <int TEAMS>
+__global__ void __launch_bounds__(128 * TEAMS, TEAMS == 2 ? 3 : 1) k_gs_case(Batch b, GsArgs<CaseBasis> a, GsCloseArgs c, uint32_t* err,
+                                                          int rows_max) {
+  grid_wait();
+  using TB = CaseBasis;
+  extern __shared__ __align__(16) unsigned char gs_sm[];
+  const uint32_t size = cluster_size(), rank = cluster_rank();
+  const int cs_id = blockIdx.x / size;
+  if (!case_live(b, cs_id, a.need)) return;   // the whole cluster leaves
+  const CaseDev cs = b.cases[cs_id];
+  const int nq = a.nq, stride = nq + 1, rows = cs.nchunks * kRows;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int team = warp >> 2, m = warp & 3, nwarps = blockDim.x >> 5;
+  const CaseSmem sm(blockDim.x >> 7, rows_max, nq);
+  uint2* tile = reinterpret_cast<uint2*>(gs_sm + sm.tile) + (size_t)team * nq * 128;
+  double* wp = reinterpret_cast<double*>(gs_sm + sm.wp) + team * kChain * 32;
+  double* msg = reinterpret_cast<double*>(gs_sm + sm.msg);
+  double* norm = reinterpret_cast<double*>(gs_sm + sm.norm);
+  double* rs = reinterpret_cast<double*>(gs_sm + sm.rowsum) + team * (kMaxRestart + 1);
+  double* coef = reinterpret_cast<double*>(gs_sm + sm.coef);
+  double* scale = reinterpret_cast<double*>(gs_sm + sm.scale);
+  double* h1 = reinterpret_cast<double*>(gs_sm + sm.h1);
+  double* h2 = reinterpret_cast<double*>(gs_sm + sm.h2);
+  double* wn0 = reinterpret_cast<double*>(gs_sm + sm.wn0);
+  uint64_t* bar = reinterpret_cast<uint64_t*>(gs_sm + sm.bar);
+  if (threadIdx.x == 0) {
+    for (int q = 0; q < 3; ++q) mbar_init(bar + q, 1);
+    mbar_init_fence();
+    mbar_arrive_expect(bar, rows * stride * 8);
+    mbar_arrive_expect(bar + 1, rows * nq * 8);
+    mbar_arrive_expect(bar + 2, rank == 0 ? rows * 8 : 0);
+  }
+  __syncwarp();
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+
+  const int row = team * (int)size + (int)rank;
+  const bool have = row < rows;               // the same for a team
+  const Chunk ch = b.chunks[cs.chunk0 + (have ? row / kRows : 0)];
+  const int r = row % kRows, len = ch.len;
+  const size_t base = 4 * cs.cell_off + ch.begin;
+  double w0[4] = {0.0, 0.0, 0.0, 0.0};
+  if (have) {
+    const int e = Quad<TB>::at(r, m, lane);
+    const uint32_t bytes = e < len ? 8u : 0u;
+    const TB* src = a.V + base + (e < len ? e : 0);
+    uint32_t dst = smem_u32(tile + m * 32 + lane);
+#pragma unroll 4
+    for (int q = 0; q < nq; ++q) {
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+      dst += 128 * sizeof(uint2);
+      src += a.vstride;
+    }
+    load_w<TB>(a.w + base, r, m, lane, len, w0);
+#pragma unroll
+    for (int t = 0; t < 4; ++t) wp[(4 * m + t) * 32 + lane] = w0[t];
+  }
+  for (int q = threadIdx.x; q < nq; q += blockDim.x) scale[q] = a.scale[(size_t)q * b.ncases + cs_id];
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  __syncthreads();
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");   // every CTA's mbarriers exist
+
+  auto whole = [&](Quad<TB>& v, int q, int k) { v.raw = tile[(size_t)q * 128 + k * 32 + lane]; };
+  auto mine = [&](Quad<TB>& v, int q) { v.raw = tile[(size_t)q * 128 + m * 32 + lane]; };
+  // the row's first n sums to every CTA
+  auto publish = [&](int pass, int n) {
+    for (int v = threadIdx.x & 127; v < n * (int)size; v += 128) {
+      const int q = v / (int)size;
+      const uint32_t peer = v - q * (int)size;
+      peer_store1(peer_addr(msg + ((size_t)pass * rows_max + row) * stride + q, peer), rs[q], peer_addr(bar + pass, peer));
+    }
+  };
+  // project the row in wp on the basis and publish; pass 0 also its w . w
+  auto project = [&](int pass) {
+    double wv[kChain];
+#pragma unroll
+    for (int i = 0; i < kChain; ++i) wv[i] = wp[i * 32 + lane];
+    if (pass == 0 && m == 0) {
+      double n[1] = {0.0};
+#pragma unroll
+      for (int i = 0; i < kChain; ++i) n[0] = fma(wv[i], wv[i], n[0]);
+      const double s = warp_tree<1>(n);
+      if (lane == 0) rs[nq] = s;
+    }
+    project_row<TB>(nq, m, 4, whole, wv, rs);
+    team_sync(team);
+    publish(pass, pass == 0 ? nq + 1 : nq);
+  };
+  // a pass's sums over the case's chunks, and the coefficients of the next subtraction
+  auto fold = [&](int pass) {
+    bool ok = wait_cluster(bar + pass, 0);
+    const int n = pass == 0 ? nq + 1 : nq;
+    if (ok) {
+#pragma unroll 2
+      for (int q = warp; q < n; q += nwarps) {
+        double s = 0.0;
+        if (lane < cs.nchunks) {
+          const double* v = msg + ((size_t)pass * rows_max + lane * kRows) * stride + q;
+#pragma unroll
+          for (int k = 0; k < kRows; ++k) s += v[k * stride];
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        if (lane == 0) {
+          if (q < nq) {
+            const double sc = scale[q];
+            const double h = __dmul_rn(s, sc);
+            (pass == 0 ? h1 : h2)[q] = h;
+            const double hh = pass == 0 ? h : __dadd_rn(h1[q], h);
+            coef[q] = hh * sc;
+          } else {
+            *wn0 = sqrt(s);
+          }
+        }
+      }
+    }
+    return __syncthreads_and(ok) != 0;
+  };
+
+  if (have) project(0);
+  bool ok = fold(0);
+  if (ok) {
+    if (have) {
+      double x[4] = {w0[0], w0[1], w0[2], w0[3]};
+      subtract<TB>(nq, mine, coef, x);
+#pragma unroll
+      for (int t = 0; t < 4; ++t) wp[(4 * m + t) * 32 + lane] = x[t];
+      team_sync(team);
+      project(1);
+    }
+    ok = fold(1);
+  }
+  if (ok) {
+    if (have) {
+      double x[4] = {w0[0], w0[1], w0[2], w0[3]};
+      subtract<TB>(nq, mine, coef, x);
+      store_quad(a.Vout + base, r, m, lane, len, x);
+#pragma unroll
+      for (int t = 0; t < 4; ++t) wp[(4 * m + t) * 32 + lane] = x[t];
+      team_sync(team);
+      if (m == 0) {
+        double n[1] = {0.0};
+#pragma unroll
+        for (int i = 0; i < kChain; ++i) {
+          const double y = wp[i * 32 + lane];
+          n[0] = fma(y, y, n[0]);
+        }
+        const double s = warp_tree<1>(n);
+        if (lane == 0) peer_store1(peer_addr(norm + row, 0), s, peer_addr(bar + 2, 0));
+      }
+    }
+    if (rank == 0 && warp == 0) {
+      ok = wait_cluster(bar + 2, 0);
+      if (ok) {
+        double s = 0.0;
+        if (lane < cs.nchunks) {
+#pragma unroll
+          for (int k = 0; k < kRows; ++k) s += norm[lane * kRows + k];
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        close_step(c, b.ncases, cs_id, sqrt(s), *wn0, h1, h2);
+      }
+    }
+  }
+  if (!ok) {
+    if (lane == 0 && err != nullptr) atomicExch(err, 1u);
+    __syncwarp();
+    cluster_sync();   // the other threads of the cluster finish, or give up and come here too, first
+  }
+}
+
 // start vector: V_raw[0] = r and its squared norm ------------------------------
 constexpr int kGB = 256;                 // threads per block
 constexpr int kGE = kChunk / kGB;        // entries per thread
@@ -649,18 +881,7 @@ __global__ void __launch_bounds__(32) k_gs_close(Batch b, GsCloseArgs a) {
     else a.live[cs_id] &= ~kLiveKrylov;
     return;
   }
-  const int k = a.k;
-  const bool use = hn > DBL_EPSILON * a.wn0[cs_id];
-  double* H = a.H + (size_t)cs_id * kMaxRestart * (kMaxRestart + 1) + (size_t)k * (kMaxRestart + 1);
-  const double* h1 = a.h1 + (size_t)cs_id * kHStride;
-  const double* h2 = a.h2 + (size_t)cs_id * kHStride;
-  for (int q = lane; q <= k; q += 32) H[q] = h1[q] + h2[q];
-  if (lane == 0) {
-    H[k + 1] = use ? hn : 0.0;
-    a.scale[(size_t)(k + 1) * b.ncases + cs_id] = use ? 1.0 / hn : 0.0;
-    c.k_used = k + 1;
-    if (!use) a.live[cs_id] &= ~kLiveKrylov;
-  }
+  close_step(a, b.ncases, cs_id, hn, a.wn0[cs_id], a.h1 + (size_t)cs_id * kHStride, a.h2 + (size_t)cs_id * kHStride);
 }
 
 // ---------------------------------------------------------------------------
@@ -717,6 +938,48 @@ void launch_gs_close(const Batch& b, const GsCloseArgs& a, cudaStream_t s) {
   if (b.ncases) launch(k_gs_close, b.ncases, 32, 0, s, b, a);
 }
 
+// the launch of k_gs_case for all cases of up to `rows` rows
+struct CaseLaunch {
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute at[2];
+  void (*kernel)(Batch, GsArgs<CaseBasis>, GsCloseArgs, uint32_t*, int);
+  CaseLaunch(int ncases, int cluster, int rows, int nq, cudaStream_t s) {
+    const int teams = (rows + cluster - 1) / cluster;
+    // two teams at most: room for three CTAs on an SM, which a batch of 16 cases of 32 rows needs
+    kernel = teams <= 2 ? k_gs_case<2> : k_gs_case<kTeams>;
+    cfg.gridDim = dim3((unsigned)(ncases * cluster));
+    cfg.blockDim = dim3((unsigned)(128 * teams));
+    cfg.dynamicSmemBytes = CaseSmem(teams, rows, nq).bytes;
+    cfg.stream = s;
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = (unsigned)cluster;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    at[1] = dependent_launch();
+    cfg.attrs = at;
+    cfg.numAttrs = 2;
+  }
+};
+int gs_case_vectors(int ncases, int cluster, int max_chunks, int nq) {
+  const int rows = max_chunks * kRows;
+  if (rows > kTeams * cluster || max_chunks > 32) return 0;
+  auto fits = [&](int q) {
+    CaseLaunch l(ncases, cluster, rows, q, nullptr);
+    if (l.cfg.dynamicSmemBytes > kCaseMaxSmem) return false;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, l.kernel, &l.cfg) == cudaSuccess) return n >= ncases;
+    (void)cudaGetLastError();
+    return false;
+  };
+  if (!fits(1)) return 0;
+  while (!fits(nq)) --nq;
+  return nq;
+}
+void launch_gs_case(const Batch& b, const GsArgs<CaseBasis>& a, const GsCloseArgs& c, uint32_t* err, int cluster,
+                    int max_chunks, cudaStream_t s) {
+  CaseLaunch l(b.ncases, cluster, max_chunks * kRows, a.nq, s);
+  (void)cudaLaunchKernelEx(&l.cfg, l.kernel, b, a, c, err, max_chunks * kRows);   // as <<<>>>: see cudaGetLastError
+}
+
 #define A2D_GS_INST(TB)                                                                 \
   template void launch_gs_dots<TB>(const Batch&, const GsArgs<TB>&, cudaStream_t);     \
   template void launch_gs_project<TB>(const Batch&, const GsArgs<TB>&, cudaStream_t);  \
@@ -731,6 +994,10 @@ cudaError_t gs_init() {
   auto set = [&](const void* f, size_t bytes) {
     if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
   };
+  for (auto f : {k_gs_case<2>, k_gs_case<kTeams>}) {
+    set(reinterpret_cast<const void*>(f), kCaseMaxSmem);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  }
   set(reinterpret_cast<const void*>(&k_gs_project<__nv_bfloat16, true>), gs_tile_bytes<__nv_bfloat16>(kMaxRestart));
 #define A2D_GS_ATTR(TB)                                                                       \
   set(reinterpret_cast<const void*>(&k_gs_dots<TB, false>), kRows * Ring<TB>::kBytes);       \

@@ -1,6 +1,7 @@
 // Argument blocks and launchers of the Gram-Schmidt kernels (gs.cu).
 #pragma once
 #include <cstdint>
+#include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
 #include "batch.cuh"
@@ -49,6 +50,12 @@ template <typename TB> void launch_gs_project(const Batch& b, const GsArgs<TB>& 
 template <typename TB> void launch_gs_finish(const Batch& b, const GsArgs<TB>& a, cudaStream_t s);
 template <typename TB> void launch_gs_start(const Batch& b, const GsArgs<TB>& a, cudaStream_t s);
 void launch_gs_close(const Batch& b, const GsCloseArgs& a, cudaStream_t s);
+// A whole Arnoldi step (passes 1 to 3 and the close) in one launch, a cluster per case: the most
+// vectors, up to nq, that a case of max_chunks chunks takes with clusters of `cluster` CTAs while
+// every case's runs at once (0: none), and the launch
+int gs_case_vectors(int ncases, int cluster, int max_chunks, int nq);
+void launch_gs_case(const Batch& b, const GsArgs<__nv_bfloat16>& a, const GsCloseArgs& c, uint32_t* err, int cluster,
+                    int max_chunks, cudaStream_t s);
 // raises the dynamic shared-memory limit of the passes (host, once per device)
 cudaError_t gs_init();
 

@@ -34,6 +34,7 @@
 #include <type_traits>
 
 #include "batch.cuh"
+#include "cluster.cuh"
 #include "kernels.cuh"
 #include "launch.cuh"
 #include "tma.cuh"
@@ -190,26 +191,6 @@ __device__ __forceinline__ T add_dot4(T s, const T (&a)[4], const T (&b)[4]) {
   return s;
 }
 
-// ---- the cluster ----
-__device__ __forceinline__ uint32_t cluster_rank() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-__device__ __forceinline__ uint32_t cluster_size() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
-  return r;
-}
-// every thread of the cluster that has not exited (whole warps)
-__device__ __forceinline__ void cluster_sync() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-__device__ __forceinline__ uint32_t peer_addr(const void* p, uint32_t rank) {
-  uint32_t r;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_u32(p)), "r"(rank));
-  return r;
-}
 // one 4-vector into another CTA's shared memory, its bytes counted on an mbarrier there: the
 // waiter needs no fence or arrival of ours (a cluster fence takes longer than a pack's rows)
 __device__ __forceinline__ void peer_store(uint32_t addr, const float (&v)[4], uint32_t bar) {
@@ -226,31 +207,6 @@ __device__ __forceinline__ void peer_store(uint32_t addr, const double (&v)[4], 
                "d"(v[2]), "d"(v[3]), "r"(bar)
                : "memory");
 }
-// bounded wait that acquires other CTAs' stores
-__device__ __forceinline__ bool wait_cluster(uint64_t* bar, uint32_t parity) {
-  auto try_once = [&]() {
-    uint32_t ok;
-    asm volatile(
-        "{\n"
-        " .reg .pred p;\n"
-        " mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2, %3;\n"
-        " selp.u32 %0, 1, 0, p;\n"
-        "}\n"
-        : "=r"(ok)
-        : "r"(smem_u32(bar)), "r"(parity), "r"(kSuspendNs)
-        : "memory");
-    return ok != 0;
-  };
-#pragma unroll 1
-  for (int q = 0; q < kWaitTries; ++q)
-    if (try_once()) return true;
-  const unsigned long long t0 = global_ns();
-  while (!try_once()) {
-    if (global_ns() - t0 > kWaitLimitNs) return false;
-  }
-  return true;
-}
-
 extern __shared__ __align__(128) unsigned char lines_sm[];
 
 // the CTA's view of its lines; everything shared is addressed from lines_sm, so that the

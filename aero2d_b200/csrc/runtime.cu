@@ -99,6 +99,7 @@ struct a2d_plan {
   };
   std::vector<LineClass> line_classes;
   std::vector<int> line_cases;
+  int gs_cluster = 0, gs_vectors = 0, max_chunks = 0;   // Arnoldi steps in one launch: cluster size, up to this step
   bool lines_fit = false;      // every class runs on the device bound to (set at bind)
   size_t irs_entries = 0, irs_smem = 0, o_irs = 0;   // smoothing tables (explicit.cu), a shape's once
   bool irs_ready = false;      // filled since bind
@@ -174,6 +175,7 @@ static void build_tables(a2d_plan* P, const int* ni, const int* nc, const void* 
     for (long long b0 = 0; b0 < n4; b0 += kChunk)
       P->chunks.push_back(Chunk{k, (int)b0, (int)std::min<long long>(kChunk, n4 - b0)});
     c.nchunks = (int)P->chunks.size() - c.chunk0;
+    P->max_chunks = std::max(P->max_chunks, c.nchunks);
     c.group0 = (int)P->groups.size();
     for (int g = 0; g < ngr; ++g)
       P->groups.push_back(Group{k, g, g * kLanes, std::min(kLanes, ni[k] - g * kLanes)});
@@ -674,6 +676,24 @@ static void newton_step_launches(a2d_plan* P, cudaStream_t s) {
     g.pstride = P->pstride;
     g.scale = scale;
     g.need = KR;
+    GsCloseArgs ck;
+    ck.part_norm = cpartn;
+    ck.wn0 = wn0;
+    ck.h1 = h1;
+    ck.h2 = h2;
+    ck.H = P->at<double>(P->o_H);
+    ck.scale = scale;
+    ck.ctl = ctl;
+    ck.live = live;
+    ck.k = k;
+    ck.need = KR;
+    if constexpr (std::is_same<TB, Basis16>::value) {
+      if (k < P->gs_vectors) {
+        g.Vout = V + (size_t)(k + 1) * vs;
+        launch_gs_case(B, g, ck, P->at<uint32_t>(P->o_cnt) + 1, P->gs_cluster, P->max_chunks, s);
+        continue;
+      }
+    }
     GsArgs<TB> gd = g;
     gd.part = cpart;
     launch_gs_dots<TB>(B, gd, s);
@@ -690,17 +710,6 @@ static void newton_step_launches(a2d_plan* P, cudaStream_t s) {
     gf.Vout = V + (size_t)(k + 1) * vs;
     gf.part_norm = cpartn;
     launch_gs_finish<TB>(B, gf, s);
-    GsCloseArgs ck;
-    ck.part_norm = cpartn;
-    ck.wn0 = wn0;
-    ck.h1 = h1;
-    ck.h2 = h2;
-    ck.H = P->at<double>(P->o_H);
-    ck.scale = scale;
-    ck.ctl = ctl;
-    ck.live = live;
-    ck.k = k;
-    ck.need = KR;
     launch_gs_close(B, ck, s);
   }
   nvtxRangePop();
@@ -969,6 +978,19 @@ int a2d_plan_bind(a2d_plan* P, void* workspace, size_t bytes, void* stream) {
     P->lines_fit = P->lines_fit && (mixed ? n > 0 : n >= c.count);
   }
   A2D_CK(gs_init());
+  // Arnoldi steps in one launch while every case's cluster runs at once (a second wave would cost
+  // more than the launches saved); of the cluster sizes the one whose shared memory takes
+  // the most vectors, and of these the largest
+  P->gs_cluster = P->gs_vectors = 0;
+  if (P->p.precision == A2D_MIXED) {
+    for (int c = 16; c >= 4; --c) {
+      const int n = gs_case_vectors(P->ncases, c, P->max_chunks, P->m);
+      if (n > P->gs_vectors) {
+        P->gs_cluster = c;
+        P->gs_vectors = n;
+      }
+    }
+  }
   A2D_CK(irs_init());
   A2D_CK(factor_init());
   P->irs_ready = false;

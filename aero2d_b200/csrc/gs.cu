@@ -962,6 +962,7 @@ struct CaseLaunch {
 int gs_case_vectors(int ncases, int cluster, int max_chunks, int nq) {
   const int rows = max_chunks * kRows;
   if (rows > kTeams * cluster || max_chunks > 32) return 0;
+  if (ncases * cluster > 148 * (rows <= 2 * cluster ? 3 : 1)) return 0;   // more CTAs than run at once
   auto fits = [&](int q) {
     CaseLaunch l(ncases, cluster, rows, q, nullptr);
     if (l.cfg.dynamicSmemBytes > kCaseMaxSmem) return false;

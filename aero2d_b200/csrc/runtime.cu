@@ -983,7 +983,7 @@ int a2d_plan_bind(a2d_plan* P, void* workspace, size_t bytes, void* stream) {
   // the most vectors, and of these the largest
   P->gs_cluster = P->gs_vectors = 0;
   if (P->p.precision == A2D_MIXED) {
-    for (int c = 16; c >= 4; --c) {
+    for (int c = 16; c >= 4 && P->gs_vectors < P->m; --c) {
       const int n = gs_case_vectors(P->ncases, c, P->max_chunks, P->m);
       if (n > P->gs_vectors) {
         P->gs_cluster = c;

@@ -7,7 +7,8 @@ are bitwise the same; include/aero2d_b200.h, a2d_plan_set_tuning):
   jvp_tile  the tile shape (i x j cells per CTA) of the FP32 Jacobian-vector
             stencil, run gmres_restart + 1 times per Newton step: "32x8",
             "32x16", "64x4" or "16x16" (the halo is recomputed per tile, so
-            taller tiles compute less and hold more shared memory);
+            taller tiles compute less and hold more shared memory; batches whose
+            16x4 tiles run at once take these at "32x16");
   sweep     the line sweep's kernel: a launch per sweep, by warps per half line
             group "lanes" (one warp, a lane solving all four block rows of its
             line), "pairs" (two warps, two lanes per line with two block rows

@@ -103,8 +103,8 @@ struct SweepArgs {
 void launch_metrics(int n, int ni, int nc, const double* x, const double* y, void* metrics, size_t stride,
                     size_t float_off, cudaStream_t s);
 
-// shape: the tile shape of b's tile list (kTile*; only the FP32 linearised
-// stencil has shapes other than kTile32x8)
+// shape: the tile shape of b's tile list (kTile*; kTile32x8 and kTile16x4 for every stencil, the others
+// for the FP32 linearised one)
 template <typename T, bool LIN, typename VT>
 void launch_stencil(const Batch& b, const StencilArgs<VT>& a, cudaStream_t s, int shape = kTile32x8);
 // resident-CTA queries of the persistent stencil launches (host, before any capture)

@@ -2,7 +2,7 @@
 // forward linearisation (the Jacobian-vector product of the Newton-Krylov
 // solver), plus the grid metrics, the wall forces and the circulation.
 //
-// One CTA owns a 32 (i) x 8 (j) tile of cells of one case.  It stages the
+// One CTA owns a tile of cells of one case, 32 (i) x 8 (j) or, in small batches, 16 x 4.  It stages the
 // primitive state of the tile and a 2-cell halo in shared memory (wall and
 // far-field ghosts are formed while staging), computes every i- and j-face
 // flux of the tile once (MUSCL + smooth van Albada + positivity clamp + HLLC),

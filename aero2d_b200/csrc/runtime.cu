@@ -102,7 +102,6 @@ struct a2d_plan {
   int gs_cluster = 0, gs_vectors = 0, max_chunks = 0;   // Arnoldi steps in one launch: cluster size, up to this step
   bool lines_fit = false;      // every class runs on the device bound to (set at bind)
   size_t irs_entries = 0, irs_smem = 0, o_irs = 0;   // smoothing tables (explicit.cu), a shape's once
-  bool irs_ready = false;      // filled since bind
   size_t o_lcases = 0, o_E0 = 0;   // o_E0: inv r of the lines, kept between the sweeps of an application
   long long C = 0, rows_nc = 0, rows_nc1 = 0, total_ni = 0;
   size_t tj = 8, tb = 8;   // bytes of face-Jacobian and basis storage entries
@@ -519,16 +518,15 @@ static void precond_setup(a2d_plan* P, const Batch& B, uint32_t need, cudaStream
   launch_factor<TJ, typename FactorStore<TJ>::type>(B, factor_args(P, need), s);
 }
 
+// whether the plan smooths, and its shapes fit the fused kernel, whose tables bind fills
+static bool irs_fits(const a2d_plan* P) { return P->p.irs_eps > 0 && P->irs_smem <= kIrsMaxSmem; }
+
 // one smoothing of R by the plan's coefficient: the stage update U = U0 - a (dt / vol) R~, or
 // (U0 null) out = R~; false where the fused kernel does not run
 static bool irs_fused(a2d_plan* P, const Batch& B, const double* R, const double* U0, double* out, double a,
                       cudaStream_t s) {
-  if (P->p.irs_eps <= 0 || P->irs_smem > kIrsMaxSmem) return false;
+  if (!irs_fits(P)) return false;
   const bool fp32 = P->p.precision == A2D_MIXED;
-  if (!P->irs_ready) {
-    launch_irs_table(B, P->at<double>(P->o_irs), P->p.irs_eps, fp32, s);
-    P->irs_ready = true;
-  }
   IrsArgs p;
   p.R = R;
   p.U0 = U0;
@@ -993,8 +991,10 @@ int a2d_plan_bind(a2d_plan* P, void* workspace, size_t bytes, void* stream) {
     }
   }
   A2D_CK(irs_init());
+  // here and not at the first smoothing, which may be made under capture, where nothing runs
+  if (irs_fits(P))
+    launch_irs_table(B, P->at<double>(P->o_irs), P->p.irs_eps, P->p.precision == A2D_MIXED, s);
   A2D_CK(factor_init());
-  P->irs_ready = false;
   stencil_init_fp64();
   stencil_init_fp32();
   k_reset<<<(P->ncases + 63) / 64, 64, 0, s>>>(P->ncases, P->ctl(), P->live(), P->p.cfl0);

@@ -77,7 +77,7 @@ __global__ void __launch_bounds__(256) k_local_dt_prim(GridDev g, const double* 
 // compute type (values stay in FP64 arrays, rounded to T when T is FP32)
 template <typename T>
 __global__ void __launch_bounds__(256) k_irs_i(Batch b, const double* __restrict__ R, double* __restrict__ out,
-                                               double e_) {
+                                               double e_, int reach) {
   grid_wait();
   const int row = blockIdx.x;   // rows enumerated as (case, k, j) via the row table below
   const int cs_id = blockIdx.y;
@@ -96,8 +96,7 @@ __global__ void __launch_bounds__(256) k_irs_i(Batch b, const double* __restrict
   const double e = e_;
   const double lam = ((1.0 + 2.0 * e) - sqrt(1.0 + 4.0 * e)) / (2.0 * e);
   const double G0 = 1.0 / (e * (1.0 / lam - lam));
-  int M = (int)ceil(log(1e-18) / log(lam));
-  if (M > ni / 2) M = ni / 2;
+  const int M = min(reach, ni / 2);
   const double ln = pow(lam, (double)ni);
   for (int m = threadIdx.x; m <= M; m += blockDim.x)
     gm[m] = T(G0 * (pow(lam, (double)m) + pow(lam, (double)(ni - m))) / (1.0 - ln));
@@ -192,25 +191,26 @@ constexpr int kIrsCols = 32;
 // entries of a shape's table: M, g_0 .. g_{ni/2}, then per row the pivot, its reciprocal and c'
 __host__ __device__ inline int irs_gm_entries(int ni) { return ni / 2 + 2; }
 
-// reach of the Green's function: terms below 1e-18 of the diagonal are dropped
-int irs_reach(double e, int ni) {
+// reach of the Green's function on a long ring: terms below 1e-18 of the diagonal are dropped.  Formed
+// on the host alone: it sizes the shared memory, and a device logarithm that rounds the other way
+// at an integer would lay out more than that
+static int irs_reach(double e) {
   const double lam = ((1.0 + 2.0 * e) - std::sqrt(1.0 + 4.0 * e)) / (2.0 * e);
-  const int M = (int)std::ceil(std::log(1e-18) / std::log(lam));
-  return M > ni / 2 ? ni / 2 : M;
+  const double M = std::ceil(std::log(1e-18) / std::log(lam));
+  return M > 0.0 ? (int)std::min(M, 1e9) : 0;   // 0 too where lam has cancelled away
 }
 size_t irs_table_entries(int ni, int nc) { return (size_t)irs_gm_entries(ni) + 3 * (size_t)nc; }
 
 // tables of every case's shape (cases of one shape share a table and write the same values)
 template <typename T>
-__global__ void __launch_bounds__(64) k_irs_table(Batch b, double* __restrict__ tab, double e_) {
+__global__ void __launch_bounds__(64) k_irs_table(Batch b, double* __restrict__ tab, double e_, int reach) {
   const CaseDev cs = b.cases[blockIdx.x];
   const int ni = cs.g.ni, nc = cs.g.nc;
   double* t = tab + cs.irs_off;
   const double e = e_;
   const double lam = ((1.0 + 2.0 * e) - sqrt(1.0 + 4.0 * e)) / (2.0 * e);
   const double G0 = 1.0 / (e * (1.0 / lam - lam));
-  int M = (int)ceil(log(1e-18) / log(lam));
-  if (M > ni / 2) M = ni / 2;
+  const int M = min(reach, ni / 2);
   const double ln = pow(lam, (double)ni);
   for (int m = threadIdx.x; m <= M; m += blockDim.x)
     t[1 + m] = (double)T(G0 * (pow(lam, (double)m) + pow(lam, (double)(ni - m))) / (1.0 - ln));
@@ -625,17 +625,17 @@ void launch_irs(const Batch& b, double* R, double* tmp, double e, int max_ni, in
   const size_t sm = (size_t)(max_ni + max_ni / 2 + 2) * sizeof(double);
   dim3 gj((4 * max_ni + 127) / 128, b.ncases);
   if (fp32) {
-    launch(k_irs_i<float>, gi, 256, sm, s, b, R, tmp, e);
+    launch(k_irs_i<float>, gi, 256, sm, s, b, R, tmp, e, irs_reach(e));
     launch(k_irs_j<float>, gj, 128, (size_t)max_nc * sizeof(double), s, b, tmp, e);
   } else {
-    launch(k_irs_i<double>, gi, 256, sm, s, b, R, tmp, e);
+    launch(k_irs_i<double>, gi, 256, sm, s, b, R, tmp, e, irs_reach(e));
     launch(k_irs_j<double>, gj, 128, (size_t)max_nc * sizeof(double), s, b, tmp, e);
   }
 }
 void launch_irs_table(const Batch& b, double* tab, double e, bool fp32, cudaStream_t s) {
   if (b.ncases == 0) return;
-  if (fp32) k_irs_table<float><<<b.ncases, 64, 0, s>>>(b, tab, e);
-  else k_irs_table<double><<<b.ncases, 64, 0, s>>>(b, tab, e);
+  if (fp32) k_irs_table<float><<<b.ncases, 64, 0, s>>>(b, tab, e, irs_reach(e));
+  else k_irs_table<double><<<b.ncases, 64, 0, s>>>(b, tab, e, irs_reach(e));
 }
 template <typename T, bool STAGE>
 static void irs_launch(const Batch& b, const IrsArgs& p, size_t smem, cudaStream_t s) {
@@ -654,7 +654,7 @@ void launch_irs_fused(const Batch& b, const IrsArgs& p, bool fp32, cudaStream_t 
   }
 }
 size_t irs_smem_bytes(int ni, int nc, double e, bool fp32) {
-  const int M = irs_reach(e, ni);
+  const int M = std::min(irs_reach(e), ni / 2);
   const IrsShape sh = irs_shape(M, ni);
   return fp32 ? irs_smem<float>(sh.width, nc, M) : irs_smem<double>(sh.width, nc, M);
 }

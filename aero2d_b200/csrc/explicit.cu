@@ -15,6 +15,7 @@
 #include "explicit.cuh"
 #include "launch.cuh"
 #include "physics.cuh"
+#include "quotient.cuh"
 
 namespace a2d {
 
@@ -180,10 +181,8 @@ __global__ void __launch_bounds__(128) k_irs_j(Batch b, double* __restrict__ R, 
 // What bounded the three kernels this replaces: the Green's function's pow calls in every
 // block, two shared-memory reads per term, and along j a global load and a division in
 // every step of the recurrence.  The tables (irs_table) are now made once per plan, and
-// the division by the step's constant pivot is one multiplication by its reciprocal with
-// Markstein's correction (P. Markstein, IBM J. Res. Dev. 34, 1990: with y = RN(1/b), q = RN(a y)
-// and r = RN(a - q b), RN(q + r y) is RN(a/b)), the quotient itself.  The FP32 iteration is
-// bitwise what it was.
+// the division by the step's constant pivot is one multiplication by its reciprocal and a
+// correction (quotient.cuh), the quotient to the bit.
 // Measured (B200, per stage): FP32, 32 cases of 256 x 64, 120 -> 31 us; FP64, 3 cases of
 // 128 x 48, 31 -> 13 us.  Left: the Thomas recurrence's length, one warp of a CTA.
 constexpr int kIrsCols = 32;
@@ -239,14 +238,6 @@ __device__ __forceinline__ void ld4(const float* p, float (&v)[4]) {
 __device__ __forceinline__ void ld4(const double* p, double (&v)[4]) {
   const double2 t = reinterpret_cast<const double2*>(p)[0], u = reinterpret_cast<const double2*>(p)[1];
   v[0] = t.x; v[1] = t.y; v[2] = u.x; v[3] = u.y;
-}
-
-// a / b for a normal b with y = RN(1/b); an infinite or NaN quotient stays what a y is
-template <typename T>
-__device__ __forceinline__ T quotient(T a, T b, T y) {
-  const T q = a * y;
-  const T r = fma(-q, b, a);
-  return fabs(q) <= T(1e30) ? fma(r, y, q) : a / b;
 }
 
 struct IrsShape {

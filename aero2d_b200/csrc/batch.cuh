@@ -65,7 +65,7 @@ struct CaseDev {
   int tile0, ntiles;     // stencil tiles
   int chunk0, nchunks;   // reduction chunks over the 4*ni*nc vector entries
   int group0, ngroups;   // line groups
-  int irs_off;           // first entry of the case's smoothing table (explicit.cu)
+  int irs_off;           // first entry of the case's smoothing table (explicit.cu); -1: it has none
 };
 
 struct Tile {

@@ -83,6 +83,7 @@ __global__ void __launch_bounds__(256) k_irs_i(Batch b, const double* __restrict
   const int row = blockIdx.x;   // rows enumerated as (case, k, j) via the row table below
   const int cs_id = blockIdx.y;
   const CaseDev cs = b.cases[cs_id];
+  if (cs.irs_off >= 0) return;   // k_irs takes it
   const GridDev& g = cs.g;
   const int ni = g.ni, nc = g.nc;
   if (row >= 4 * nc) return;
@@ -132,6 +133,7 @@ __global__ void __launch_bounds__(128) k_irs_j(Batch b, double* __restrict__ R, 
   grid_wait();
   const int cs_id = blockIdx.y;
   const CaseDev cs = b.cases[cs_id];
+  if (cs.irs_off >= 0) return;
   const GridDev& g = cs.g;
   const int ni = g.ni, nc = g.nc;
   extern __shared__ __align__(8) unsigned char irs_sm[];
@@ -204,6 +206,7 @@ size_t irs_table_entries(int ni, int nc) { return (size_t)irs_gm_entries(ni) + 3
 template <typename T>
 __global__ void __launch_bounds__(64) k_irs_table(Batch b, double* __restrict__ tab, double e_, int reach) {
   const CaseDev cs = b.cases[blockIdx.x];
+  if (cs.irs_off < 0) return;
   const int ni = cs.g.ni, nc = cs.g.nc;
   double* t = tab + cs.irs_off;
   const double e = e_;
@@ -266,7 +269,7 @@ __global__ void __launch_bounds__(256) k_irs(Batch b, const double* __restrict__
   const CaseDev cs = b.cases[blockIdx.z];
   const GridDev& g = cs.g;
   const int ni = g.ni, nc = g.nc, c0 = blockIdx.x * kIrsCols, comp = blockIdx.y;
-  if (c0 >= ni) return;
+  if (c0 >= ni || cs.irs_off < 0) return;
   const double* t = tab + cs.irs_off;
   const int M = (int)t[0];
   const IrsShape sh = irs_shape(M, ni);
@@ -407,14 +410,16 @@ __global__ void __launch_bounds__(256) k_irs(Batch b, const double* __restrict__
 }
 
 // U = U0 - a (dt / vol) R   (euler.py:344), in the compute type T (with FP32
-// the state is rounded to FP32 at every stage, as the reference's float32 run keeps it)
+// the state is rounded to FP32 at every stage, as the reference's float32 run keeps it);
+// rest: of the cases that k_irs does not take
 template <typename T>
 __global__ void __launch_bounds__(256) k_rk_stage(Batch b, const double* __restrict__ U0,
                                                   const double* __restrict__ R, const double* __restrict__ dt,
-                                                  double* __restrict__ U, double a) {
+                                                  double* __restrict__ U, double a, bool rest) {
   grid_wait();
   const Tile t = b.tiles[blockIdx.x];
   const CaseDev cs = b.cases[t.cs];
+  if (rest && cs.irs_off >= 0) return;
   const GridDev& g = cs.g;
   const Metric<T> m{g};
   const size_t base = 4 * cs.cell_off;
@@ -661,10 +666,10 @@ cudaError_t irs_init() {
   return e;
 }
 void launch_rk_stage(const Batch& b, const double* U0, const double* R, const double* dt, double* U, double a,
-                     bool fp32, cudaStream_t s) {
+                     bool rest, bool fp32, cudaStream_t s) {
   if (b.ntiles == 0) return;
-  if (fp32) launch(k_rk_stage<float>, b.ntiles, 256, 0, s, b, U0, R, dt, U, a);
-  else launch(k_rk_stage<double>, b.ntiles, 256, 0, s, b, U0, R, dt, U, a);
+  if (fp32) launch(k_rk_stage<float>, b.ntiles, 256, 0, s, b, U0, R, dt, U, a, rest);
+  else launch(k_rk_stage<double>, b.ntiles, 256, 0, s, b, U0, R, dt, U, a, rest);
 }
 void launch_rk_res(const Batch& b, const double* U0, const double* U, const double* dt, double* tpart,
                    cudaStream_t s) {

@@ -33,7 +33,7 @@ cudaError_t irs_init();
 void launch_irs(const Batch& b, double* R, double* tmp, double e, int max_ni, int max_nc, bool fp32,
                 cudaStream_t s);
 void launch_rk_stage(const Batch& b, const double* U0, const double* R, const double* dt, double* U, double a,
-                     bool fp32, cudaStream_t s);
+                     bool rest, bool fp32, cudaStream_t s);
 void launch_rk_res(const Batch& b, const double* U0, const double* U, const double* dt, double* tpart,
                    cudaStream_t s);
 void launch_rk_finish(const Batch& b, const double* tpart, const double* coef, double* res, double* circ,

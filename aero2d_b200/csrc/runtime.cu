@@ -101,7 +101,10 @@ struct a2d_plan {
   std::vector<int> line_cases;
   int gs_cluster = 0, gs_vectors = 0, max_chunks = 0;   // Arnoldi steps in one launch: cluster size, up to this step
   bool lines_fit = false;      // every class runs on the device bound to (set at bind)
-  size_t irs_entries = 0, irs_smem = 0, o_irs = 0;   // smoothing tables (explicit.cu), a shape's once
+  // smoothing tables (explicit.cu), a shape's once, of the cases whose shape fits the fused kernel;
+  // irs_rest: cases that it does not fit
+  size_t irs_entries = 0, irs_smem = 0, o_irs = 0;
+  bool irs_rest = false;
   size_t o_lcases = 0, o_E0 = 0;   // o_E0: inv r of the lines, kept between the sweeps of an application
   long long C = 0, rows_nc = 0, rows_nc1 = 0, total_ni = 0;
   size_t tj = 8, tb = 8;   // bytes of face-Jacobian and basis storage entries
@@ -200,12 +203,17 @@ static void build_tables(a2d_plan* P, const int* ni, const int* nc, const void* 
   if ((int)P->ftiles.size() > kFineTiles32) P->ftiles.clear();
   std::map<std::pair<int, int>, int> irs_at;
   for (int k = 0; k < P->ncases; ++k) {
+    P->cases[k].irs_off = -1;
+    if (P->p.irs_eps <= 0) continue;
+    const size_t smem = irs_smem_bytes(ni[k], nc[k], P->p.irs_eps, P->p.precision == A2D_MIXED);
+    if (smem > kIrsMaxSmem) {
+      P->irs_rest = true;
+      continue;
+    }
     const auto it = irs_at.emplace(std::make_pair(ni[k], nc[k]), (int)P->irs_entries);
     P->cases[k].irs_off = it.first->second;
-    if (!it.second) continue;
-    P->irs_entries += irs_table_entries(ni[k], nc[k]);
-    if (P->p.irs_eps > 0)
-      P->irs_smem = std::max(P->irs_smem, irs_smem_bytes(ni[k], nc[k], P->p.irs_eps, P->p.precision == A2D_MIXED));
+    if (it.second) P->irs_entries += irs_table_entries(ni[k], nc[k]);
+    P->irs_smem = std::max(P->irs_smem, smem);
   }
   std::map<int, std::vector<int>> by_groups;
   for (int k = 0; k < P->ncases; ++k) by_groups[P->cases[k].ngroups].push_back(k);
@@ -518,31 +526,28 @@ static void precond_setup(a2d_plan* P, const Batch& B, uint32_t need, cudaStream
   launch_factor<TJ, typename FactorStore<TJ>::type>(B, factor_args(P, need), s);
 }
 
-// whether the plan smooths, and its shapes fit the fused kernel, whose tables bind fills
-static bool irs_fits(const a2d_plan* P) { return P->p.irs_eps > 0 && P->irs_smem <= kIrsMaxSmem; }
-
-// one smoothing of R by the plan's coefficient: the stage update U = U0 - a (dt / vol) R~, or
-// (U0 null) out = R~; false where the fused kernel does not run
-static bool irs_fused(a2d_plan* P, const Batch& B, const double* R, const double* U0, double* out, double a,
-                      cudaStream_t s) {
-  if (!irs_fits(P)) return false;
+// one smoothing of R by the plan's coefficient (> 0): the stage update U = U0 - a (dt / vol) R~, or
+// (U0 null) out = R~.  A case's own shape says which kernels take it, whatever it is beside;
+// tmp: the smoothed R of those that the fused one does not
+static void smoothed(a2d_plan* P, const Batch& B, double* R, const double* U0, double* out, double* tmp, double a,
+                     cudaStream_t s) {
   const bool fp32 = P->p.precision == A2D_MIXED;
-  IrsArgs p;
-  p.R = R;
-  p.U0 = U0;
-  p.dt = P->at<double>(P->o_dt);
-  p.out = out;
-  p.tab = P->at<double>(P->o_irs);
-  p.e = P->p.irs_eps;
-  p.a = a;
-  p.max_ni = P->max_ni;
-  p.smem = P->irs_smem;
-  launch_irs_fused(B, p, fp32, s);
-  return true;
-}
-static void smoothed(a2d_plan* P, const Batch& B, double* R, double* out, cudaStream_t s) {
-  if (!irs_fused(P, B, R, nullptr, out, 0.0, s))
-    launch_irs(B, R, out, P->p.irs_eps, P->max_ni, P->max_nc, P->p.precision == A2D_MIXED, s);
+  if (P->irs_entries > 0) {
+    IrsArgs p;
+    p.R = R;
+    p.U0 = U0;
+    p.dt = P->at<double>(P->o_dt);
+    p.out = out;
+    p.tab = P->at<double>(P->o_irs);
+    p.e = P->p.irs_eps;
+    p.a = a;
+    p.max_ni = P->max_ni;
+    p.smem = P->irs_smem;
+    launch_irs_fused(B, p, fp32, s);
+  }
+  if (!P->irs_rest) return;
+  launch_irs(B, R, tmp, P->p.irs_eps, P->max_ni, P->max_nc, fp32, s);
+  if (U0 != nullptr) launch_rk_stage(B, U0, tmp, P->at<double>(P->o_dt), out, a, true, fp32, s);
 }
 
 // the vector of case k, or of all cases (k < 0), one after another
@@ -992,7 +997,7 @@ int a2d_plan_bind(a2d_plan* P, void* workspace, size_t bytes, void* stream) {
   }
   A2D_CK(irs_init());
   // here and not at the first smoothing, which may be made under capture, where nothing runs
-  if (irs_fits(P))
+  if (P->irs_entries > 0)
     launch_irs_table(B, P->at<double>(P->o_irs), P->p.irs_eps, P->p.precision == A2D_MIXED, s);
   A2D_CK(factor_init());
   stencil_init_fp64();
@@ -1514,9 +1519,10 @@ int a2d_smooth(a2d_plan* P, void* stream) {
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   Batch B = P->batch;
   B.live = nullptr;
-  smoothed(P, B, P->vec(kR), P->vec(kPA), s);
-  if (P->p.irs_eps > 0)
+  if (P->p.irs_eps > 0) {
+    smoothed(P, B, P->vec(kR), nullptr, P->vec(kPA), P->vec(kPA), 0.0, s);
     A2D_CK(cudaMemcpyAsync(P->vec(kR), P->vec(kPA), 8 * 4 * (size_t)P->C, cudaMemcpyDeviceToDevice, s));
+  }
   A2D_CK(cudaGetLastError());
   return A2D_OK;
 }
@@ -1550,7 +1556,6 @@ static cudaError_t rk_iter(a2d_plan* P, const double* circ, const double* forcin
   double* U = P->vec(kU);
   double* U0 = P->vec(kU0);
   double* R = P->vec(kR);
-  double* Rs = P->vec(kPA);
   double* dt = P->at<double>(P->o_dt);
   const double alphas[4] = {0.25, 1.0 / 3.0, 0.5, 1.0};
   // dtype=float32: residual, local time steps, smoothing and stage update in FP32
@@ -1566,13 +1571,8 @@ static cudaError_t rk_iter(a2d_plan* P, const double* circ, const double* forcin
     if (fp32) tile_stencil<float, false>(P, nullptr, a, s);
     else tile_stencil<double, false>(P, nullptr, a, s);
     if (forcing != nullptr) launch_add_forcing(B, R, forcing, s);
-    if (irs_fused(P, B, R, U0, U, alphas[st], s)) continue;
-    const double* Ruse = R;
-    if (P->p.irs_eps > 0) {
-      launch_irs(B, R, Rs, P->p.irs_eps, P->max_ni, P->max_nc, fp32, s);
-      Ruse = Rs;
-    }
-    launch_rk_stage(B, U0, Ruse, dt, U, alphas[st], fp32, s);
+    if (P->p.irs_eps > 0) smoothed(P, B, R, U0, U, P->vec(kPA), alphas[st], s);
+    else launch_rk_stage(B, U0, R, dt, U, alphas[st], false, fp32, s);
   }
   return cudaGetLastError();
 }

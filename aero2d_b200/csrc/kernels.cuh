@@ -125,8 +125,8 @@ void launch_factor(const Batch& b, const FactorArgs& a, cudaStream_t s);
 // by warps per half line group: one, a lane solving all four block rows of its line
 // (lanes, sweep.cu); two, two lanes per line with two block rows each (pairs, sweep_pairs.cu);
 // four, a warp per block row (rows, sweep_rows.cu).  All sweeps of an application
-// in one launch, a cluster per case (lines.cu): halves, and on FP64 plans lanes, where
-// every case fits it (lines_clusters); the per-sweep kernels otherwise
+// in one launch, a cluster per case (lines.cu): halves, and on FP64 plans lanes, for the
+// cases that bind chooses it for (choose_lines); the per-sweep kernels for the others
 enum : int { kSweepLanes = 0, kSweepRows = 1, kSweepPairs = 2, kSweepHalves = 3, kNumSweepVariants = 4 };
 
 // one line-Jacobi sweep; FIRST: the sweep without i-coupling; last: x is the
@@ -144,7 +144,10 @@ void launch_sweep_pairs(const Batch& b, const SweepArgs& a, bool last, cudaStrea
 template <typename TI>
 void launch_lines(const Batch& b, const SweepArgs& a, const int* cases, int count, int groups, int rows, int sweeps,
                   cudaStream_t s);
-// clusters of that launch that the current device holds at once; 0: it cannot run there (host)
+// whether a case of that shape fits that launch, and the clusters of it that the current device
+// holds at once; 0: it cannot run there (host)
+template <typename TI>
+bool lines_take(int groups, int rows);
 template <typename TI>
 int lines_clusters(int groups, int rows);
 

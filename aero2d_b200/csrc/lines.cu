@@ -697,8 +697,13 @@ struct LinesLaunch {
 };
 
 template <typename TI>
+bool lines_take(int groups, int rows) {
+  return groups <= lines::kMaxCluster && lines::Smem<TI>::bytes(rows) <= (uint32_t)lines::kMaxSmem;
+}
+
+template <typename TI>
 int lines_clusters(int groups, int rows) {
-  if (groups > lines::kMaxCluster || lines::Smem<TI>::bytes(rows) > (uint32_t)lines::kMaxSmem) return 0;
+  if (!lines_take<TI>(groups, rows)) return 0;
   LinesLaunch<TI> l(1, groups, rows, nullptr);
   int n = 0;
   if (cudaOccupancyMaxActiveClusters(&n, lines::k_lines<TI>, &l.cfg) != cudaSuccess) {
@@ -727,6 +732,8 @@ cudaError_t lines_init() {
   return e;
 }
 
+template bool lines_take<float>(int, int);
+template bool lines_take<double>(int, int);
 template int lines_clusters<float>(int, int);
 template int lines_clusters<double>(int, int);
 template void launch_lines<float>(const Batch&, const SweepArgs&, const int*, int, int, int, int, cudaStream_t);

@@ -92,15 +92,19 @@ struct a2d_plan {
   std::vector<Chunk> chunks;
   std::vector<Group> groups;
   std::vector<long long> cp_off;
-  // cases by line-group count, for the one-launch preconditioner (lines.cu): a launch per
-  // class; line_cases holds the case indices class after class
+  // cases by line-group count, and those that the one-launch preconditioner (lines.cu) cannot take
+  // apart: a launch per class that `one` is set for; line_cases holds the case indices
+  // class after class, rest_groups the line groups of all other classes, which the per-sweep
+  // kernels take together (both set at bind, choose_lines)
   struct LineClass {
     int groups, rows, first, count;
+    bool fits, one;
   };
   std::vector<LineClass> line_classes;
   std::vector<int> line_cases;
   int gs_cluster = 0, gs_vectors = 0, max_chunks = 0;   // Arnoldi steps in one launch: cluster size, up to this step
-  bool lines_fit = false;      // every class runs on the device bound to (set at bind)
+  std::vector<Group> rest_groups;
+  size_t o_rgroups = 0;
   // smoothing tables (explicit.cu), a shape's once, of the cases whose shape fits the fused kernel;
   // irs_rest: cases that it does not fit
   size_t irs_entries = 0, irs_smem = 0, o_irs = 0;
@@ -215,10 +219,14 @@ static void build_tables(a2d_plan* P, const int* ni, const int* nc, const void* 
     if (it.second) P->irs_entries += irs_table_entries(ni[k], nc[k]);
     P->irs_smem = std::max(P->irs_smem, smem);
   }
-  std::map<int, std::vector<int>> by_groups;
-  for (int k = 0; k < P->ncases; ++k) by_groups[P->cases[k].ngroups].push_back(k);
+  std::map<std::pair<int, bool>, std::vector<int>> by_groups;
+  for (int k = 0; k < P->ncases; ++k) {
+    const int groups = P->cases[k].ngroups;
+    const bool fits = P->p.precision == A2D_MIXED ? lines_take<float>(groups, nc[k]) : lines_take<double>(groups, nc[k]);
+    by_groups[{groups, fits}].push_back(k);
+  }
   for (const auto& g : by_groups) {
-    a2d_plan::LineClass c{g.first, 0, (int)P->line_cases.size(), (int)g.second.size()};
+    a2d_plan::LineClass c{g.first.first, 0, (int)P->line_cases.size(), (int)g.second.size(), g.first.second, false};
     for (int k : g.second) c.rows = std::max(c.rows, nc[k]);
     P->line_cases.insert(P->line_cases.end(), g.second.begin(), g.second.end());
     P->line_classes.push_back(c);
@@ -273,6 +281,7 @@ static void layout(a2d_plan* P) {
   P->o_ftiles = cv.take(sizeof(Tile) * P->ftiles.size());
   P->o_irs = cv.take(8 * P->irs_entries);
   P->o_lcases = cv.take(sizeof(int) * (size_t)B);
+  P->o_rgroups = cv.take(sizeof(Group) * P->groups.size());
   P->bytes = cv.off + 256;
 }
 
@@ -479,9 +488,103 @@ static FactorArgs factor_args(const a2d_plan* P, uint32_t need) {
   return fa;
 }
 
-// whether an application's sweeps run as one launch per line-group count (lines.cu)
+// whether an application's sweeps run as one launch for some cases (lines.cu)
 static bool one_launch(const a2d_plan* P) {
-  return P->lines_fit && P->sweep_variant == (P->p.precision == A2D_MIXED ? kSweepHalves : kSweepLanes);
+  return P->rest_groups.size() < P->groups.size() &&
+         P->sweep_variant == (P->p.precision == A2D_MIXED ? kSweepHalves : kSweepLanes);
+}
+
+// Which classes take the one-launch preconditioner.  Its launches follow each other, a class at a time, while the
+// per-sweep kernels take every group of the batch at once, so one class alone is faster in one
+// launch while its clusters run together, but not always in several waves of them, nor several small
+// classes one after another.  The estimate, in us per row of a line for four sweeps on a B200: a wave
+// of clusters `few` to `full` as it fills the device, a wave of per-sweep CTAs `sfew` to
+// `sfull`.  The figures are fitted to 559 uniform mixed batches (2 to 16 groups, 48 to 300 rows, 8 to
+// 128 cases: within 0.5 % of the better path on average, 1.95x faster than always one launch at 96
+// cases of 384 x 143, and slower than that nowhere) and 128 FP64 ones.  Ragged, one launch a class
+// against the per-sweep kernels (48 rows, a case each, mixed / FP64): two classes 58 and 66 us / 96 and 128, three
+// 86 and 66 / 143 and 129, sixteen 530 and 69 / 763 and 138.
+static void choose_lines(a2d_plan* P) {
+  const bool mixed = P->p.precision == A2D_MIXED;
+  struct Fit {
+    double few, full, full1;   // full1: where only one CTA fits an SM
+    int two_rows;              // rows up to which two do
+    double sfew, sfull;
+    int ctas;                  // per-sweep CTAs that run at once
+  };
+  const Fit f = mixed ? Fit{0.5, 0.75, 0.9, 142, 1.3, 2.8, 4 * 148} : Fit{1.0, 1.2, 1.2, 0, 2.45, 4.7, 3 * 148};
+  const size_t n = P->line_classes.size();
+  std::vector<double> cost(n, 0.0);
+  for (size_t q = 0; q < n; ++q) {
+    a2d_plan::LineClass& c = P->line_classes[q];
+    c.one = false;
+    if (!c.fits) continue;
+    const int at_once = mixed ? lines_clusters<float>(c.groups, c.rows) : lines_clusters<double>(c.groups, c.rows);
+    // FP64: one CTA per SM, and a second wave loses to the per-sweep kernels (256 x 64: 8 cases
+    // 111 against 193 us, 16 cases in two waves 196 against 180)
+    c.fits = at_once > 0 && (mixed || c.count <= at_once);
+    if (!c.fits) continue;
+    const double full = c.rows <= f.two_rows ? f.full : f.full1;
+    const int waves = (c.count - 1) / at_once;
+    const double last = (double)(c.count - waves * at_once) / at_once;
+    cost[q] = c.rows * (waves * full + f.few + (full - f.few) * last);
+  }
+  auto total = [&](const std::vector<char>& one) {
+    double t = 0.0;
+    int groups = 0, rows = 0;
+    for (size_t q = 0; q < n; ++q) {
+      const a2d_plan::LineClass& c = P->line_classes[q];
+      if (one[q]) {
+        t += cost[q];
+      } else {
+        groups += c.groups * c.count;
+        rows = std::max(rows, c.rows);
+      }
+    }
+    if (groups == 0) return t;
+    const int waves = (groups - 1) / f.ctas;
+    const double last = (double)(groups - waves * f.ctas) / f.ctas;
+    return t + rows * (waves * f.sfull + f.sfew + (f.sfull - f.sfew) * last);
+  };
+  // from every class that fits, and from none: change the class that gains most while one does
+  std::vector<char> best(n, 0);
+  double best_t = total(best);
+  for (int start = 0; start < 2; ++start) {
+    std::vector<char> one(n, 0);
+    if (start == 0)
+      for (size_t q = 0; q < n; ++q) one[q] = P->line_classes[q].fits;
+    double t = total(one);
+    for (bool more = true; more;) {
+      more = false;
+      size_t at = 0;
+      for (size_t q = 0; q < n; ++q) {
+        if (!P->line_classes[q].fits) continue;
+        one[q] ^= 1;
+        const double u = total(one);
+        one[q] ^= 1;
+        if (u < t) {
+          t = u;
+          at = q;
+          more = true;
+        }
+      }
+      if (more) one[at] ^= 1;
+    }
+    if (t <= best_t) {
+      best_t = t;
+      best = one;
+    }
+  }
+  P->rest_groups.clear();
+  for (size_t q = 0; q < n; ++q) {
+    a2d_plan::LineClass& c = P->line_classes[q];
+    c.one = best[q] != 0;
+    if (c.one) continue;
+    for (int k = c.first; k < c.first + c.count; ++k) {
+      const CaseDev& cs = P->cases[P->line_cases[k]];
+      P->rest_groups.insert(P->rest_groups.end(), P->groups.begin() + cs.group0, P->groups.begin() + cs.group0 + cs.ngroups);
+    }
+  }
 }
 
 // x = M^-1 r: jacobi_sweeps line-Jacobi sweeps (aero2d/implicit.py:150-157);
@@ -490,24 +593,27 @@ template <typename TJ>
 static void precond(a2d_plan* P, const Batch& B, const double* rin, double* dst, uint32_t need, cudaStream_t s) {
   SweepArgs a = sweep_args(P, need);
   const int sweeps = std::max(1, P->p.jacobi_sweeps);
+  Batch rest = B;
   if (one_launch(P)) {
     a.r = rin;
     a.e0 = P->at<double>(P->o_E0);
     a.x = dst;
     for (const a2d_plan::LineClass& c : P->line_classes)
-      launch_lines<TJ>(B, a, P->at<int>(P->o_lcases) + c.first, c.count, c.groups, c.rows, sweeps, s);
-    return;
+      if (c.one) launch_lines<TJ>(B, a, P->at<int>(P->o_lcases) + c.first, c.count, c.groups, c.rows, sweeps, s);
+    if (P->rest_groups.empty()) return;
+    rest.groups = P->at<Group>(P->o_rgroups);
+    rest.ngroups = (int)P->rest_groups.size();
   }
   double* bufs[2] = {P->vec(kPA), P->vec(kPB)};
   a.r = rin;
   a.e0 = sweeps > 1 ? P->vec(kPE) : nullptr;
   a.x = sweeps > 1 ? bufs[0] : dst;
-  launch_sweep<TJ, true>(B, a, sweeps == 1, s, P->sweep_variant);
+  launch_sweep<TJ, true>(rest, a, sweeps == 1, s, P->sweep_variant);
   for (int sw = 1; sw < sweeps; ++sw) {
     const bool last = sw == sweeps - 1;
     a.xprev = a.x;
     a.x = last ? dst : bufs[sw & 1];
-    launch_sweep<TJ, false>(B, a, last, s, P->sweep_variant);
+    launch_sweep<TJ, false>(rest, a, last, s, P->sweep_variant);
   }
 }
 
@@ -971,16 +1077,9 @@ int a2d_plan_bind(a2d_plan* P, void* workspace, size_t bytes, void* stream) {
   A2D_CK(cudaMemsetAsync(P->ws + P->o_cnt, 0, 8, s));
   A2D_CK(cudaMemsetAsync(P->ws + P->o_sat, 0, sizeof(unsigned long long), s));
   A2D_CK(sweep_init());
-  P->lines_fit = true;
-  for (const a2d_plan::LineClass& c : P->line_classes) {
-    const bool mixed = P->p.precision == A2D_MIXED;
-    const int n = mixed ? lines_clusters<float>(c.groups, c.rows) : lines_clusters<double>(c.groups, c.rows);
-    // FP64 holds one CTA per SM, and a cluster is bound by the length of its lines: past
-    // the cases that run at once the per-sweep kernels win (256 x 64, B200: 8 cases 111 against
-    // 193 us, 16 cases in two waves 196 against 180); the mixed one wins at every count measured
-    // (1 to 64 cases: 39 against 85, 137 against 180)
-    P->lines_fit = P->lines_fit && (mixed ? n > 0 : n >= c.count);
-  }
+  choose_lines(P);
+  A2D_CK(cudaMemcpyAsync(P->ws + P->o_rgroups, P->rest_groups.data(), sizeof(Group) * P->rest_groups.size(),
+                         cudaMemcpyHostToDevice, s));
   A2D_CK(gs_init());
   // Arnoldi steps in one launch while every case's cluster runs at once (a second wave would cost
   // more than the launches saved); of the cluster sizes the one whose shared memory takes

@@ -503,7 +503,8 @@ static bool one_launch(const a2d_plan* P) {
 // 128 cases: within 0.5 % of the better path on average, 1.95x faster than always one launch at 96
 // cases of 384 x 143, and slower than that nowhere) and 128 FP64 ones.  Ragged, one launch a class
 // against the per-sweep kernels (48 rows, a case each, mixed / FP64): two classes 58 and 66 us / 96 and 128, three
-// 86 and 66 / 143 and 129, sixteen 530 and 69 / 763 and 138.
+// 86 and 66 / 143 and 129, sixteen 530 and 69 / 763 and 138; two cases each of
+// 96 x 24, 128 x 32, 192 x 48, 256 x 64 and 384 x 96 cells 179 and 129 / 267 and 267.
 static void choose_lines(a2d_plan* P) {
   const bool mixed = P->p.precision == A2D_MIXED;
   struct Fit {
@@ -512,7 +513,7 @@ static void choose_lines(a2d_plan* P) {
     double sfew, sfull;
     int ctas;                  // per-sweep CTAs that run at once
   };
-  const Fit f = mixed ? Fit{0.5, 0.75, 0.9, 142, 1.3, 2.8, 4 * 148} : Fit{1.0, 1.2, 1.2, 0, 2.45, 4.7, 3 * 148};
+  const Fit f = mixed ? Fit{0.58, 0.85, 0.86, 142, 1.2, 2.9, 4 * 148} : Fit{1.0, 1.2, 1.2, 0, 2.45, 4.7, 3 * 148};
   const size_t n = P->line_classes.size();
   std::vector<double> cost(n, 0.0);
   for (size_t q = 0; q < n; ++q) {

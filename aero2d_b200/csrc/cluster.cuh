@@ -26,7 +26,7 @@ __device__ __forceinline__ uint32_t peer_addr(const void* p, uint32_t rank) {
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_u32(p)), "r"(rank));
   return r;
 }
-// bounded wait that acquires other CTAs' stores
+// bounded wait of a whole warp that acquires other CTAs' stores, with one verdict
 __device__ __forceinline__ bool wait_cluster(uint64_t* bar, uint32_t parity) {
   auto try_once = [&]() {
     uint32_t ok;
@@ -41,14 +41,7 @@ __device__ __forceinline__ bool wait_cluster(uint64_t* bar, uint32_t parity) {
         : "memory");
     return ok != 0;
   };
-#pragma unroll 1
-  for (int q = 0; q < kWaitTries; ++q)
-    if (try_once()) return true;
-  const unsigned long long t0 = global_ns();
-  while (!try_once()) {
-    if (global_ns() - t0 > kWaitLimitNs) return false;
-  }
-  return true;
+  return bounded_wait(try_once, global_ns, warp_all);
 }
 
 }  // namespace a2d

@@ -29,7 +29,10 @@
 // (sweep.cu, sweep_rows.cu, sweep_pairs.cu), so results are bitwise the same.  Every wait is
 // bounded (tma.cuh); a wait that runs out records an error, and its CTA stays until
 // the other CTAs of the cluster are done or have given up too, so none of them
-// stores into the shared memory of a CTA that has gone.  No cluster multicast.
+// stores into the shared memory of a CTA that has gone.  A warp leaves as a whole (waits.cuh):
+// helper and service warps by their waits' vote, which costs 1 to 2 % of an application in the
+// recurrence warps; there a lane whose wait runs out is no longer `alive`, waits for nothing
+// further and signals nothing, and the warp votes once, at the end.  No cluster multicast.
 #include <algorithm>
 #include <type_traits>
 
@@ -307,7 +310,7 @@ __device__ __forceinline__ bool serve(const Cta<TI> c, const SweepArgs& a, size_
   uint32_t ph = 0;
 #pragma unroll 1
   for (int p = 0; p < total; ++p) {
-    if (!mbar_wait(c.empty(h, s), ph)) {
+    if (!mbar_wait_warp(c.empty(h, s), ph)) {
       // the recurrence stopped: the copies in flight get a bounded time to land
       for (int u = p; u < min(p + S, total); ++u) (void)mbar_wait(c.full(h, u % S), (u / S) & 1);
       return false;
@@ -469,6 +472,7 @@ __device__ __forceinline__ bool recur(const Cta<TI> c, const SweepArgs& a, size_
   const int dir = h == 0 ? 1 : -1;
   int s = 0;              // ring stage
   uint32_t sph = 0;       // and its phase
+  bool alive = true;
   // block u of the stage, this lane's four rows
   auto block = [&](int u, Raw(&raw)[4]) {
     const TF* b = reinterpret_cast<const TF*>(c.stage(h, s) + u * kBlk) + lane * 4;
@@ -480,7 +484,7 @@ __device__ __forceinline__ bool recur(const Cta<TI> c, const SweepArgs& a, size_
   // overwritten
   auto retire = [&]() {
     __syncwarp();
-    if (lane == 0) mbar_arrive(c.empty(h, s));
+    if (lane == 0 && alive) mbar_arrive(c.empty(h, s));
     if (++s == S) {
       s = 0;
       sph ^= 1;
@@ -526,8 +530,8 @@ __device__ __forceinline__ bool recur(const Cta<TI> c, const SweepArgs& a, size_
 #pragma unroll 1
     for (int t = 0; t < nf; t += kPack) {
       const int j = c.row_of(h, t);
-      if (!have && !mbar_wait(c.full(h, s), sph)) return false;
-      if (!have_e && !mbar_wait(c.ready(h, t / kBatch), ph)) return false;
+      alive = alive && (have || mbar_wait(c.full(h, s), sph));
+      alive = alive && (have_e || mbar_wait(c.ready(h, t / kBatch), ph));
       have = try_next();
       have_e = t + kPack < nf && mbar_test(c.ready(h, t / kBatch + 1), ph);
       int u0 = 0;
@@ -547,9 +551,9 @@ __device__ __forceinline__ bool recur(const Cta<TI> c, const SweepArgs& a, size_
     // the halves meet at row k
     TC x[4];
     if (h == 0) {
-      if (!mbar_wait(c.ready(0, k / kBatch), ph)) return false;
-      if (!have && !mbar_wait(c.full(h, s), sph)) return false;
-      if (!mbar_wait(c.meet(0), ph)) return false;
+      alive = alive && mbar_wait(c.ready(0, k / kBatch), ph);
+      alive = alive && (have || mbar_wait(c.full(h, s), sph));
+      alive = alive && mbar_wait(c.meet(0), ph);
       have = try_next();
       TC e[4], dp[4] = {TC(0), TC(0), TC(0), TC(0)};
       row_load(c.row(k), lane, e);
@@ -572,7 +576,7 @@ __device__ __forceinline__ bool recur(const Cta<TI> c, const SweepArgs& a, size_
       row_store(c.xk(), lane, x);
       if (!last) row_store(c.row(k), lane, x);
       __syncwarp();
-      if (lane == 0) mbar_arrive(c.meet(1));
+      if (lane == 0 && alive) mbar_arrive(c.meet(1));
       retire();
       if (last && owner) {
 #pragma unroll
@@ -580,9 +584,9 @@ __device__ __forceinline__ bool recur(const Cta<TI> c, const SweepArgs& a, size_
       }
     } else {
       __syncwarp();
-      if (lane == 0) mbar_arrive(c.meet(0));
+      if (lane == 0 && alive) mbar_arrive(c.meet(0));
       // also without rows of its own: a half runs at most one sweep ahead of the other
-      if (!mbar_wait(c.meet(1), ph)) return false;
+      alive = alive && mbar_wait(c.meet(1), ph);
       row_load(c.xk(), lane, x);
     }
     // back substitution outward from row k: x_j = d_j - C_j x_{j+-1}
@@ -591,7 +595,7 @@ __device__ __forceinline__ bool recur(const Cta<TI> c, const SweepArgs& a, size_
     for (int t = 0; t < nf; t += kPack) {
       const int j = h == 0 ? k - 1 - t : k + 1 + t;
       const int top = min(kPack, nf - t) - 1;    // the wall half walks down the pack's rows
-      if (!have && !mbar_wait(c.full(h, s), sph)) return false;
+      alive = alive && (have || mbar_wait(c.full(h, s), sph));
       have = try_next();
       int u0 = 0;
       auto in = [&](int u, TC(&y)[4], Raw(&raw)[4]) {
@@ -616,7 +620,7 @@ __device__ __forceinline__ bool recur(const Cta<TI> c, const SweepArgs& a, size_
       retire();
     }
   }
-  return true;
+  return warp_all(alive);
 }
 
 template <typename TI>

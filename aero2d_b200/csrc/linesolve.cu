@@ -336,8 +336,8 @@ __global__ void __launch_bounds__(factor_threads(H), 512 / factor_threads(H)) k_
     for (int q = 0, h = 0; q < rows; ++q) {
       FactorRow& row = sm.row[half][h];
       const bool twist = half == 0 && q == k;
-      ok = mbar_wait(&sm.assembled[half][h], phase);
-      if (ok && twist) ok = mbar_wait(&sm.far, 0);
+      ok = mbar_wait_warp(&sm.assembled[half][h], phase);
+      if (ok && twist) ok = mbar_wait_warp(&sm.far, 0);
       if (!ok) break;
       if (own) {
         double D[16], B[16], inv[16];
@@ -444,7 +444,7 @@ __global__ void __launch_bounds__(factor_threads(H), 512 / factor_threads(H)) k_
       for (int e = 0; e < 16; ++e) row.D[e][lane] = D[e];
     }
     warp_arrive(&sm.assembled[half][helper], lane);
-    ok = mbar_wait(&sm.inverted[half][helper], phase);
+    ok = mbar_wait_warp(&sm.inverted[half][helper], phase);
     if (!ok) break;
     if (own) {
       // row j's sweep factors: inv, C (the back-substitution coupling), G (the

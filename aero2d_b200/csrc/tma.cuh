@@ -8,9 +8,9 @@
 #pragma once
 #include <cstdint>
 
-namespace a2d {
+#include "waits.cuh"
 
-constexpr unsigned long long kWaitLimitNs = 1000000000ull;   // 1 s
+namespace a2d {
 
 // how long one try of a wait may suspend its warp (it wakes when the phase completes)
 constexpr uint32_t kSuspendNs = 100000;
@@ -69,20 +69,18 @@ __device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
   return ok != 0;
 }
 
-// tries before a wait starts to read the clock: most waits are over by then, and a
-// %globaltimer read takes longer than they do
-constexpr int kWaitTries = 64;
-
-// waits for the phase of parity `parity` to complete; false after kWaitLimitNs
+// waits for the phase of parity `parity` to complete; false after kWaitLimitNs.  By lanes each for
+// itself, which vote on the verdicts before they go different ways
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
-#pragma unroll 1
-  for (int q = 0; q < kWaitTries; ++q)
-    if (mbar_try_wait(bar, parity)) return true;
-  const unsigned long long t0 = global_ns();
-  while (!mbar_try_wait(bar, parity)) {
-    if (global_ns() - t0 > kWaitLimitNs) return false;
-  }
-  return true;
+  return bounded_wait([&] { return mbar_try_wait(bar, parity); }, global_ns, [](bool b) { return b; });
+}
+
+// a verdict of the whole warp
+__device__ __forceinline__ bool warp_all(bool b) { return __all_sync(0xffffffffu, b); }
+
+// the same by a whole warp, with one verdict
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity) {
+  return bounded_wait([&] { return mbar_try_wait(bar, parity); }, global_ns, warp_all);
 }
 
 // bulk copy of `bytes` (multiple of 16, both addresses 16-byte aligned) into

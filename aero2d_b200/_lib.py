@@ -85,6 +85,7 @@ SIGNATURES = {
     "a2d_plan_ncases": (_I, [_P]),
     "a2d_plan_set_tuning": (_I, [_P, _I, _I, _P]),
     "a2d_plan_get_tuning": (_I, [_P, C.POINTER(_I), C.POINTER(_I)]),
+    "a2d_plan_paths": (_I, [_P, C.POINTER(C.c_uint)]),
     "a2d_vec_set": (_I, [_P, _I, _I, _P, _P]),
     "a2d_vec_get": (_I, [_P, _I, _I, _P, _P]),
     "a2d_vec_get_prim": (_I, [_P, _I, _I, _P, _P]),

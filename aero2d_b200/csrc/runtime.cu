@@ -1032,6 +1032,21 @@ int a2d_plan_get_tuning(const a2d_plan* P, int* jvp_tile, int* sweep_variant) {
   return A2D_OK;
 }
 
+int a2d_plan_paths(const a2d_plan* P, unsigned* paths) {
+  if (paths == nullptr) return fail(A2D_ERR_ARG, "null output");
+  A2D_BOUND(P);
+  const bool mixed = P->p.precision == A2D_MIXED;
+  unsigned v = 0;
+  if (!P->ftiles.empty() && P->ftiles.size() <= (size_t)(mixed ? kFineTiles32 : kFineTiles64)) v |= A2D_PATH_FINE_TILES;
+  if (P->rest_groups.size() < P->groups.size()) v |= A2D_PATH_LINES;
+  if (!P->rest_groups.empty()) v |= A2D_PATH_SWEEPS;
+  if (P->gs_vectors > 0) v |= A2D_PATH_ARNOLDI;
+  if (P->irs_entries > 0) v |= A2D_PATH_SMOOTH;
+  if (P->irs_rest) v |= A2D_PATH_SMOOTH_ROWS;
+  *paths = v;
+  return A2D_OK;
+}
+
 int a2d_plan_bind(a2d_plan* P, void* workspace, size_t bytes, void* stream) {
   if (P == nullptr || workspace == nullptr) return fail(A2D_ERR_ARG, "bind: null argument");
   if (bytes < P->bytes) return fail(A2D_ERR_ARG, "bind: workspace too small");

@@ -129,6 +129,14 @@ class Plan:
         inv_v = {b: a for a, b in _lib.SWEEP_VARIANTS.items()}
         return inv_t[t.value], inv_v[v.value]
 
+    PATHS = ("fine_tiles", "lines", "sweeps", "arnoldi", "smooth", "smooth_rows")
+
+    def paths(self) -> set[str]:
+        """Which paths the plan's sizes take in the starting configuration (include/aero2d_b200.h, A2D_PATH_*)."""
+        v = C.c_uint()
+        _lib.check(self.lib.a2d_plan_paths(self.handle, C.byref(v)))
+        return {n for k, n in enumerate(self.PATHS) if v.value >> k & 1}
+
     @property
     def stream(self) -> int:
         return stream_handle(self.device)

@@ -122,6 +122,15 @@ int a2d_plan_ncases(const a2d_plan* plan);
 /* any time, bound or not; a change re-captures the Newton step's graph at the next step */
 int a2d_plan_set_tuning(a2d_plan* plan, int jvp_tile, int sweep_variant, void* stream);
 int a2d_plan_get_tuning(const a2d_plan* plan, int* jvp_tile, int* sweep_variant);
+/* which paths a bound plan's sizes take in the starting configuration, on the device it is bound to (no effect
+ * on results) */
+#define A2D_PATH_FINE_TILES 1   /* stencils on 16 x 4 tiles                                       */
+#define A2D_PATH_LINES 2        /* the preconditioner's sweeps in one launch, for some cases       */
+#define A2D_PATH_SWEEPS 4       /* a launch per sweep, for some cases                              */
+#define A2D_PATH_ARNOLDI 8      /* Arnoldi steps in one launch                                     */
+#define A2D_PATH_SMOOTH 16      /* explicit iteration: smoothing and update fused, for some cases  */
+#define A2D_PATH_SMOOTH_ROWS 32 /* and in kernels of their own, for some cases                     */
+int a2d_plan_paths(const a2d_plan* plan, unsigned* paths);
 
 /* vector I/O in the reference layout [4][ni][nc] of one case (device pointers) */
 int a2d_vec_set(a2d_plan* plan, int slot, int case_index, const double* src, void* stream);

@@ -44,11 +44,7 @@ def test_short_cases_keep_the_fused_kernel(cuda):
     solvers = [EulerSolver(ring(*s), dtype=np.float64, device=cuda) for s in SHAPES]
     w = solvers[0].freestream(np.array([0.4, 0.5, 0.6]), np.array([0.0, 1.0, 2.0]))
     pl = Plan([s.dgrid for s in solvers], w, solvers[0].params(), cuda, tuning=None)
-    pl.init_freestream()
-    pl.set_circulation(0.05)
-    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
-        for _ in range(6):   # the profiler can lose a window's first launches
-            pl.rk_iterate(1)
-            torch.cuda.synchronize()
-    names = [e.key for e in prof.key_averages()]
-    assert any("k_irs<" in n for n in names) and any("k_irs_i<" in n for n in names), names
+    assert {"smooth", "smooth_rows"} <= pl.paths()
+    pl.close()
+    pl = Plan([solvers[0].dgrid], w[:1], solvers[0].params(), cuda, tuning=None)
+    assert "smooth" in pl.paths() and "smooth_rows" not in pl.paths()

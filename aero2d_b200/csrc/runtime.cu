@@ -130,6 +130,7 @@ struct a2d_plan {
   char* ws = nullptr;
   Batch batch{};
   cudaGraphExec_t graph = nullptr;
+  bool graph_failed = false;   // by the step before
   cudaStream_t graph_stream = nullptr;
   // a step's live count and failure flag on the host; not pinned: 8 bytes whose reader waits anyway, while
   // cudaMallocHost and cudaFreeHost took 0.9 to 2.5 and 0.4 ms of a plan's life
@@ -857,6 +858,42 @@ static void newton_dispatch(a2d_plan* P, cudaStream_t s) {
   else newton_step_launches<double, double, double>(P, s);
 }
 
+// the graph of a Newton step, captured on a stream of its own; a failure leaves no error behind
+static int build_graph(a2d_plan* P) {
+  auto failed = [](const char* what, cudaError_t e) {
+    (void)cudaGetLastError();
+    return fail(A2D_ERR_CUDA, std::string(what) + ": " + cudaGetErrorString(e));
+  };
+  cudaStream_t cap;
+  if (cudaError_t e = cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking)) return failed("graph capture", e);
+  cudaGraph_t g = nullptr;
+  cudaError_t e = cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal);
+  if (e == cudaSuccess) {
+    newton_dispatch(P, cap);
+    e = cudaStreamEndCapture(cap, &g);
+  }
+  cudaStreamDestroy(cap);
+  if (e != cudaSuccess) return failed("graph capture", e);
+  size_t nn = 0;
+  if (cudaGraphGetNodes(g, nullptr, &nn) == cudaSuccess && nn > 0) {
+    std::vector<cudaGraphNode_t> nodes(nn);
+    if (cudaGraphGetNodes(g, nodes.data(), &nn) == cudaSuccess) {
+      int nk = 0;
+      for (size_t q = 0; q < nn; ++q) {
+        cudaGraphNodeType ty;
+        if (cudaGraphNodeGetType(nodes[q], &ty) == cudaSuccess && ty == cudaGraphNodeTypeKernel) ++nk;
+      }
+      P->kernels_per_step = nk;
+    }
+  }
+  cudaGraphExec_t exec = nullptr;
+  e = cudaGraphInstantiate(&exec, g, 0);
+  cudaGraphDestroy(g);
+  if (e != cudaSuccess) return failed("graph instantiate", e);
+  P->graph = exec;
+  return A2D_OK;
+}
+
 static int newton_step(a2d_plan* P, cudaStream_t s) {
   if (!P->p.use_graph) {
     newton_dispatch(P, s);
@@ -865,38 +902,18 @@ static int newton_step(a2d_plan* P, cudaStream_t s) {
   }
   if (P->graph == nullptr) {
     // a plan's first step goes out kernel by kernel, and the graph of the later ones is captured
-    // and instantiated while it runs
+    // and instantiated while it runs.  If that fails the step is made all the same; the next
+    // one then builds the graph before anything of it runs, so that no error follows a step
     cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
     A2D_CK(cudaStreamIsCapturing(s, &status));
-    const bool first = status == cudaStreamCaptureStatusNone;
-    if (first) {
+    if (status == cudaStreamCaptureStatusNone && !P->graph_failed) {
       newton_dispatch(P, s);
       A2D_CK(cudaGetLastError());
+      P->graph_failed = build_graph(P) != A2D_OK;
+      return A2D_OK;
     }
-    cudaStream_t cap;
-    A2D_CK(cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking));
-    cudaGraph_t g;
-    A2D_CK(cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal));
-    newton_dispatch(P, cap);
-    cudaError_t e = cudaStreamEndCapture(cap, &g);
-    cudaStreamDestroy(cap);
-    if (e != cudaSuccess) return fail(A2D_ERR_CUDA, std::string("graph capture: ") + cudaGetErrorString(e));
-    size_t nn = 0;
-    if (cudaGraphGetNodes(g, nullptr, &nn) == cudaSuccess && nn > 0) {
-      std::vector<cudaGraphNode_t> nodes(nn);
-      if (cudaGraphGetNodes(g, nodes.data(), &nn) == cudaSuccess) {
-        int nk = 0;
-        for (size_t q = 0; q < nn; ++q) {
-          cudaGraphNodeType ty;
-          if (cudaGraphNodeGetType(nodes[q], &ty) == cudaSuccess && ty == cudaGraphNodeTypeKernel) ++nk;
-        }
-        P->kernels_per_step = nk;
-      }
-    }
-    e = cudaGraphInstantiate(&P->graph, g, 0);
-    cudaGraphDestroy(g);
-    if (e != cudaSuccess) return fail(A2D_ERR_CUDA, std::string("graph instantiate: ") + cudaGetErrorString(e));
-    if (first) return A2D_OK;
+    if (int e = build_graph(P)) return e;
+    P->graph_failed = false;
   }
   A2D_CK(cudaGraphLaunch(P->graph, s));
   return A2D_OK;
@@ -1018,6 +1035,7 @@ int a2d_plan_set_tuning(a2d_plan* P, int jvp_tile, int sweep_variant, void* stre
     }
   }
   P->sweep_variant = sweep_variant;
+  P->graph_failed = false;
   if (P->graph != nullptr) {   // the captured step holds the old launch configuration
     cudaGraphExecDestroy(P->graph);
     P->graph = nullptr;
@@ -1052,6 +1070,7 @@ int a2d_plan_bind(a2d_plan* P, void* workspace, size_t bytes, void* stream) {
   if (bytes < P->bytes) return fail(A2D_ERR_ARG, "bind: workspace too small");
   if ((reinterpret_cast<uintptr_t>(workspace) & 255) != 0) return fail(A2D_ERR_ARG, "bind: workspace not 256-byte aligned");
   cudaStream_t s = static_cast<cudaStream_t>(stream);
+  P->graph_failed = false;
   if (P->graph != nullptr) {
     cudaGraphExecDestroy(P->graph);
     P->graph = nullptr;

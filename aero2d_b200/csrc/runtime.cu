@@ -275,7 +275,7 @@ static void layout(a2d_plan* P) {
   P->o_cp = cv.take(8 * (size_t)P->total_ni);
   P->o_hrn = cv.take(8 * (size_t)B * P->p.max_iter);
   P->o_hcl = cv.take(8 * (size_t)B * P->p.max_iter);
-  P->o_cnt = cv.take(8);   // [0] live-case count, [1] failure flag of the bounded waits of the sweeps and the factors
+  P->o_cnt = cv.take(8);   // [0] live-case count, [1] failure flag of the kernels' bounded waits
   P->o_idx = cv.take(sizeof(int) * (size_t)B);   // case index lists of a2d_case_restart / _retire
   P->o_sat = cv.take(sizeof(unsigned long long));
   P->o_jtiles = cv.take(sizeof(Tile) * (size_t)P->max_jtiles);
@@ -858,6 +858,12 @@ static void newton_dispatch(a2d_plan* P, cudaStream_t s) {
   else newton_step_launches<double, double, double>(P, s);
 }
 
+// what the failure word of a plan's kernels stands for
+static int wait_failure() {
+  return fail(A2D_ERR_CUDA,
+              "a bounded wait inside a kernel ran out of time (line sweeps, line factors or a one-launch Arnoldi step)");
+}
+
 // the graph of a Newton step, captured on a stream of its own; a failure leaves no error behind
 static int build_graph(a2d_plan* P) {
   auto failed = [](const char* what, cudaError_t e) {
@@ -1408,7 +1414,7 @@ int a2d_newton_run(a2d_plan* P, int max_steps, int* steps, void* stream) {
     k_count<<<1, 256, 0, s>>>(P->ncases, P->ctl(), P->live(), P->p.retire, dcount);
     A2D_CK(cudaMemcpyAsync(P->host_count, dcount, 2 * sizeof(int), cudaMemcpyDeviceToHost, s));
     A2D_CK(cudaStreamSynchronize(s));
-    if (P->host_count[1] != 0) return fail(A2D_ERR_CUDA, "line sweep: a bulk-copy wait ran out of time");
+    if (P->host_count[1] != 0) return wait_failure();
     if (*P->host_count == 0) break;
   }
   if (steps != nullptr) *steps = done;
@@ -1433,7 +1439,7 @@ int a2d_live_count(a2d_plan* P, int* n, void* stream) {
   k_count<<<1, 256, 0, s>>>(P->ncases, P->ctl(), P->live(), P->p.retire, dcount);
   A2D_CK(cudaMemcpyAsync(P->host_count, dcount, 2 * sizeof(int), cudaMemcpyDeviceToHost, s));
   A2D_CK(cudaStreamSynchronize(s));
-  if (P->host_count[1] != 0) return fail(A2D_ERR_CUDA, "line sweep: a bulk-copy wait ran out of time");
+  if (P->host_count[1] != 0) return wait_failure();
   *n = *P->host_count;
   return A2D_OK;
 }

@@ -19,9 +19,11 @@ The best configuration depends on the grid sizes in a batch, the batch size and
 the precision.  `apply(plan, measure=True)` looks the plan's key up in the
 cache; on a miss it times a few Newton steps of the plan under every candidate
 (CUDA events on the plan's stream), keeps the fastest, stores it and leaves the
-plan at the freestream.  The key is the GPU model, the library's version, the
-precision and the plan's signature: its grid sizes with the number of cases of
-each size rounded up to a power of two.
+plan at the freestream.  The key is the GPU model, the library's version and the
+kernels' (KERNELS), the precision, the plan's signature, its grid sizes with the
+number of cases of each size rounded up to a power of two, and which of the paths
+that the two knobs choose between its exact sizes take (Plan.paths): a choice
+timed on one side of a dispatch limit is not applied on the other.
 
 The cache is one JSON file, $AERO2D_B200_TUNING or
 ~/.cache/aero2d_b200/tuning.json, written atomically (a temporary file
@@ -40,6 +42,11 @@ JVP_TILES = ("32x8", "32x16", "64x4", "16x16")
 SWEEPS = ("lanes", "rows", "pairs", "halves")
 MIXED_ONLY_SWEEPS = ("rows", "halves")   # refused on FP64 plans
 DEFAULT = ("32x16", "halves")   # a new plan's configuration (the library's defaults)
+# Raised with every change of the kernels or of their dispatch that moves what the tuner times, so that
+# choices stored before it are measured anew.  2: the sweeps of an application in one launch,
+# 16x4 stencil tiles in small batches
+KERNELS = 2
+KEY_PATHS = ("fine_tiles", "lines", "sweeps")
 
 
 def default_path() -> Path:
@@ -66,8 +73,8 @@ def signature(shapes: Iterable[tuple[int, int]], precision: int) -> str:
 
 def candidates(precision: int) -> list[tuple[str, str]]:
     """Every configuration worth timing: the JVP tile shapes matter only in
-    the mixed precision (the FP64 JVP always runs 32 x 8 tiles), and the rows
-    and halves sweeps run mixed-precision plans only."""
+    the mixed precision (the FP64 JVP runs 32 x 8 tiles, small batches 16 x 4,
+    whatever is set), and the rows and halves sweeps run mixed-precision plans only."""
     if precision:
         return [(t, v) for t in JVP_TILES for v in SWEEPS]
     return [(JVP_TILES[0], v) for v in SWEEPS if v not in MIXED_ONLY_SWEEPS]
@@ -128,15 +135,17 @@ def device_key(device) -> str:
     import torch
     from . import _lib
     name = torch.cuda.get_device_name(device)
-    return f"{name}|lib{_lib.load().a2d_version()}"
+    return f"{name}|lib{_lib.load().a2d_version()}.{KERNELS}"
 
 
 def plan_key(plan) -> str:
     """The cache key of a plan (a service's lanes: the first lane's cases and the
     lane count, since the lanes are timed stepping together)."""
     lanes = int(getattr(plan, "lanes", 1))
+    taken = plan.paths() if hasattr(plan, "paths") else ()
+    paths = "+".join(p for p in KEY_PATHS if p in taken)
     return (device_key(plan.device) + "|" + signature(plan.shapes, plan.params.precision) +
-            (f"|lanes{lanes}" if lanes > 1 else ""))
+            (f"|{paths}" if paths else "") + (f"|lanes{lanes}" if lanes > 1 else ""))
 
 
 def time_newton_steps(plan, steps: int = 2) -> float:

@@ -34,6 +34,15 @@ def _ptr(t: torch.Tensor) -> int:
     return t.data_ptr()
 
 
+PATHS = ("fine_tiles", "lines", "sweeps", "arnoldi", "smooth", "smooth_rows")
+
+
+def paths_of(lib, handle) -> set[str]:
+    v = C.c_uint()
+    _lib.check(lib.a2d_plan_paths(handle, C.byref(v)))
+    return {n for k, n in enumerate(PATHS) if v.value >> k & 1}
+
+
 class DeviceGrid:
     """An O-grid resident on the device: node coordinates and the metrics blob
     (cell areas, face vectors, wall and far-field face midpoints, FP64 and FP32)."""
@@ -129,13 +138,9 @@ class Plan:
         inv_v = {b: a for a, b in _lib.SWEEP_VARIANTS.items()}
         return inv_t[t.value], inv_v[v.value]
 
-    PATHS = ("fine_tiles", "lines", "sweeps", "arnoldi", "smooth", "smooth_rows")
-
     def paths(self) -> set[str]:
         """Which paths the plan's sizes take in the starting configuration (include/aero2d_b200.h, A2D_PATH_*)."""
-        v = C.c_uint()
-        _lib.check(self.lib.a2d_plan_paths(self.handle, C.byref(v)))
-        return {n for k, n in enumerate(self.PATHS) if v.value >> k & 1}
+        return paths_of(self.lib, self.handle)
 
     @property
     def stream(self) -> int:

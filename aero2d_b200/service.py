@@ -31,7 +31,7 @@ import torch
 from . import _lib
 from .euler import GAMMA, _precision_of
 from .grid import OGrid
-from .plan import DeviceGrid, _ptr, device_of, stream_handle
+from .plan import DeviceGrid, _ptr, device_of, paths_of, stream_handle
 
 
 def freestream(mach, alpha_deg) -> np.ndarray:
@@ -281,6 +281,9 @@ class _PlanView:
         _lib.check(self.lib.a2d_plan_get_tuning(self.handle, C.byref(t), C.byref(v)))
         return ({b: a for a, b in _lib.JVP_TILES.items()}[t.value],
                 {b: a for a, b in _lib.SWEEP_VARIANTS.items()}[v.value])
+
+    def paths(self) -> set[str]:
+        return paths_of(self.lib, self.handle)
 
     def init_freestream(self) -> None:
         self._each("a2d_init_freestream")

@@ -76,6 +76,7 @@ SIGNATURES = {
     "a2d_default_params": (None, [C.POINTER(Params)]),
     "a2d_metrics_bytes": (_I, [_I, _I, C.POINTER(_SZ)]),
     "a2d_metrics_build": (_I, [_I, _I, _P, _P, _P, _P]),
+    "a2d_metrics_build_each": (_I, [_I, _I, _I, _P, _P, C.POINTER(_P), _P]),
     "a2d_metrics_build_batch": (_I, [_I, _I, _I, _P, _P, _P, _SZ, _P]),
     "a2d_plan_create": (_I, [_I, C.POINTER(_I), C.POINTER(_I), C.POINTER(_P), C.POINTER(_D),
                              C.POINTER(Params), C.POINTER(_P)]),

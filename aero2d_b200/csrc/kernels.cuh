@@ -100,8 +100,8 @@ struct SweepArgs {
   uint32_t need = 0;
 };
 
-void launch_metrics(int n, int ni, int nc, const double* x, const double* y, void* metrics, size_t stride,
-                    size_t float_off, cudaStream_t s);
+void launch_metrics(int n, int ni, int nc, const double* x, const double* y, void* const* metrics, size_t float_off,
+                    cudaStream_t s);
 
 // shape: the tile shape of b's tile list (kTile*; kTile32x8 and kTile16x4 for every stencil, the others
 // for the FP32 linearised one)

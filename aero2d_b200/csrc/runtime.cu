@@ -969,7 +969,18 @@ int a2d_metrics_bytes(int ni, int nj, size_t* bytes) {
 }
 
 int a2d_metrics_build(int ni, int nj, const double* x, const double* y, void* metrics, void* stream) {
-  return a2d_metrics_build_batch(1, ni, nj, x, y, metrics, 0, stream);
+  return a2d_metrics_build_each(1, ni, nj, x, y, &metrics, stream);
+}
+
+int a2d_metrics_build_each(int n, int ni, int nj, const double* x, const double* y, void* const* metrics, void* stream) {
+  if (x == nullptr || y == nullptr || metrics == nullptr || ni < 4 || nj < 3 || n < 1)
+    return fail(A2D_ERR_ARG, "metrics: bad arguments");
+  for (int k = 0; k < n; ++k)
+    if (metrics[k] == nullptr || reinterpret_cast<uintptr_t>(metrics[k]) % 8 != 0)
+      return fail(A2D_ERR_ARG, "metrics: bad arguments");
+  launch_metrics(n, ni, nj - 1, x, y, metrics, metrics_float_offset(ni, nj - 1), static_cast<cudaStream_t>(stream));
+  A2D_CK(cudaGetLastError());
+  return A2D_OK;
 }
 
 int a2d_metrics_build_batch(int n, int ni, int nj, const double* x, const double* y, void* metrics, size_t stride,
@@ -977,10 +988,9 @@ int a2d_metrics_build_batch(int n, int ni, int nj, const double* x, const double
   if (x == nullptr || y == nullptr || metrics == nullptr || ni < 4 || nj < 3 || n < 1 || n > 65535 || stride % 8 != 0 ||
       (n > 1 && stride < metrics_total_bytes(ni, nj - 1)))
     return fail(A2D_ERR_ARG, "metrics: bad arguments");
-  launch_metrics(n, ni, nj - 1, x, y, metrics, stride, metrics_float_offset(ni, nj - 1),
-                 static_cast<cudaStream_t>(stream));
-  A2D_CK(cudaGetLastError());
-  return A2D_OK;
+  std::vector<void*> each(n);
+  for (int k = 0; k < n; ++k) each[k] = static_cast<char*>(metrics) + stride * k;
+  return a2d_metrics_build_each(n, ni, nj, x, y, each.data(), stream);
 }
 
 int a2d_plan_create(int ncases, const int* ni, const int* nc, const void* const* metrics, const double* winf,

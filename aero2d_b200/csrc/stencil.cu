@@ -13,6 +13,7 @@
 //
 // Reference: aero2d/euler.py:44-60 (metrics), :259-287 (residual),
 // :315-331 (forces), aero2d/implicit.py:160-181 (circulation and JVP).
+#include <algorithm>
 #include <type_traits>
 
 #include "batch.cuh"
@@ -26,10 +27,14 @@ namespace a2d {
 // ---------------------------------------------------------------------------
 // metrics from node coordinates (reference layout x[i][j], nj = nc + 1)
 // ---------------------------------------------------------------------------
-// a grid per blockIdx.y: nodes one grid after another, metrics `stride` bytes apart
-__global__ void k_metrics(int ni, int nc, const double* __restrict__ x, const double* __restrict__ y,
-                          char* __restrict__ metrics, size_t stride, size_t float_off) {
-  metrics += stride * blockIdx.y;
+// a grid per blockIdx.y: nodes one grid after another, metrics where each wants its own
+constexpr int kMetricsGrids = 128;   // of one launch, 1 KB of arguments
+struct MetricsOut {
+  char* at[kMetricsGrids];
+};
+__global__ void k_metrics(int ni, int nc, const double* __restrict__ x, const double* __restrict__ y, MetricsOut out,
+                          size_t float_off) {
+  char* __restrict__ metrics = out.at[blockIdx.y];
   double* __restrict__ md = reinterpret_cast<double*>(metrics);
   float* __restrict__ mf = reinterpret_cast<float*>(metrics + float_off);
   x += (size_t)ni * (nc + 1) * blockIdx.y;
@@ -138,11 +143,16 @@ __global__ void __launch_bounds__(256) k_forces(Batch b, const double* __restric
 // ---------------------------------------------------------------------------
 // host launchers
 // ---------------------------------------------------------------------------
-void launch_metrics(int n, int ni, int nc, const double* x, const double* y, void* metrics, size_t stride,
-                    size_t float_off, cudaStream_t s) {
+void launch_metrics(int n, int ni, int nc, const double* x, const double* y, void* const* metrics, size_t float_off,
+                    cudaStream_t s) {
   const size_t total = (size_t)ni * (nc + 1);
   const int blocks = (int)((total + 255) / 256);
-  k_metrics<<<dim3(blocks, n), 256, 0, s>>>(ni, nc, x, y, static_cast<char*>(metrics), stride, float_off);
+  for (int k = 0; k < n; k += kMetricsGrids) {
+    const int m = std::min(n - k, kMetricsGrids);
+    MetricsOut out;
+    for (int q = 0; q < m; ++q) out.at[q] = static_cast<char*>(metrics[k + q]);
+    k_metrics<<<dim3(blocks, m), 256, 0, s>>>(ni, nc, x + total * k, y + total * k, out, float_off);
+  }
 }
 
 template void launch_stencil<double, false, double>(const Batch&, const StencilArgs<double>&, cudaStream_t, int);

@@ -56,15 +56,15 @@ def ogrid_batch(airfoils: list[Airfoil], nj: int = 64, ds0: float = 2e-3, radius
             _lib.check(lib.a2d_grid_build(n, ni, nj, C.c_void_p(_ptr(ring_d)), C.c_void_p(_ptr(sp_d)),
                                           int(normal_smoothing), C.c_void_p(_ptr(x)), C.c_void_p(_ptr(y)),
                                           C.c_void_p(_ptr(amin)), C.c_void_p(s)))
-            # the metrics of them all and the grid objects, while the nodes are being computed
-            if ni >= 4 and nj >= 3 and n <= 65535:
+            # the metrics of them all, each in memory of its own that goes with its grid, and the grid
+            # objects, while the nodes are being computed
+            if ni >= 4 and nj >= 3:
                 size = C.c_size_t()
                 _lib.check(lib.a2d_metrics_bytes(ni, nj, C.byref(size)))
-                stride = -(-size.value // 256) * 256
-                blobs = torch.empty((n, stride), dtype=torch.uint8, device=dev)
-                _lib.check(lib.a2d_metrics_build_batch(n, ni, nj, C.c_void_p(_ptr(x)), C.c_void_p(_ptr(y)),
-                                                       C.c_void_p(_ptr(blobs)), stride, C.c_void_p(s)))
-                for k, xk, yk, m in zip(ks, x.unbind(), y.unbind(), blobs.unbind()):
+                blobs = [torch.empty(size.value, dtype=torch.uint8, device=dev) for _ in range(n)]
+                _lib.check(lib.a2d_metrics_build_each(n, ni, nj, C.c_void_p(_ptr(x)), C.c_void_p(_ptr(y)),
+                                                      (C.c_void_p * n)(*map(_ptr, blobs)), C.c_void_p(s)))
+                for k, xk, yk, m in zip(ks, x.unbind(), y.unbind(), blobs):
                     out[k] = DeviceGrid(nodes=(xk, yk), metrics=m)
             am = amin.cpu().numpy()
             for q, k in enumerate(ks):

@@ -89,8 +89,11 @@ int a2d_grid_build(int n, int ni, int nj, const double* ring, const double* spac
 int a2d_metrics_bytes(int ni, int nj, size_t* bytes);
 /* x, y: device FP64 node coordinates [ni][nj]; metrics: device blob of a2d_metrics_bytes */
 int a2d_metrics_build(int ni, int nj, const double* x, const double* y, void* metrics, void* stream);
-/* the metrics of n grids of one size, their nodes one after another, `stride` bytes (a multiple of
- * 8, at least a2d_metrics_bytes) apart: one launch */
+/* the metrics of n grids of one size, their nodes one after another, into n blobs (metrics: host array of
+ * device pointers): a launch per 128 grids */
+int a2d_metrics_build_each(int n, int ni, int nj, const double* x, const double* y, void* const* metrics, void* stream);
+/* the same into one allocation, `stride` bytes (a multiple of
+ * 8, at least a2d_metrics_bytes) apart */
 int a2d_metrics_build_batch(int n, int ni, int nj, const double* x, const double* y, void* metrics, size_t stride,
                             void* stream);
 

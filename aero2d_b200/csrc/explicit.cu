@@ -285,8 +285,8 @@ __global__ void __launch_bounds__(256) k_irs(Batch b, const double* __restrict__
   for (int x = lane; x < sh.width; x += 32) {
     int i = sh.full ? x : c0 - sh.halo + x;
     i += i < 0 ? ni : 0;
-    i -= i >= ni ? ni : 0;     // the last CTA's columns past the ring (full: past ni, not used) wrap
-    i -= i >= ni ? ni : 0;
+    i -= i >= ni ? ni : 0;     // the last CTA's columns past the ring wrap
+    i = min(i, ni - 1);        // and what lies past its halo is not used
     const double* src = R + base + i;
     for (int j0 = warp; j0 < nc; j0 += kWarps * kRowsAtOnce) {
       double v[kRowsAtOnce];

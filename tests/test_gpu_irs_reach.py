@@ -42,3 +42,14 @@ def test_reach_at_an_integer(cuda, reach):
         Ro = smoothed(R, e)
         Rs = EulerSolver(g, dtype=np.float64, irs_eps=e, device=cuda).smooth(torch.as_tensor(R)).cpu().numpy()
         assert np.max(np.abs(Rs - Ro)) / np.max(np.abs(Ro)) < 1e-12
+
+
+@pytest.mark.parametrize("ni", [4, 8, 9, 10, 11, 14])
+@pytest.mark.parametrize("e", [1e-3, 1e-6])
+def test_small_rings_shorter_than_a_block_of_columns(cuda, ni, e):
+    """Rings that a CTA's 32 columns go round several times, with a reach that does not cover them."""
+    nc = 5
+    R = np.random.default_rng(ni).standard_normal((4, ni, nc))
+    Ro = smoothed(R, e)
+    Rs = EulerSolver(ring(ni, nc), dtype=np.float64, irs_eps=e, device=cuda).smooth(torch.as_tensor(R)).cpu().numpy()
+    assert np.max(np.abs(Rs - Ro)) / np.max(np.abs(Ro)) < 1e-12

@@ -1500,8 +1500,8 @@ int a2d_time_kernel(a2d_plan* P, int which, int reps, float* ms, void* stream) {
       }
       case A2D_K_SWEEP: {
         if (whole) {
-          if (mixed) precond<float>(P, B, P->vec(kZ), P->vec(kPA), 0, s);
-          else precond<double>(P, B, P->vec(kZ), P->vec(kPA), 0, s);
+          if (mixed) precond<float>(P, B, P->vec(kZ), P->vec(kT), 0, s);
+          else precond<double>(P, B, P->vec(kZ), P->vec(kT), 0, s);
           break;
         }
         SweepArgs a = sweep_args(P, 0);
@@ -1514,8 +1514,8 @@ int a2d_time_kernel(a2d_plan* P, int which, int reps, float* ms, void* stream) {
       }
       case A2D_K_SWEEP_FIRST: {
         if (whole) {
-          if (mixed) precond<float>(P, B, P->vec(kZ), P->vec(kPA), 0, s);
-          else precond<double>(P, B, P->vec(kZ), P->vec(kPA), 0, s);
+          if (mixed) precond<float>(P, B, P->vec(kZ), P->vec(kT), 0, s);
+          else precond<double>(P, B, P->vec(kZ), P->vec(kT), 0, s);
           break;
         }
         SweepArgs a = sweep_args(P, 0);
@@ -1538,7 +1538,7 @@ int a2d_time_kernel(a2d_plan* P, int which, int reps, float* ms, void* stream) {
           g.V = Vb;
           g.vstride = vs;
           g.nq = half;
-                g.part = P->at<double>(which == A2D_K_PROJECT ? P->o_cpart2 : P->o_cpart);
+          g.part = P->at<double>(which == A2D_K_PROJECT ? P->o_cpart2 : P->o_cpart);
           g.pstride = P->pstride;
           g.fold_part = P->at<double>(which == A2D_K_PROJECT ? P->o_cpart : P->o_cpart2);
           g.fold_h = P->at<double>(P->o_h2);

@@ -180,6 +180,7 @@ __global__ void __launch_bounds__(kVB) k_combine(Batch b, CombineArgs<TB> a) {
   }
 }
 
+// per-case norms of b and x0 -> ptol (jax gmres: ptol = ||M b|| * min(1, tol ||b|| / ||b||))
 __global__ void k_gm_setup(Batch b, const double* part, int pstride, CaseCtl* ctl, double gtol) {
   grid_wait();
   const int cs = blockIdx.x * blockDim.x + threadIdx.x;
@@ -218,20 +219,6 @@ __global__ void __launch_bounds__(kVB) k_norms2(Batch b, const double* x, const 
     part[(size_t)blockIdx.x * pstride + 0] = acc[0];
     part[(size_t)blockIdx.x * pstride + 1] = acc[1];
   }
-}
-
-// squared norm per chunk
-__global__ void __launch_bounds__(kVB) k_norm1(Batch b, const double* x, double* part, uint32_t need) {
-  grid_wait();
-  const Chunk ch = b.chunks[blockIdx.x];
-  if (!case_live(b, ch.cs, need)) return;
-  const CaseDev cs = b.cases[ch.cs];
-  const size_t base = 4 * cs.cell_off + ch.begin;
-  __shared__ double scratch[32];
-  double acc[1] = {0.0};
-  for (int e = threadIdx.x; e < ch.len; e += blockDim.x) acc[0] += x[base + e] * x[base + e];
-  block_sum_k<double, 1>(acc, scratch);
-  if (threadIdx.x == 0) part[blockIdx.x] = acc[0];
 }
 
 // ---------------------------------------------------------------------------
@@ -382,9 +369,6 @@ void launch_gm_setup(const Batch& b, const double* part, int pstride, CaseCtl* c
 void launch_norms2(const Batch& b, const double* x, const double* y, double* part, int pstride,
                    uint32_t need, cudaStream_t s) {
   if (b.nchunks) launch(k_norms2, b.nchunks, kVB, 0, s, b, x, y, part, pstride, need);
-}
-void launch_norm1(const Batch& b, const double* x, double* part, uint32_t need, cudaStream_t s) {
-  if (b.nchunks) launch(k_norm1, b.nchunks, kVB, 0, s, b, x, part, need);
 }
 void launch_update_rel(const Batch& b, const double* U, const double* dU, double* tpart, uint32_t need,
                        cudaStream_t s) {

@@ -32,7 +32,6 @@ void launch_gm_setup(const Batch& b, const double* part, int pstride, CaseCtl* c
                      cudaStream_t s);
 void launch_norms2(const Batch& b, const double* x, const double* y, double* part, int pstride,
                    uint32_t need, cudaStream_t s);
-void launch_norm1(const Batch& b, const double* x, double* part, uint32_t need, cudaStream_t s);
 void launch_update_rel(const Batch& b, const double* U, const double* dU, double* tpart, uint32_t need,
                        cudaStream_t s);
 void launch_update_check(const Batch& b, const double* U, const double* dU, double* tpart, CaseCtl* ctl,

@@ -1,6 +1,6 @@
 // Launches of a plan's kernel sequences with programmatic dependent launch: a kernel's CTAs are
 // set up as the last ones of the kernel before leave, and wait in grid_wait() for its end, so the
-// next launch overlaps the drain and the memory flush of the last.  An explicit iteration is 13
+// next launch overlaps the drain and the memory flush of the last.  An explicit iteration is 12
 // dependent launches of 2 to 14 us: 60 iterations of three 128x48 cases in FP64 take 8.3 ms with
 // plain launches and 7.0 with these, 40 of 32 256x64 cases in FP32 13.2 and 12.2.  A Newton step's
 // graph takes the same time either way.  Letting the next kernel in earlier, by

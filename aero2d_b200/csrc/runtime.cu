@@ -517,15 +517,15 @@ static void choose_lines(a2d_plan* P) {
   const Fit f = mixed ? Fit{0.58, 0.85, 0.86, 142, 1.2, 2.9, 4 * 148} : Fit{1.0, 1.2, 1.2, 0, 2.45, 4.7, 3 * 148};
   const size_t n = P->line_classes.size();
   std::vector<double> cost(n, 0.0);
+  std::vector<char> can(n, 0);
   for (size_t q = 0; q < n; ++q) {
-    a2d_plan::LineClass& c = P->line_classes[q];
-    c.one = false;
+    const a2d_plan::LineClass& c = P->line_classes[q];
     if (!c.fits) continue;
     const int at_once = mixed ? lines_clusters<float>(c.groups, c.rows) : lines_clusters<double>(c.groups, c.rows);
     // FP64: one CTA per SM, and a second wave loses to the per-sweep kernels (256 x 64: 8 cases
     // 111 against 193 us, 16 cases in two waves 196 against 180)
-    c.fits = at_once > 0 && (mixed || c.count <= at_once);
-    if (!c.fits) continue;
+    can[q] = at_once > 0 && (mixed || c.count <= at_once);
+    if (!can[q]) continue;
     const double full = c.rows <= f.two_rows ? f.full : f.full1;
     const int waves = (c.count - 1) / at_once;
     const double last = (double)(c.count - waves * at_once) / at_once;
@@ -553,14 +553,13 @@ static void choose_lines(a2d_plan* P) {
   double best_t = total(best);
   for (int start = 0; start < 2; ++start) {
     std::vector<char> one(n, 0);
-    if (start == 0)
-      for (size_t q = 0; q < n; ++q) one[q] = P->line_classes[q].fits;
+    if (start == 0) one = can;
     double t = total(one);
     for (bool more = true; more;) {
       more = false;
       size_t at = 0;
       for (size_t q = 0; q < n; ++q) {
-        if (!P->line_classes[q].fits) continue;
+        if (!can[q]) continue;
         one[q] ^= 1;
         const double u = total(one);
         one[q] ^= 1;

@@ -114,12 +114,12 @@ int a2d_plan_ncases(const a2d_plan* plan);
 #define A2D_JVP_TILE_64x4 2
 #define A2D_JVP_TILE_16x16 3
 #define A2D_SWEEP_LANES 0       /* a launch per sweep: one warp per half line group, a lane per line;   */
-                                /* FP64 plans: as HALVES while every case's cluster runs at once       */
+                                /* FP64 plans: as HALVES for the cases that bind chooses it for        */
 #define A2D_SWEEP_ROWS 1        /* a launch per sweep: four warps per half line group, a warp per block row */
 #define A2D_SWEEP_PAIRS 2       /* a launch per sweep: two warps per half line group, two lanes per line */
 #define A2D_SWEEP_HALVES 3      /* every sweep of an application in one launch: a cluster per case, a   */
-                                /* CTA per line group, a recurrence warp per half (cases of more than  */
-                                /* 512 lines or rows past the shared memory: as ROWS)                   */
+                                /* CTA per line group, a recurrence warp per half; for the cases that   */
+                                /* it takes and is the faster path for (a2d_plan_paths), others as ROWS */
 /* a new plan starts with A2D_JVP_TILE_32x16 and A2D_SWEEP_HALVES (FP64 plans: A2D_SWEEP_LANES);
  * A2D_SWEEP_ROWS and A2D_SWEEP_HALVES are refused on FP64 plans (A2D_ERR_ARG) */
 /* any time, bound or not; a change re-captures the Newton step's graph at the next step */
